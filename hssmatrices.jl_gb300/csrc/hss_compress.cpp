@@ -36,6 +36,39 @@ int sm_count(int device) {
   return n;
 }
 
+// The product on the tensor cores, with stream-ordered scratch, so that calls
+// on different streams do not share it.
+int sample_tc(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_t trans, const double* dX, int64_t ldx,
+              int64_t r, double* dY, int64_t ldy, double alpha, double beta, int device, cudaStream_t st) {
+  const SampleTcPlan pl = sample_tc_plan(rows, inner, r, sm_count(device));
+  unsigned char* scratch = nullptr;
+  RC_TRY(cudaMallocAsync((void**)&scratch, pl.scratch_bytes, st));
+  cudaError_t e = launch_sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, pl, scratch, st);
+  count_launches(pl.nsplit > 1 ? 3 : 2);
+  const cudaError_t f = cudaFreeAsync(scratch, st);
+  if (e == cudaSuccess) e = f;
+  return e == cudaSuccess ? HSS_OK : set_cuda_error(e, "sample product");
+}
+
+// The product on the CUDA cores, in FP64 or (HSS_OPT_SAMPLE_DF) double-float.
+int sample_cores(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_t trans, const double* dX,
+                 int64_t ldx, int64_t r, double* dY, int64_t ldy, double alpha, double beta, int device,
+                 cudaStream_t st) {
+  const int nsplit = sample_ksplit(rows, inner, r, sm_count(device), g_sample_df);
+  // split-K partial sums: stream-ordered scratch, so calls on different streams do not share it
+  double* partial = nullptr;
+  if (nsplit > 1) RC_TRY(cudaMallocAsync((void**)&partial, (size_t)nsplit * rows * r * sizeof(double), st));
+  launch_sample_gemm(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, nsplit, partial, g_sample_df,
+                     nullptr, nullptr, st);
+  count_launches(nsplit > 1 ? 2 : 1);
+  cudaError_t e = cudaGetLastError();
+  if (partial) {
+    cudaError_t f = cudaFreeAsync(partial, st);
+    if (e == cudaSuccess) e = f;
+  }
+  return e == cudaSuccess ? HSS_OK : set_cuda_error(e, "sample product");
+}
+
 }  // namespace
 
 struct hss_rc_s {
@@ -265,26 +298,13 @@ int hss_sample(const double* dA, int64_t lda, int64_t m, int64_t n, int32_t tran
   cudaStream_t st = (cudaStream_t)stream;
   int dev = 0;
   RC_TRY(cudaGetDevice(&dev));
-  const int nsplit = sample_ksplit(rows, inner, r, sm_count(dev), g_sample_df);
-  // split-K partial sums: stream-ordered scratch, so calls on different streams do not share it
-  double* partial = nullptr;
-  if (nsplit > 1) RC_TRY(cudaMallocAsync((void**)&partial, (size_t)nsplit * rows * r * sizeof(double), st));
-  launch_sample_gemm(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, nsplit, partial, g_sample_df,
-                     nullptr, nullptr, st);
-  count_launches(nsplit > 1 ? 2 : 1);
-  cudaError_t e = cudaGetLastError();
-  if (partial) {
-    cudaError_t f = cudaFreeAsync(partial, st);
-    if (e == cudaSuccess) e = f;
-  }
-  if (e != cudaSuccess) return set_cuda_error(e, "sample product");
-  return HSS_OK;
+  if (sample_tc_pays(inner)) return sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, dev, st);
+  return sample_cores(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, dev, st);
 }
 
 int hss_rc_sample(hss_rc R, const double* dA, int64_t lda, int32_t trans, const double* dX, int64_t ldx, int64_t r,
                   double* dY, int64_t ldy, void* stream) {
   if (!R) return set_error(HSS_ERR_INVALID, "null handle");
-  if (!g_sample_df) return hss_sample(dA, lda, R->m, R->n, trans, dX, ldx, r, dY, ldy, 1.0, 0.0, stream);
   const int64_t m = R->m, n = R->n;
   if (r < 0 || (trans != 0 && trans != 1)) return set_error(HSS_ERR_BAD_DIMS, "bad sizes");
   const int64_t rows = trans ? n : m, inner = trans ? m : n;
@@ -292,6 +312,14 @@ int hss_rc_sample(hss_rc R, const double* dA, int64_t lda, int32_t trans, const 
   if (r == 0) return HSS_OK;
   if (!dA || !dX || !dY) return set_error(HSS_ERR_INVALID, "null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  if (!g_sample_df) {
+    // the rank decisions that follow depend on the samples' rounding at the
+    // tolerance: the FP64 sums in the order they always had
+    int dev = 0;
+    RC_TRY(cudaGetDevice(&dev));
+    return rows == 0 ? HSS_OK
+                     : sample_cores(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, 1.0, 0.0, dev, st);
+  }
   RC_TRY(cudaSetDevice(R->device));
   const int32_t* lr = R->d_leafof.p;        // rows of A
   const int32_t* lc = R->d_leafof.p + m;    // columns of A

@@ -613,6 +613,13 @@ void launch_sample_gemm(const double* A, int64_t lda, int64_t m, int64_t k, int 
   }
 }
 
+cudaError_t launch_sample_reduce(const double* partial, int nsplit, int64_t m, int64_t r, double* Y, int64_t ldy,
+                                 double alpha, double beta, cudaStream_t st) {
+  const unsigned blocks = (unsigned)std::min<int64_t>((m * r + 255) / 256, 4096);
+  sample_reduce_kernel<<<blocks, 256, 0, st>>>(partial, nsplit, m, r, Y, ldy, alpha, beta);
+  return cudaGetLastError();
+}
+
 void launch_blockdiag_gemm(int32_t count, int64_t max_dim, const double* A, int64_t lda, const int64_t* row0,
                            const int64_t* rows, const int64_t* col0, const int64_t* cols, int trans,
                            const double* X, int64_t ldx, int64_t r, double* Y, int64_t ldy, double alpha,

@@ -59,6 +59,31 @@ int sample_ksplit(int64_t m, int64_t k, int64_t r, int sms, bool df);
 void launch_sample_gemm(const double* A, int64_t lda, int64_t m, int64_t k, int trans, const double* X,
                         int64_t ldx, int64_t r, double* Y, int64_t ldy, double alpha, double beta, int nsplit,
                         double* partial, bool df, const int32_t* lrow, const int32_t* lin, cudaStream_t st);
+// Y = alpha sum_z partial_z + beta Y in the order of z (partial_z: m x r, ld m).
+cudaError_t launch_sample_reduce(const double* partial, int nsplit, int64_t m, int64_t r, double* Y, int64_t ldy,
+                                 double alpha, double beta, cudaStream_t st);
+// The FP64 product on the tensor cores (hss_sample_tc.cu): the column tile, the
+// split of K and the scratch a call needs (digit slices of X, partial sums).
+struct SampleTcPlan {
+  int nc = 0, nsplit = 1;
+  int64_t per = 1;                          // chunks of 128 per split
+  size_t slice_bytes = 0, scratch_bytes = 0;
+};
+// Whether hss_sample's product over k inner terms takes that kernel, with either
+// setting of HSS_OPT_SAMPLE_DF (it is more accurate than the double-float product
+// and no slower: 8192 x 8192, 30 columns: 440 us against 1420 us and, in FP64 on
+// the FP64 pipe, 3750 us; 4096 x 4096, 1 column: 97, 104 and 212 us).  It is also
+// faster below (1242 x 1242, 13 columns: 33 and 80 us).  The line at 2048 terms,
+// and hss_rc_sample staying with the former kernels at every size, keep the rank
+// decisions of compressions what they were: at a tolerance of 1e-9 they depend on
+// the rounding of the samples (2048 points of the Cauchy kernel: one node in 31
+// differs from the reference algorithm's ranks with the former rounding, three
+// with samples that are exact to the last bit).
+inline bool sample_tc_pays(int64_t k) { return k > 2048; }
+SampleTcPlan sample_tc_plan(int64_t m, int64_t k, int64_t r, int sms);
+cudaError_t launch_sample_tc(const double* A, int64_t lda, int64_t m, int64_t k, int trans, const double* X,
+                             int64_t ldx, int64_t r, double* Y, int64_t ldy, double alpha, double beta,
+                             const SampleTcPlan& pl, unsigned char* scratch, cudaStream_t st);
 // HSS_OPT_SAMPLE_DF: hss_sample computes in double-float (default: FP64).
 extern bool g_sample_df;
 // Diagonal-block products of the leaves (see hss_sample.cu).
