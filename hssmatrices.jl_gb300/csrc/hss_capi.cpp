@@ -66,24 +66,9 @@ struct SlotTable {
   DBuf<Slot> dev;
   std::vector<Slot> last;
   GraphCache graph;
-  // a second stream and two events, for launches of a product that may overlap
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  cudaError_t ensure_side() {
-    cudaError_t e = cudaSuccess;
-    if (!side) e = cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-    if (e == cudaSuccess && !ev_fork) e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming);
-    if (e == cudaSuccess && !ev_join) e = cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming);
-    return e;
-  }
   SlotTable() = default;
   SlotTable(const SlotTable&) = delete;
   SlotTable& operator=(const SlotTable&) = delete;
-  ~SlotTable() {
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
-  }
   DBuf<uint32_t> pstate;             // launch counters: zero between launches
   DBuf<unsigned long long> pq;       // queue entries, tagged with the epoch of their launch
   uint32_t epoch = 0;                // tag of the last persistent launch on pq
@@ -217,8 +202,8 @@ struct hss_plan_s {
   hss_factor_s* fused[2] = {nullptr, nullptr};   // storage reused by hss_ulvfactsolve_host
   int64_t gen_len = 0;                  // elements of d_gen
   float2* d_gen_df = nullptr;           // generators as (hi, lo) float pairs, made on first use
-  unsigned char* d_dx = nullptr;        // slices of the leaf blocks D for the tensor-core residual (first use)
-  int64_t dx_bytes = 0;
+  unsigned char* d_oz = nullptr;        // digit slices of the generators for the tensor-core product (first use)
+  int64_t oz_bytes = 0;
   int32_t* d_sync = nullptr;            // per-node arrival counters of the persistent product
   int pmv_nleaf = 0, pmv_mleaf = 0, pmv_kmax = 0;   // largest leaf columns / rows, largest rank
   int64_t pmv_ninner = 0;                           // branches that are not roots
@@ -297,7 +282,7 @@ hss_plan_s::~hss_plan_s() {
   delete fused[0];
   delete fused[1];
   if (d_gen_df) cudaFree(d_gen_df);
-  if (d_dx) cudaFree(d_dx);
+  if (d_oz) cudaFree(d_oz);
   if (d_gen) cudaFree(d_gen);
   if (d_nodes) cudaFree(d_nodes);
   if (d_tasks) cudaFree(d_tasks);
@@ -531,11 +516,6 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
         x.fT21 = fac; fac += align16((int64_t)c2.mr * c1.kv);
       }
       if (x.root) { x.fpiv = fac; fac += align16(x.m); }
-      x.fdx = -1;
-      if (x.leaf && !x.root && dx_tc_fits(x.m, x.n)) {
-        x.fdx = P->dx_bytes;
-        P->dx_bytes += (dx_leaf_bytes(x.n) + 255) & ~int64_t(255);
-      }
       if (!x.root && x.mk > 0) {
         x.fTq = fac; fac += align16((int64_t)((x.k + 31) / 32) * 1024);
         x.fTl = fac; fac += align16((int64_t)((x.mk + 31) / 32) * 1024);
@@ -553,6 +533,16 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
         x.cwz[c] = y.wz;
         x.cwf[c] = y.wf;
       }
+    }
+    for (int32_t i : pre) {
+      Node& x = N[i];
+      auto image = [&](bool up) -> int64_t {
+        const int64_t b = (x.root && !up) ? 0 : ozmv_image_bytes(x, up), o = P->oz_bytes;
+        P->oz_bytes += (b + 255) & ~int64_t(255);
+        return b > 0 ? o : -1;
+      };
+      x.fozu = image(true);
+      x.fozd = image(false);
     }
     nbase += nn;
   }
@@ -822,10 +812,7 @@ bool use_flat(const Levels& L, bool pairs, int rmax) {
   return !pairs && g_flat_product && L.flat_dep > 0 && pmv_flat_fits(L.nleaf, L.kmax, L.flat_dep, rmax);
 }
 
-// dx: the slots carry prepared slices of their leaf blocks (pairs only): the
-// leaf products D X run on the tensor cores before the persistent product.
-int run_pmv(const Levels& L, const Slot* slots, int rmax, bool pairs, SlotTable& pm, cudaStream_t st,
-            bool dx_slices = false) {
+int run_pmv(const Levels& L, const Slot* slots, int rmax, bool pairs, SlotTable& pm, cudaStream_t st) {
   if (use_flat(L, pairs, rmax)) {
     CUDA_TRY(pm.ensure_pmv(1, st));
     CUDA_TRY(pm.ensure_flat(pmv_flat_ctb_elems(L.leaves.cnt, L.flat_dep, L.kmax, rmax),
@@ -848,57 +835,15 @@ int run_pmv(const Levels& L, const Slot* slots, int rmax, bool pairs, SlotTable&
   // a recorded launch replays with this epoch: its queue entries are cleared first
   if (t_graph_capture) CUDA_TRY(cudaMemsetAsync(pm.pq.p, 0, (size_t)qents * sizeof(unsigned long long), st));
   cudaError_t e = cudaSuccess;
-  // double-float residual: the leaf products D X on the tensor cores first,
-  // and the leaf products Z = V^T X and C = alpha (D X + U F) + beta Y as
-  // streams over all leaves around the persistent launch, which keeps the tree
-  // part.  D X and Z = V^T X (both read X, write different buffers) run
-  // concurrently on two streams, joined before the persistent launch.
-  const bool dx = pairs && dx_slices && dx_tc_fits(L.mleaf, L.nleaf);
-  const bool ext = dx && leaf_ext_fits(L.nleaf, L.mleaf, L.kmax);
-  cudaStream_t sv = st;   // stream of the V^T X launch
-  if (ext) {
-    CUDA_TRY(pm.ensure_side());
-    CUDA_TRY(cudaEventRecord(pm.ev_fork, st));
-    CUDA_TRY(cudaStreamWaitEvent(pm.side, pm.ev_fork, 0));
-    sv = pm.side;
-    traced(HSS_TRACE_MV_UP, L.leaves.cnt, sv, [&] {
-      e = launch_leaf_ext(false, L.d_tasks + L.leaves.off, L.leaves.cnt, slots, rmax, L.nleaf, L.mleaf, L.kmax, sv);
-    });
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return cuda_fail(e, "leaf upsweep launch");
-    }
-  }
-  if (dx) {
-    traced(HSS_TRACE_MV_DX, L.leaves.cnt, st, [&] { e = launch_dx_tc(L.d_tasks + L.leaves.off, L.leaves.cnt,
-                                                                     slots, rmax, st); });
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return cuda_fail(e, "tensor-core leaf product launch");
-    }
-  }
-  if (ext) {
-    CUDA_TRY(cudaEventRecord(pm.ev_join, sv));
-    CUDA_TRY(cudaStreamWaitEvent(st, pm.ev_join, 0));
-  }
   traced(HSS_TRACE_MV_LEAF, L.leaves.cnt, st, [&] {
     const void* pf = pairs ? (const void*)L.pfdf : (const void*)L.pf64;
     e = launch_pmv(pairs, L.d_tasks + L.leaves.off, L.leaves.cnt, slots, L.ntasks, L.ninner, rmax, L.nleaf, L.kmax,
                    pm.pstate.p,
-                   pm.pq.p, pm.epoch, pf, pf ? L.pf_elems * 8 : 0, L.device, st, dx, ext);
+                   pm.pq.p, pm.epoch, pf, pf ? L.pf_elems * 8 : 0, L.device, st);
   });
   if (e != cudaSuccess) {
     cudaGetLastError();
     return cuda_fail(e, "persistent product launch");
-  }
-  if (ext) {
-    traced(HSS_TRACE_MV_FINAL, L.leaves.cnt, st, [&] {
-      e = launch_leaf_ext(true, L.d_tasks + L.leaves.off, L.leaves.cnt, slots, rmax, L.nleaf, L.mleaf, L.kmax, st);
-    });
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return cuda_fail(e, "leaf final launch");
-    }
   }
   return HSS_OK;
 }
@@ -915,8 +860,50 @@ cudaError_t pmv_prepare(const Levels& L, bool pairs, int rmax, SlotTable& pm, cu
   } else {
     e = pm.ensure_pmv(pmv_queue_entries(L.ntasks, L.ninner, pmv_chunks(pairs, rmax)), st);
   }
-  if (e == cudaSuccess) e = pm.ensure_side();
   return e;
+}
+
+int sm_count(int device) {
+  static std::atomic<int> known[16];
+  std::atomic<int>& k = known[device & 15];
+  int n = k.load();
+  if (n <= 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || n <= 0) n = 132;
+    k = n;
+  }
+  return n;
+}
+
+// The tensor-core product over the task lists: the slots carry their plan's
+// digit slices (Slot::oz) and FP64 workspaces.
+int run_oz(const Levels& L, const Slot* slots, int rmax, cudaStream_t st) {
+  const Task* T = L.d_tasks;
+  const int sms = sm_count(L.device);
+  cudaError_t e = cudaSuccess;
+  auto step = [&](int trace, int kind, int64_t off, int64_t cnt, int rows) {
+    traced(trace, cnt, st, [&] {
+      if (e == cudaSuccess) e = launch_ozmv(kind, T + off, cnt, slots, rmax, rows, sms, st);
+    });
+  };
+  step(HSS_TRACE_MV_DX, OZ_UP_LEAF, L.leaves.off, L.leaves.cnt, L.mleaf + L.kmax);
+  for (size_t h = 1; h < L.mv_up->size(); ++h) {
+    const Seg& g = (*L.mv_up)[h];
+    step(HSS_TRACE_MV_UP, OZ_UP_BRANCH, g.off, g.cnt, g.kvmax + g.c1u + g.c2u);
+  }
+  const Seg& root = (*L.by_d)[0];
+  if (L.ntasks > 0) {   // not single leaves alone
+    step(HSS_TRACE_MV_UP, OZ_UP_BRANCH, root.off, root.cnt, root.c1u + root.c2u);
+    for (size_t d = 1; d < L.mv_dn->size(); ++d) {
+      const Seg& g = (*L.mv_dn)[d];
+      step(HSS_TRACE_MV_DOWN, OZ_DOWN, g.off, g.cnt, g.c1u + g.c2u);
+    }
+    step(HSS_TRACE_MV_FINAL, OZ_FINAL, L.leaves.off, L.leaves.cnt, L.mleaf);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return cuda_fail(e, "tensor-core product launch");
+  }
+  return HSS_OK;
 }
 
 int run_matvec(const Levels& L, const Slot* slots, int rmax, cudaStream_t st, SlotTable* pm = nullptr) {
@@ -949,9 +936,8 @@ int run_matvec(hss_plan_s* P, const Slot* slots, int rmax, cudaStream_t st, Slot
   return run_matvec(plan_levels(P), slots, rmax, st, pm);
 }
 
-int run_matvec_df(const Levels& L, const Slot* slots, int rmax, cudaStream_t st, SlotTable* pm = nullptr,
-                  bool dx_slices = false) {
-  if (use_pmv(L, pm, true, rmax)) return run_pmv(L, slots, rmax, true, *pm, st, dx_slices);
+int run_matvec_df(const Levels& L, const Slot* slots, int rmax, cudaStream_t st, SlotTable* pm = nullptr) {
+  if (use_pmv(L, pm, true, rmax)) return run_pmv(L, slots, rmax, true, *pm, st);
   const Task* T = L.d_tasks;
   traced(HSS_TRACE_MV_LEAF, L.leaves.cnt, st,
          [&] { launch_dfmv_leaf(T + L.leaves.off, L.leaves.cnt, slots, rmax, st); });
@@ -966,24 +952,37 @@ int run_matvec_df(const Levels& L, const Slot* slots, int rmax, cudaStream_t st,
   return HSS_OK;
 }
 
-// The tensor-core residual's slices of every leaf block D, made once per plan
-// (the generators do not change); false when the plan has no such leaves or
-// the buffer cannot be allocated (the residual then runs without them).
-bool ensure_dx(hss_plan_s* P, cudaStream_t st) {
-  if (P->d_dx) return true;
-  if (P->dx_bytes <= 0 || P->leaves.cnt <= 0) return false;
-  if (dev_alloc((void**)&P->d_dx, (size_t)P->dx_bytes) != cudaSuccess) {
-    P->d_dx = nullptr;
+// The digit slices of the plan's generators for the tensor-core product, made
+// once per plan (the generators do not change); false when the buffer cannot be
+// allocated (other products run then).
+bool ensure_oz(hss_plan_s* P, cudaStream_t st) {
+  if (P->d_oz) return true;
+  if (P->oz_bytes <= 0) return false;
+  if (dev_alloc((void**)&P->d_oz, (size_t)P->oz_bytes) != cudaSuccess) {
+    P->d_oz = nullptr;
     cudaGetLastError();
     return false;
   }
-  if (launch_dx_prep(P->d_tasks + P->leaves.off, P->leaves.cnt, P->d_dx, st) != cudaSuccess) {
+  cudaError_t e = cudaSuccess;
+  auto prep = [&](int kind, const Seg& g, int rows, int inner) {
+    if (e != cudaSuccess || g.cnt <= 0 || rows <= 0 || inner <= 0) return;
+    e = launch_ozmv_prep(kind, P->d_tasks + g.off, g.cnt, rows, inner, P->d_oz, st);
+    add_launches(1);
+  };
+  const int k = P->pmv_kmax;
+  Seg br;   // the branches' lists follow one another
+  br.off = P->mv_dn.empty() ? 0 : P->mv_dn.front().off;
+  for (const Seg& g : P->mv_dn) br.cnt += g.cnt;
+  prep(OZ_UP_LEAF, P->leaves, P->pmv_mleaf + k, P->pmv_nleaf);
+  prep(OZ_FINAL, P->leaves, P->pmv_mleaf, k);
+  prep(OZ_UP_BRANCH, br, 3 * k, 2 * k);
+  prep(OZ_DOWN, br, 2 * k, k);
+  if (e != cudaSuccess) {
     cudaGetLastError();
-    cudaFree(P->d_dx);
-    P->d_dx = nullptr;
+    cudaFree(P->d_oz);
+    P->d_oz = nullptr;
     return false;
   }
-  add_launches(1);
   return true;
 }
 
@@ -1221,6 +1220,20 @@ int check_cols(hss_plan_s* P, const std::vector<Cols>& io, bool solve) {
   return HSS_OK;
 }
 
+// Whether the tensor-core product takes a product of r columns.  It needs one
+// launch per tree level (about 5 us each) and, once per plan, the digit slices
+// (100-400 us with their allocation), and then hardly depends on r up to 32,
+// where the FP64 products grow with entries x columns at the FP64 pipe's rate:
+// n = 65536, k = 32 (15.7 M entries) 276 -> 194 us at r = 6, 938 -> 287 at 32,
+// 1838 -> 422 at 64; n = 16384 166 -> 103 at r = 6; n = 4096 (0.98 M) 105 -> 79
+// at r = 16, 87 -> 69 at 6; n = 10007, leaves of 39, k = 20 (1.3 M) 123 -> 115 at
+// r = 6, 155 -> 130 at 16; n = 2000, k = 16 (0.2 M) 88 -> 76 at r = 64.  The line is
+// where the gain repays the slices within a few products.  Up to 5 columns one
+// launch of the flat or the queued product is as fast (r = 4, n = 65536: 221).
+bool oz_product_pays(const hss_plan_s* P, int64_t r) {
+  return !g_level_product && r >= 6 && P->gen_len * r >= 16000000;
+}
+
 int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double beta,
                 cudaStream_t st, const double* const* Y, double* colnorm2, const int64_t* cn_off,
                 SlotTable& table) {
@@ -1228,6 +1241,7 @@ int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double
   for (auto& c : io) rmax = std::max(rmax, c.r);
   if (rmax == 0) return HSS_OK;
   CUDA_TRY(P->mv_ws.ensure((size_t)P->ws_mv * rmax));
+  const bool oz = oz_product_pays(P, rmax) && ensure_oz(P, st);
   std::vector<Slot> s(P->ntrees);
   for (int32_t t = 0; t < P->ntrees; ++t) {
     Slot& x = s[t];
@@ -1243,9 +1257,11 @@ int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double
     x.err = P->d_err;
     x.nodes = P->d_nodes;
     x.sync = P->d_sync;
+    x.oz = oz ? P->d_oz : nullptr;
   }
   CUDA_TRY(table.upload(s, st));
-  int rc = run_matvec(P, table.dev.p, (int)rmax, st, &table);
+  int rc = oz ? run_oz(plan_levels(P), table.dev.p, (int)rmax, st)
+              : run_matvec(P, table.dev.p, (int)rmax, st, &table);
   if (rc) return rc;
   CUDA_TRY(cudaGetLastError());
   return HSS_OK;
@@ -1702,14 +1718,19 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
   };
   // refinement: R = b - A x (double-float product for FP32 factors unless
   // the FP64 product is forced), x += A_f^{-1} R
-  bool dfres = fp32 && !g_residual_fp64;
-  for (auto& it : items) dfres = dfres && it.f->plan->d_gen_df != nullptr;
+  bool ozres = fp32 && !g_residual_fp64 && g_tensor_dx && !g_level_product && !(tf && tf->tune_pmv == 0);
+  for (auto& it : items) ozres = ozres && ensure_oz(it.f->plan, st);
+  bool dfres = fp32 && !g_residual_fp64 && !ozres;
+  if (dfres)
+    for (auto& it : items) {
+      int rc = ensure_df(it.f->plan, st);
+      if (rc) return rc;
+    }
   if (dfres) {
     CUDA_TRY(B.xs.ensure(std::max<int64_t>(xoff[ni], 1)));
     CUDA_TRY(B.tmp.ensure(std::max<int64_t>(roff[ni], 1)));
   }
   std::vector<Slot> ms(ni);
-  bool dx_slices = dfres && g_tensor_dx;   // every item's plan has its leaf slices prepared
   for (size_t i = 0; i < ni; ++i) {
     const Item& it = items[i];
     hss_plan_s* P = it.f->plan;
@@ -1734,8 +1755,11 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
       x.ldws = P->ws_mv;
       x.gdf = P->d_gen_df;
       x.gbase = P->d_gen;
-      x.dxs = (g_tensor_dx && ensure_dx(P, st)) ? P->d_dx : nullptr;
-      dx_slices = dx_slices && x.dxs != nullptr;
+    } else if (ozres) {
+      CUDA_TRY(it.f->ws2.ensure((size_t)P->ws_mv * rmax));
+      x.ws = it.f->ws2.p;   // as doubles
+      x.ldws = P->ws_mv;
+      x.oz = P->d_oz;
     } else {
       CUDA_TRY(P->mv_ws.ensure((size_t)P->ws_mv * rmax));
       x.ws = P->mv_ws.p;
@@ -1744,7 +1768,7 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
   }
   // the tuned residual product of this factor, else the persistent one where it fits
   SlotTable* pm = (tf && tf->tune_pmv == 0) ? nullptr : &B.mv;
-  const bool persistent = use_pmv(L, pm, dfres, (int)rmax);
+  const bool persistent = !ozres && use_pmv(L, pm, dfres, (int)rmax);
   // R = b - A x and ||R_j||^2 into rn2
   auto issue_residual = [&]() -> int {
     CUDA_TRY(cudaMemsetAsync(B.rn2.p, 0, rtot * sizeof(double), st));
@@ -1754,8 +1778,8 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
         launch_df_split_cols(it.io.C, it.io.ldc, it.f->plan->tree_n[it.tree], it.io.r, B.xs.p + xoff[i], st);
         add_launches(1);
       }
-    return dfres ? run_matvec_df(L, B.mv.dev.p, (int)rmax, st, pm, dx_slices)
-                 : run_matvec(L, B.mv.dev.p, (int)rmax, st, pm);
+    if (ozres) return run_oz(L, B.mv.dev.p, (int)rmax, st);
+    return dfres ? run_matvec_df(L, B.mv.dev.p, (int)rmax, st, pm) : run_matvec(L, B.mv.dev.p, (int)rmax, st, pm);
   };
   const bool loop_on_device = g_graphs && st != nullptr && g_trace.kind < 0 && g_pick_force < 0 &&
                               maxit >= 0 && maxit <= kLoopMaxIt && ni <= (size_t)INT32_MAX;
@@ -1789,7 +1813,7 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
     std::memcpy(&tolbits, &tolv, sizeof(tolbits));
     for (uint64_t v : {(uint64_t)(uintptr_t)fuse, (uint64_t)(uintptr_t)ready, tolbits, (uint64_t)maxit,
                        (uint64_t)fp32, (uint64_t)dfres,
-                       (uint64_t)persistent, (uint64_t)dx_slices, (uint64_t)(uintptr_t)pm,
+                       (uint64_t)persistent, (uint64_t)ozres, (uint64_t)(uintptr_t)pm,
                        (uint64_t)g_generic_factor, (uint64_t)g_flat_product, (uint64_t)pmv_poll_limit(),
                        (uint64_t)(uintptr_t)B.mv.pq.p, (uint64_t)(uintptr_t)B.mv.pstate.p,
                        (uint64_t)(uintptr_t)B.mv.ctb.p, (uint64_t)(uintptr_t)B.mv.dcnt.p,
@@ -2370,10 +2394,8 @@ int hss_ulvfactor(hss_handle h, int32_t precision, hss_factor* out, void* stream
     delete f;
     return cuda_fail(e, "device allocation (factor)");
   }
-  int rc = precision == HSS_PREC_FP32 ? ensure_df(h, (cudaStream_t)stream) : HSS_OK;
-  if (!rc)
-    rc = precision == HSS_PREC_FP32 ? factor_impl<float>(f, (cudaStream_t)stream)
-                                    : factor_impl<double>(f, (cudaStream_t)stream);
+  int rc = precision == HSS_PREC_FP32 ? factor_impl<float>(f, (cudaStream_t)stream)
+                                      : factor_impl<double>(f, (cudaStream_t)stream);
   if (rc) { delete f; return rc; }
   *out = f;
   return HSS_OK;
@@ -2505,7 +2527,7 @@ int hss_device_bytes(hss_handle h, hss_factor f, int64_t* bytes) {
     const int64_t nn = (int64_t)h->nodes.size();
     b += h->gen_len * 8;
     if (h->d_gen_df) b += h->gen_len * 8;
-    if (h->d_dx) b += h->dx_bytes;
+    if (h->d_oz) b += h->oz_bytes;
     // node descriptors, task lists, flat-product links, paths and counters
     b += nn * (int64_t)(sizeof(Node) + 4 * sizeof(Task) + sizeof(FlatLink) + 4 * (h->flat_dep + 1));
     b += (int64_t)(h->mv_ws.cap + h->hB.cap + h->hC.cap) * 8 + slots(h->mv_slots);
@@ -2654,7 +2676,6 @@ int hss_batcher_factor(hss_batcher b, int32_t count, const hss_handle* hs, int32
     cudaError_t e = dev_alloc(&f->d_fac, f->fac_bytes);
     if (e != cudaSuccess) { delete f; rc = cuda_fail(e, "device allocation (factor)"); break; }
     fs[i] = f;
-    if (precision == HSS_PREC_FP32) rc = ensure_df(plans[i], st);
   }
   if (!rc) rc = batcher_levels(b, plans, st);
   if (!rc)

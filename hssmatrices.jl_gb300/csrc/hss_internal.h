@@ -41,9 +41,9 @@ struct Node {
   // column-major) of the QL (fTq, ceil(k/32) panels) and LQ (fTl, ceil(mk/32))
   // reflectors, and the inverses of L1's 32 x 32 diagonal blocks (fLi)
   int64_t fTq, fTl, fLi;
-  // tensor-core residual: byte offset of this leaf's prepared slices of D in
-  // the plan's slice buffer (-1: none)
-  int64_t fdx;
+  // tensor-core product (hss_ozmv.cu): byte offsets of the digit slices of the
+  // node's stacked generators of the upward and the downward sweep (-1: none)
+  int64_t fozu, fozd;
   // the children's ranks, leaf flags and product workspace offsets (left, right),
   // so that a product task reads one descriptor
   int32_t cku[2], ckv[2], cleaf[2];
@@ -94,8 +94,8 @@ struct Slot {
   // its per-node event counters (even between launches)
   const Node* nodes;
   int32_t* sync;
-  // tensor-core residual: the plan's prepared slices of the leaf blocks D
-  const unsigned char* dxs;
+  // tensor-core product: the plan's digit slices
+  const unsigned char* oz;
 };
 
 // Entry extraction (hss_getindex.cu): per node, the node's part of the sorted
@@ -165,6 +165,9 @@ struct PqrTask {
   double atol, rtol;
   int32_t* rank;
 };
+
+// Steps of the tensor-core product (hss_ozmv.cu): stacked generators times columns.
+enum { OZ_UP_LEAF = 0, OZ_UP_BRANCH = 1, OZ_DOWN = 2, OZ_FINAL = 3 };
 
 // device status codes written into Slot::err
 enum { DEV_OK = 0, DEV_SINGULAR = 1, DEV_BAD = 2, DEV_TIMEOUT = 3 };

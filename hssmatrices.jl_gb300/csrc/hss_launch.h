@@ -58,26 +58,16 @@ uint32_t pmv_poll_limit();
 cudaError_t launch_pmv(bool pairs, const Task* leaves, int64_t nleaves, const Slot* slots, int64_t ntasks,
                        int64_t ninner, int rmax,
                        int nleaf, int kmax, uint32_t* state, unsigned long long* qent, uint32_t epoch,
-                       const void* prefetch, int64_t prefetch_bytes, int device, cudaStream_t st,
-                       bool dx_ready = false, bool leaf_ext = false);
-// The other leaf products of the double-float residual, outside the persistent
-// launch (hss_pmv.cu): final_part = false: Z = V^T X of every non-root leaf
-// into the pair workspace (before the launch); true: C = alpha (D X + U F) +
-// beta Y with the column sums of squares (after it).  With dx_ready the
-// persistent launch skips both.
-bool leaf_ext_fits(int nleaf, int mleaf, int kmax);
-cudaError_t launch_leaf_ext(bool final_part, const Task* leaves, int64_t nleaves, const Slot* slots, int rmax, int nleaf,
-                            int mleaf, int kmax, cudaStream_t st);
-// Tensor-core leaf products of the double-float residual (hss_dx_tc.cu): for
-// every non-root leaf task and chunk of 32 columns, D X at ~48-bit accuracy
-// into the slot's pair buffer (sl.tmp), X = the slot's B; leaves up to 128 x 128.
-// A persistent pair product launched after it with dx_ready skips those products.
-bool dx_tc_fits(int mleaf, int nleaf);
-// Bytes of one leaf's prepared slices (n columns), and the once-per-plan
-// preparation over the plan's leaf tasks (regions at each leaf's fdx in base).
-int64_t dx_leaf_bytes(int n);
-cudaError_t launch_dx_prep(const Task* leaves, int64_t nleaves, unsigned char* base, cudaStream_t st);
-cudaError_t launch_dx_tc(const Task* leaves, int64_t nleaves, const Slot* slots, int rmax, cudaStream_t st);
+                       const void* prefetch, int64_t prefetch_bytes, int device, cudaStream_t st);
+// Tensor-core product (hss_ozmv.cu): one launch per step and tree level.  The
+// digit slices of a node's stacked generators (bytes: ozmv_image_bytes of the
+// upward / downward sweep) are made once per plan over its task lists; `rows`
+// and `inner` bound the stacked rows and their columns over the list's nodes.
+// Honours the poll limit above.
+int64_t ozmv_image_bytes(const Node& nd, bool up);
+cudaError_t launch_ozmv_prep(int kind, const Task* t, int64_t nt, int rows, int inner, unsigned char* base,
+                             cudaStream_t st);
+cudaError_t launch_ozmv(int kind, const Task* t, int64_t nt, const Slot* s, int rmax, int rows, int sms, cudaStream_t st);
 
 // Flat persistent product (hss_pmv.cu), FP64 with few right-hand sides: every
 // leaf carries its own chain of small products up to the root and back, so

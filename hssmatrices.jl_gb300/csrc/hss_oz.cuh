@@ -4,25 +4,26 @@
 // an FP64 sum to that sum.  Shared by the kernels that use it.
 //
 // Splitting.  A row a of K entries has the exponent E of its largest entry; its
-// entries are cut to 56-bit fixed point, a_k = F_k 2^(E - 1078) with E biased and
-// |F_k| < 2^56, and F_k cut into eight 7-bit digits, each exact in bf16.  A
-// column x likewise (exponent G).  A digit product summed over K <= 128 is an
-// integer below 128 * 127^2 < 2^21, so the (at most eight) products of one
-// anti-diagonal d = p + q add up exactly in FP32 (< 2^24): accumulator d of
-// tensor memory holds S_d = sum_{p + q = d} A_p X_q for d <= 8, and
+// entries are cut to 63-bit fixed point, a_k = F_k 2^(E - 1085) with E biased and
+// |F_k| < 2^63, and F_k cut into nine 7-bit digits, each exact in bf16.  A column
+// x likewise (exponent G).  A digit product summed over K <= 128 is an integer
+// below 128 * 127^2 < 2^21; the products of one anti-diagonal d = p + q <= 8 add
+// up exactly in FP32 (< 2^24: the last digit of an entry is not zero only where
+// its first is below 8, so the nine products of d = 8 come to eight at most):
+// accumulator d of tensor memory holds S_d = sum_{p + q = d} A_p X_q, and
 //     a . x = 2^(E + G - 2114) T,   T = sum_{d <= 8} S_d 2^(56 - 7 d),
 // an integer below 2^78 that is put together and rounded once to FP64 by
 // integer instructions (GB300 issues FP64 at 1/64 of its FP32 rate).
 //
 // Check.  With u = 2^(E + G - 2044), above every |a_k x_k|: the cut to fixed
 // point and the dropped digit products (d > 8) err by at most
-// 2.05 K 2^-56 u; an FP64 sum of the same terms has the bound K 2^-53 M,
+// 10 K 2^-63 u; an FP64 sum of the same terms has the bound K 2^-53 M,
 // M = sum |a_k| |x_k|.  The tensor cores also form
 // S_abs = sum |top digit of a_k| |top digit of x_k|, and M >= S_abs 2^-14 u, so
-// S_abs >= 4230 makes the first bound (with the final rounding, at K = 128) the
-// smaller one.  Outputs with S_abs below kAbsMin, and rows and columns with
-// infinities, NaN, or exponents near the ends of the range, are summed in FP64
-// from the operands instead.
+// S_abs >= 161 makes the first bound (with the final rounding, at K = 128; 320
+// at K = 2) the smaller one.  Outputs with S_abs below kAbsMin, and rows and
+// columns with infinities, NaN, or exponents near the ends of the range, are
+// summed in FP64 from the operands instead.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -32,10 +33,10 @@
 namespace hss {
 namespace oz {
 
-constexpr int kDigits = 8;           // 7-bit digits per value
+constexpr int kDigits = 9;           // 7-bit digits per value
 constexpr int kSlices = kDigits + 1; // and |top digit|, for the check
 constexpr int kAcc = 9;              // accumulators S_0 .. S_8; S_abs follows them
-constexpr float kAbsMin = 8192.f;
+constexpr float kAbsMin = 512.f;
 constexpr uint32_t kWaitLimit = 1u << 24;
 
 // Exponent codes of a row (column): its largest biased exponent, or one of
@@ -109,33 +110,37 @@ __device__ __forceinline__ int exp_code(int emax, bool any) {
   return !any ? kZero : (emax < 64 || emax == 0x7FF) ? kFar : emax;
 }
 
-// |x| cut to 56-bit fixed point relative to biased exponent emax, as two 28-bit
-// halves (digits 0..3 and 4..7).  shr.b64 gives 0 for shifts of 64 and more, which
+// |x| cut to 63-bit fixed point relative to biased exponent emax: digits 0..3 and
+// 4..7 as 28-bit words, digit 8.  shr.b64 gives 0 for shifts of 64 and more, which
 // takes care of zeros and subnormals (rows with a code have emax >= 64).
-__device__ __forceinline__ void fixed56(unsigned long long b, int emax, uint32_t& hi, uint32_t& lo) {
+__device__ __forceinline__ void fixed63(unsigned long long b, int emax, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   const uint32_t bh = (uint32_t)(b >> 32);
   const unsigned long long L = (b << 11) | (1ull << 63);
-  const uint32_t sh = (uint32_t)(emax + 8) - ((bh >> 20) & 0x7FFu);
+  const uint32_t sh = (uint32_t)(emax + 1) - ((bh >> 20) & 0x7FFu);
   unsigned long long F;
   asm("shr.b64 %0, %1, %2;" : "=l"(F) : "l"(L), "r"(sh));
-  hi = (uint32_t)(F >> 28);
-  lo = (uint32_t)F & 0xFFFFFFFu;
+  hi = (uint32_t)(F >> 35);
+  mid = (uint32_t)(F >> 7) & 0xFFFFFFFu;
+  lo = (uint32_t)F & 0x7Fu;
 }
 
 // The digits of a pair of values as packed bf16 pairs (first value in the low
 // half): a digit a < 128 is the bf16 128 + a (bits 0x4300 | a) minus 128, both
 // exact, multiplied by the sign in the same packed FMA.
 struct Pair {
-  uint32_t h0, l0, h1, l1, sg;   // sg: the signs as a packed pair of +-1
+  uint32_t h0, m0, h1, m1, l, sg;   // l: the last digits, packed; sg: the signs as a packed pair of +-1
   __device__ __forceinline__ Pair(unsigned long long b0, unsigned long long b1, int emax) {
-    fixed56(b0, emax, h0, l0);
-    fixed56(b1, emax, h1, l1);
-    const uint32_t s = ((uint32_t)(b0 >> 63) << 15) | ((uint32_t)(b1 >> 63) << 31);
+    uint32_t l0, l1;
+    fixed63(b0, emax, h0, m0, l0);
+    fixed63(b1, emax, h1, m1, l1);
+    l = l0 | (l1 << 16) | 0x43004300u;
+    const uint32_t s = ((uint32_t)(b0 >> 63) << 15) | ((uint32_t)(b1 >> 32) & 0x80000000u);
     sg = 0x3F803F80u ^ s;
   }
   __device__ __forceinline__ uint32_t raw(int p) const {   // 128 + digit, both values
+    if (p == 8) return l;
     const int s = 21 - 7 * (p & 3);
-    const uint32_t a = p < 4 ? h0 : l0, c = p < 4 ? h1 : l1;
+    const uint32_t a = p < 4 ? h0 : m0, c = p < 4 ? h1 : m1;
     const uint32_t u = s <= 16 ? c << (16 - s) : c >> (s - 16);
     return ((a >> s) & 0x7Fu) | (u & 0x7F0000u) | 0x43004300u;
   }
@@ -200,20 +205,28 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // NC columns each (accumulator d at column NC d, S_abs at NC kAcc).
 template <int NC>
 __device__ __forceinline__ void gather4(uint32_t tmem, long long (&hi)[4], long long (&lo)[4], float (&sabs)[4]) {
-  float v[kAcc][4];
+  {
+    float v[4][4];
 #pragma unroll
-  for (int d = 0; d < kAcc; ++d) tmem_ld4(tmem + (uint32_t)(NC * d), v[d]);
+    for (int d = 0; d < 4; ++d) tmem_ld4(tmem + (uint32_t)(NC * d), v[d]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      hi[i] = __float2int_rn(v[3][i]);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) hi[i] += (long long)__float2int_rn(v[d][i]) * (1 << (21 - 7 * d));
+    }
+  }
+  float v[5][4];
+#pragma unroll
+  for (int d = 0; d < 5; ++d) tmem_ld4(tmem + (uint32_t)(NC * (d + 4)), v[d]);
   tmem_ld4(tmem + (uint32_t)(NC * kAcc), sabs);
   tmem_wait_ld();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    hi[i] = 0;
-    lo[i] = __float2int_rn(v[8][i]);
+    lo[i] = __float2int_rn(v[4][i]);
 #pragma unroll
-    for (int d = 0; d < 4; ++d) {
-      hi[i] += (long long)__float2int_rn(v[d][i]) << (21 - 7 * d);
-      lo[i] += (long long)__float2int_rn(v[d + 4][i]) << (28 - 7 * d);
-    }
+    for (int d = 0; d < 4; ++d) lo[i] += (long long)__float2int_rn(v[d][i]) * (1 << (28 - 7 * d));
   }
 }
 
@@ -227,11 +240,11 @@ __device__ __forceinline__ void stage_mma(uint32_t tmem, uint32_t a0, uint32_t a
 #pragma unroll
   for (int kk = 0; kk < 2; ++kk) {
     const bool ow = first && kk == 0;
-    // p = 1 reaches S_1 .. S_8 and p = 0 then S_0 alone, so that every
+    // p = 1 reaches S_1 .. S_8 and p = 0 first S_0 alone, so that every
     // accumulator is first written by a product that overwrites it
     mma(tmem + NC, sdesc(a0 + astride + 256 * kk), sdesc(b0 + 256 * kk), idesc(M, 8 * NC), !ow);
     mma(tmem, sdesc(a0 + 256 * kk), sdesc(b0 + 256 * kk), idesc(M, NC), !ow);
-    mma(tmem + NC, sdesc(a0 + 256 * kk), sdesc(b0 + bstride + 256 * kk), idesc(M, 7 * NC), 1);
+    mma(tmem + NC, sdesc(a0 + 256 * kk), sdesc(b0 + bstride + 256 * kk), idesc(M, 8 * NC), 1);
 #pragma unroll
     for (int p = 2; p < kDigits; ++p)
       mma(tmem + NC * p, sdesc(a0 + p * astride + 256 * kk), sdesc(b0 + 256 * kk), idesc(M, (9 - p) * NC), 1);

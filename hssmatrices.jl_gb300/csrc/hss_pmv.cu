@@ -80,8 +80,6 @@ struct PmvArgs {
   int32_t cw;            // columns per chunk (<= RC)
   uint32_t epoch;
   uint32_t idle_limit;   // polls of an idle block before DEV_TIMEOUT
-  int32_t dx_ready;      // pairs: the non-root leaves' D B is already in the pair buffer (tensor cores)
-  int32_t leaf_ext;      // pairs: Z = V^T B is in the workspace and the final products follow the launch
 };
 
 // ---- arithmetic policies ----------------------------------------------------
@@ -641,8 +639,7 @@ __device__ void bulk_unit(const PmvArgs& a, int u, typename P::Acc* part, typena
     for (int64_t off = (int64_t)threadIdx.x * 128; off < bytes; off += PT * 128)
       asm volatile("prefetch.global.L2 [%0];" ::"l"(ub + off));
   }
-  constexpr bool pairs_e = !std::is_same<E, double>::value;
-  if (j0 < sl.r && !(pairs_e && a.dx_ready && !nd.root)) {
+  if (j0 < sl.r) {
     const int nc = min(a.cw, sl.r - j0), m = nd.gm, n = nd.gn;
     E* Xs = sm;
     __syncthreads();
@@ -784,7 +781,6 @@ __global__ void __launch_bounds__(PT, 4) pmv_kernel(PmvArgs a) {
   using E = typename P::E;
   using Acc = typename P::Acc;
   extern __shared__ __align__(16) unsigned char pmv_smem[];
-  constexpr bool pairs_k = !std::is_same<E, double>::value;
   Acc* part = (Acc*)pmv_smem;                    // PART_ELEMS split-K partials
   E* sm = (E*)pmv_smem + PART_ELEMS;             // per-phase staging
   __shared__ int s_cmd, s_x, s_y, s_k;
@@ -864,9 +860,7 @@ __global__ void __launch_bounds__(PT, 4) pmv_kernel(PmvArgs a) {
           node_event(a, slot, sl, node, ch);
         }
       } else if (x.leaf) {
-        // with the leaf products outside the launch (leaf_ext), the final
-        // products C = alpha (D B + U F) + beta Y follow it (leaf_uf_kernel)
-        if (!(pairs_k && a.leaf_ext)) final_leaf<P>(sl, x, j0, nc, part, sm);
+        final_leaf<P>(sl, x, j0, nc, part, sm);
       } else {
         down_node<P>(sl, x, j0, nc, part, sm);
         __syncthreads();
@@ -885,8 +879,7 @@ __global__ void __launch_bounds__(PT, 4) pmv_kernel(PmvArgs a) {
         const Node& nd = tk.nodes[tk.node];
         if (!nd.root) {
           const int j0 = ch * a.cw;
-          // leaf_ext: Z = V^T B is already in the workspace (leaf_vtx_kernel)
-          if (!(pairs_k && a.leaf_ext)) leaf_up<P>(sl, nd, j0, min(a.cw, sl.r - j0), part, sm);
+          leaf_up<P>(sl, nd, j0, min(a.cw, sl.r - j0), part, sm);
           climb_from<P>(a, tk.slot, sl, tk.nodes, tk.node, ch, part, sm);
         }
       } else {
@@ -906,197 +899,6 @@ __global__ void __launch_bounds__(PT, 4) pmv_kernel(PmvArgs a) {
       __threadfence();
       a.state[ST_DONE] = 0;
     }
-  }
-}
-
-// ---- leaf products of the double-float residual outside the persistent launch ----
-//
-// With the leaf blocks D X on the tensor cores (dx_tc_kernel), the other two
-// leaf products of the residual are streamed over all leaves at the width of
-// 32 columns, before and after the tree part: Z = V^T X into the workspace
-// (matmul.jl:34) and C = alpha (D X + U F) + beta Y with the column sums of
-// squares (:46-47).  Each block stages its leaf's generator block and column
-// block once in shared memory; a thread keeps two outputs of one row (V^T X)
-// or four of one row (U F) with their own accumulator chains.
-
-constexpr int XW = 32;   // columns per block of the leaf kernels
-constexpr int LB = 16;   // global loads in flight per thread while a block stages its operands
-
-__device__ void leaf_vtx_unit(const Task tk, const Slot* __restrict__ slots, int cb) {
-  extern __shared__ __align__(16) unsigned char ext_smem[];
-  using P = PDF;
-  using Acc = P::Acc;
-  const Slot& sl = slots[tk.slot];
-  const Node& nd = tk.nodes[tk.node];
-  const int j0 = cb * XW;
-  if (nd.root || nd.kv == 0 || j0 >= sl.r) return;
-  const int n = nd.gn, kv = nd.kv, nc = min(XW, sl.r - j0);
-  const int ld = n | 1;             // odd: a warp's rows c (or columns q) fall in distinct bank pairs
-  float2* Vs = (float2*)ext_smem;   // n x kv, ld ld
-  float2* Xs = Vs + ld * kv;        // n x nc, ld ld
-  // staging: LB loads in flight per thread before the shared-memory stores
-  const float2* V = P::gen(sl, nd.V);
-  for (int e0 = threadIdx.x; e0 < n * kv; e0 += LB * PT) {
-    float2 v[LB];
-#pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int e = e0 + u * PT;
-      v[u] = e < n * kv ? __ldg(V + e) : make_float2(0.f, 0.f);
-    }
-#pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int e = e0 + u * PT;
-      if (e < n * kv) Vs[e % n + (e / n) * ld] = v[u];
-    }
-  }
-  const double* X = sl.B + nd.col0 + (int64_t)j0 * sl.ldb;
-  for (int e0 = threadIdx.x; e0 < n * nc; e0 += LB * PT) {
-    double v[LB];
-#pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int e = e0 + u * PT;
-      v[u] = e < n * nc ? __ldg(X + e % n + (int64_t)(e / n) * sl.ldb) : 0.0;
-    }
-#pragma unroll
-    for (int u = 0; u < LB; ++u) {
-      const int e = e0 + u * PT;
-      if (e < n * nc) Xs[e % n + (e / n) * ld] = split_bits(v[u]);
-    }
-  }
-  __syncthreads();
-  float2* ws = sl.ws2;
-  // 2 x 2 tiles: rows c, c + hc of Z, columns q, q + hq
-  const int hc = (kv + 1) / 2, hq = (nc + 1) / 2;
-  for (int it = threadIdx.x; it < hc * hq; it += PT) {
-    const int c = it % hc, q = it / hc;
-    const int c2 = c + hc < kv ? c + hc : c, q2 = q + hq < nc ? q + hq : q;
-    const float2* va = Vs + c * ld;
-    const float2* vb = Vs + c2 * ld;
-    const float2* xa = Xs + q * ld;
-    const float2* xb = Xs + q2 * ld;
-    Acc s00 = P::zero(), s01 = P::zero(), s10 = P::zero(), s11 = P::zero();
-#pragma unroll 2
-    for (int l = 0; l < n; ++l) {
-      const float2 a0 = va[l], a1 = vb[l], b0 = xa[l], b1 = xb[l];
-      P::fma(s00, a0, b0);
-      P::fma(s01, a0, b1);
-      P::fma(s10, a1, b0);
-      P::fma(s11, a1, b1);
-    }
-    ws[nd.wz + c + (int64_t)(j0 + q) * sl.ldws] = P::fin(s00);
-    if (q2 != q) ws[nd.wz + c + (int64_t)(j0 + q2) * sl.ldws] = P::fin(s01);
-    if (c2 != c) ws[nd.wz + c2 + (int64_t)(j0 + q) * sl.ldws] = P::fin(s10);
-    if (c2 != c && q2 != q) ws[nd.wz + c2 + (int64_t)(j0 + q2) * sl.ldws] = P::fin(s11);
-  }
-}
-
-__device__ void leaf_uf_unit(const Task tk, const Slot* __restrict__ slots, int cb) {
-  extern __shared__ __align__(16) unsigned char ext_smem[];
-  using P = PDF;
-  using Acc = P::Acc;
-  const Slot& sl = slots[tk.slot];
-  const Node& nd = tk.nodes[tk.node];
-  const int j0 = cb * XW;
-  if (nd.root || j0 >= sl.r) return;
-  const int m = nd.gm, ku = nd.ku, nc = min(XW, sl.r - j0);
-  float2* Us = (float2*)ext_smem;   // m x ku, ld m
-  float2* Fs = Us + m * ku;         // ku x nc, ld ku
-  if (ku > 0) {
-    const float2* U = P::gen(sl, nd.U);
-    for (int e0 = threadIdx.x; e0 < m * ku; e0 += LB * PT) {
-      float2 v[LB];
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int e = e0 + u * PT;
-        v[u] = e < m * ku ? __ldg(U + e) : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int e = e0 + u * PT;
-        if (e < m * ku) Us[e] = v[u];
-      }
-    }
-    const float2* F = sl.ws2 + nd.wf + (int64_t)j0 * sl.ldws;
-    for (int e0 = threadIdx.x; e0 < ku * nc; e0 += LB * PT) {
-      float2 v[LB];
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int e = e0 + u * PT;
-        v[u] = e < ku * nc ? __ldcg(F + e % ku + (int64_t)(e / ku) * sl.ldws) : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < LB; ++u) {
-        const int e = e0 + u * PT;
-        if (e < ku * nc) Fs[e] = v[u];
-      }
-    }
-  }
-  __syncthreads();
-  const float2* T = (const float2*)sl.tmp + nd.row0 + (int64_t)j0 * sl.ldt2;
-  const double* Y = sl.Y ? sl.Y + nd.row0 + (int64_t)j0 * sl.ldy : nullptr;
-  const bool yterm = sl.beta != 0.0 && Y != nullptr;
-  double* C = sl.C + nd.row0 + (int64_t)j0 * sl.ldc;
-  double* cn = sl.colnorm2 ? sl.colnorm2 + j0 : nullptr;
-  const int tid = threadIdx.x, lane = tid & 31;
-  // a warp takes 32 consecutive rows and, per pass, 4 columns (each thread
-  // 2 rows 32 apart x 4 columns: 8 accumulator chains); warps cycle through
-  // (row block, column block) pairs
-  const int nrb = (m + 63) / 64, ncb = (nc + 3) / 4;
-  for (int job = tid >> 5; job < nrb * ncb; job += PT / 32) {
-    const int rb = job % nrb, cb = job / nrb;
-    const int i0 = rb * 64 + lane, i1 = i0 + 32;
-    const int qb = cb * 4, nq = min(4, nc - qb);
-    const bool a0 = i0 < m, a1 = i1 < m;
-    Acc acc0[4] = {P::zero(), P::zero(), P::zero(), P::zero()};
-    Acc acc1[4] = {P::zero(), P::zero(), P::zero(), P::zero()};
-    const float2* f = Fs + qb * ku;
-#pragma unroll 2
-    for (int l = 0; l < ku; ++l) {
-      const float2 u0 = a0 ? Us[i0 + l * m] : make_float2(0.f, 0.f);
-      const float2 u1 = a1 ? Us[i1 + l * m] : make_float2(0.f, 0.f);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 fq = q < nq ? f[l + q * ku] : make_float2(0.f, 0.f);
-        P::fma(acc0[q], u0, fq);
-        P::fma(acc1[q], u1, fq);
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      double v2 = 0.0;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int i = h ? i1 : i0;
-        if ((h ? a1 : a0) && q < nq) {
-          Acc t = h ? acc1[q] : acc0[q];
-          P::addE(t, __ldcg(T + i + (int64_t)(qb + q) * sl.ldt2));
-          double v = sl.alpha * P::dbl(t);
-          if (yterm) v += sl.beta * __ldcg(Y + i + (int64_t)(qb + q) * sl.ldy);
-          C[i + (int64_t)(qb + q) * sl.ldc] = v;
-          v2 = fma(v, v, v2);
-        }
-      }
-      if (cn != nullptr) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-        if (lane == 0 && q < nq && v2 != 0.0) atomicAdd(cn + qb + q, v2);
-      }
-    }
-  }
-}
-
-// Units (leaf, block of XW columns) taken in turn by a grid of resident blocks,
-// so that the last wave is not a partial one.  The final products fit four
-// blocks per SM (64 registers, 40 KB of shared memory at k = 32), so 512
-// leaves take one round instead of two.
-template <bool FINAL>
-__global__ void __launch_bounds__(PT, (FINAL ? 4 : 2)) leaf_ext_kernel(const Task* __restrict__ leaves, const Slot* __restrict__ slots,
-                                                      int nunits, int ncb) {
-  for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-    const Task tk = leaves[u / ncb];
-    if (FINAL) leaf_uf_unit(tk, slots, u % ncb);
-    else leaf_vtx_unit(tk, slots, u % ncb);
-    __syncthreads();   // the shared buffers are reused by the next unit
   }
 }
 
@@ -1562,7 +1364,7 @@ cudaError_t launch_pmv(bool pairs, const Task* leaves, int64_t nleaves, const Sl
                        int64_t ninner, int rmax,
                        int nleaf, int kmax, uint32_t* state, unsigned long long* qent, uint32_t epoch,
                        const void* prefetch,
-                       int64_t prefetch_bytes, int device, cudaStream_t st, bool dx_ready, bool leaf_ext) {
+                       int64_t prefetch_bytes, int device, cudaStream_t st) {
   if (nleaves <= 0) return cudaSuccess;
   const size_t smem = pmv_smem_elems(nleaf, kmax, nullptr) * 8;
   PmvArgs a;
@@ -1580,8 +1382,6 @@ cudaError_t launch_pmv(bool pairs, const Task* leaves, int64_t nleaves, const Sl
   a.pf = (const char*)prefetch;
   a.pf_bytes = prefetch ? prefetch_bytes : 0;
   a.idle_limit = g_idle_limit;
-  a.dx_ready = (pairs && dx_ready) ? 1 : 0;
-  a.leaf_ext = (pairs && leaf_ext) ? 1 : 0;
   void* args[] = {&a};
   const int cap = pairs ? resident_blocks<PDF>(smem, device) : resident_blocks<PF64>(smem, device);
   if (cap <= 0) return cudaErrorLaunchOutOfResources;
@@ -1646,41 +1446,6 @@ cudaError_t launch_pmv_flat(const Task* leaves, int64_t nleaves, const Task* bra
   const unsigned grid = (unsigned)std::min<int64_t>(cap, std::max<int64_t>(1, units));
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel((void*)pmv_flat_kernel, grid, PT, args, smem, st);
-}
-
-size_t leaf_ext_smem(int nleaf, int mleaf, int kmax) {
-  const size_t up = ((size_t)(nleaf | 1) * kmax + (size_t)(nleaf | 1) * XW) * sizeof(float2);
-  const size_t fin = ((size_t)mleaf * kmax + (size_t)kmax * XW) * sizeof(float2);
-  return std::max(up, fin);
-}
-
-bool leaf_ext_fits(int nleaf, int mleaf, int kmax) { return leaf_ext_smem(nleaf, mleaf, kmax) <= 160 * 1024; }
-
-cudaError_t launch_leaf_ext(bool final_part, const Task* leaves, int64_t nleaves, const Slot* slots, int rmax, int nleaf,
-                            int mleaf, int kmax, cudaStream_t st) {
-  if (nleaves <= 0 || rmax <= 0) return cudaSuccess;
-  const size_t smem = leaf_ext_smem(nleaf, mleaf, kmax);
-  void (*k)(const Task*, const Slot*, int, int) = final_part ? leaf_ext_kernel<true> : leaf_ext_kernel<false>;
-  // resident blocks per SM for this shared-memory size (cached per kernel)
-  static size_t c_smem[2] = {0, 0};
-  static int c_blocks[2] = {0, 0};
-  const int w = final_part ? 1 : 0;
-  if (c_smem[w] != smem || c_blocks[w] <= 0) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 1));
-    if (e != cudaSuccess) return e;
-    int per_sm = 0, sms = 0, dev = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, PT, smem)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    c_smem[w] = smem;
-    c_blocks[w] = std::max(1, per_sm * sms);
-  }
-  const int ncb = (rmax + XW - 1) / XW;
-  const int64_t units = nleaves * (int64_t)ncb;
-  if (units > (int64_t)INT32_MAX) return cudaErrorInvalidValue;
-  const unsigned grid = (unsigned)std::min<int64_t>(units, c_blocks[w]);
-  k<<<grid, PT, smem, st>>>(leaves, slots, (int)units, ncb);
-  return cudaGetLastError();
 }
 
 }  // namespace hss

@@ -2,7 +2,7 @@
 // (reference src/compression.jl:290-291, :326-327, :336-337) in FP64 accuracy on
 // the tensor cores (hss_oz.cuh): GB300's FP64 pipe needs 64 clocks per warp
 // instruction, so the products were bound by it (93 % of its peak) and not by
-// the bytes of A; as 44 exact bf16 digit products they come within a small
+// the bytes of A; as 45 exact bf16 digit products they come within a small
 // factor of the time that reading A takes.
 //
 // oz_prep_kernel cuts Omega (k x r, small) into digit slices once per call, in

@@ -169,15 +169,15 @@ class HssServer:
     # -- accounting --------------------------------------------------------
     @staticmethod
     def estimate_bytes(hss, precision):
-        """Generators (+ their FP32-pair copy) + factor storage + workspaces, from the sizes."""
+        """Generators (+ their digit slices) + factor storage + workspaces, from the sizes."""
         from .packing import pack_cached
         _table, packed = pack_cached(hss)
         gen = packed.size * 8
         m = hss.size()[0]
         fac_elems = 2 * packed.size + 8 * m     # factor blocks, reflector copies, tau vectors
         item = 4 if precision == "fp32" else 8
-        # FP32 + refinement: the generators' pair copy, and the bf16 slices of the
-        # leaf blocks for the tensor-core residual (7 x 2 bytes per entry)
+        # FP32 + refinement: the digit slices of the generators for the tensor-core
+        # residual (9 x 2 bytes per entry, and the zero blocks of stacked translators)
         extra = 3 * gen if precision == "fp32" else 0
         return gen + extra + fac_elems * item + 64 * m * 8
 

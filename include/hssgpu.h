@@ -218,7 +218,7 @@ enum {
   HSS_TRACE_FACTOR_MERGE = 5, /* merge + reduction per level (src/ulvfactor.jl:74-89) */
   HSS_TRACE_SOLVE_UP = 6,     /* upward solve per level */
   HSS_TRACE_SOLVE_DOWN = 7,   /* Q^T back-application per level (src/ulvfactor.jl:98-107) */
-  HSS_TRACE_MV_DX = 8,        /* tensor-core leaf products D X of the refinement residual (src/matmul.jl:46) */
+  HSS_TRACE_MV_DX = 8,        /* tensor-core leaf products D X and V^T X (src/matmul.jl:34, :46) */
   HSS_TRACE_KINDS = 9
 };
 int hss_trace_begin(int32_t kind);
@@ -290,8 +290,7 @@ int64_t hss_launch_counter(void);
  * factorization level to the global-memory kernel (used to test the on-chip
  * kernel against it); 0 (default) picks the on-chip kernel where it fits.
  * HSS_OPT_RESIDUAL_FP64 = 1 forms the refinement residual of an FP32 factor
- * with the native FP64 product instead of the default double-float product
- * on the FP32 pipe (~48-bit, made for GB300's low FP64 rate).
+ * with the product on the FP64 pipe instead of the default tensor-core product.
  * HSS_OPT_LEVEL_PRODUCT = 1 runs every product with one kernel launch per
  * tree level instead of the default single persistent launch (leaves up to
  * 512 columns, ranks up to 64); used to test the two against each other.
@@ -322,11 +321,9 @@ int64_t hss_launch_counter(void);
  * makes the waits run out on purpose (failure-detection tests).  Launch
  * sequences already captured as CUDA graphs keep the limit they were
  * captured with.
- * HSS_OPT_TENSOR_RESIDUAL = 0 turns off the tensor-core leaf products of the
- * double-float refinement residual (1, default: for leaves up to 128 x 128
- * the products D X run as exact bf16 slice products on tcgen05, with FP32
- * accumulation in tensor memory, about 48 significant bits like the rest of
- * the residual; 0: on the FP32 pipe in double-float arithmetic).
+ * HSS_OPT_TENSOR_RESIDUAL = 0 turns off the tensor-core product of the refinement
+ * residual (1, default: every step of the product as exact bf16 digit products
+ * on tcgen05, in FP64 accuracy; 0: in double-float arithmetic on the FP32 pipe).
  * HSS_OPT_FAIL_ALLOC = k > 0 makes the k-th device allocation of this library
  * from now on fail as out of memory, on the host, before the CUDA driver is
  * called (0 disarms): fault injection for the HSS_ERR_OOM paths.  The call
