@@ -113,6 +113,8 @@ struct Seg {
   int kmax = 0, mkmax = 0;                         // largest ULV k and m - k
   int c1mr = 0, c2mr = 0, c1nr = 0, c2nr = 0;      // largest children's reduced sizes
   int64_t sv_stage = 0;                            // largest upward-solve staging need
+  int mk_in = 0, rootmax = 0;                      // largest m - k of the nodes that are not roots; largest root
+  bool leaves = false, branches = false;           // kinds of node in the list
 };
 
 inline int64_t align16(int64_t x) { return (x + 15) & ~int64_t(15); }
@@ -564,6 +566,9 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
           v[lv].kvmax = std::max(v[lv].kvmax, x.kv);
           v[lv].kmax = std::max(v[lv].kmax, x.root ? 0 : x.k);
           v[lv].mkmax = std::max(v[lv].mkmax, x.mk);
+          if (x.root) v[lv].rootmax = std::max(v[lv].rootmax, x.m);
+          else v[lv].mk_in = std::max(v[lv].mk_in, x.mk);
+          (x.leaf ? v[lv].leaves : v[lv].branches) = true;
           {
             const Node* a = x.leaf ? nullptr : &P->nodes[x.left];
             const Node* b = x.leaf ? nullptr : &P->nodes[x.right];
@@ -1005,20 +1010,42 @@ inline size_t factor_extra(const Seg& g) {
 }
 
 template <typename T>
+bool factor_level_blk(const Seg& g) {
+  return factor_blk_fits<T>(g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g));
+}
+// Levels reduced by panels with the block updates on the tensor cores.  FP64: all
+// that fit (n = 65536, k = 32: 12.6 -> 5.8 ms; 256-row leaves, k = 40: 10.2 -> 5.9;
+// 1200 unknowns, k = 16: 1.18 -> 0.95).  FP32: levels whose nodes the one-block kernel
+// does not take (156-row leaves, k = 40: 1.47 -> 0.63 ms); where it fits it is faster
+// (n = 65536: 1.45 against 1.83 ms).
+template <typename T>
+bool factor_level_pan(const Seg& g) {
+  return factor_pan_fits(g.mmax, g.nmax) && (sizeof(T) == 8 || !factor_level_blk<T>(g));
+}
+template <typename T>
 bool factor_level_fast(const Seg& g) {
-  return !g_generic_factor && factor_blk_fits<T>(g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g));
+  return !g_generic_factor && (factor_level_blk<T>(g) || factor_level_pan<T>(g));
 }
 
-// One factor level (h = tree height); true when it ran the on-chip kernel.
+// One factor level (h = tree height); true when it ran one of the kernels whose
+// factors carry the panel T matrices and (FP32) the L1 block inverses.
 template <typename T>
 bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t st) {
   const Seg& g = (*L.by_h)[h];
   const bool fast = factor_level_fast<T>(g);
   traced(h == 0 ? HSS_TRACE_FACTOR_LEAF : HSS_TRACE_FACTOR_MERGE, g.cnt, st, [&] {
-    if (fast)
+    if (fast && factor_level_pan<T>(g)) {
+      FactorDims d;
+      d.mmax = g.mmax; d.nmax = g.nmax; d.kmax = g.kmax; d.mkmax = g.mk_in; d.kvmax = g.kvmax; d.rootmax = g.rootmax;
+      d.leaves = g.leaves; d.branches = g.branches;
+      int launches = 0;
+      launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
+      add_launches(launches - 1);   // traced() counts one
+    } else if (fast) {
       launch_ulv_factor_blk<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g), st);
-    else
+    } else {
       launch_ulv_factor<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, st);
+    }
   });
   return fast;
 }
@@ -1133,6 +1160,10 @@ Seg merge_seg_dims(Seg a, const Seg& b) {
   a.c1mr = std::max(a.c1mr, b.c1mr); a.c2mr = std::max(a.c2mr, b.c2mr);
   a.c1nr = std::max(a.c1nr, b.c1nr); a.c2nr = std::max(a.c2nr, b.c2nr);
   a.sv_stage = std::max(a.sv_stage, b.sv_stage);
+  a.mk_in = std::max(a.mk_in, b.mk_in);
+  a.rootmax = std::max(a.rootmax, b.rootmax);
+  a.leaves = a.leaves || b.leaves;
+  a.branches = a.branches || b.branches;
   return a;
 }
 

@@ -40,32 +40,26 @@
 #include <type_traits>
 
 #include "hss_device.cuh"
+#include "hss_factor.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
 
 namespace hss {
 
+using namespace fac;
+
 namespace {
 
-constexpr int NT = 256;             // threads per block
-constexpr int NW = NT / 32;
 constexpr int BMAX = 128;           // largest m, n
 constexpr int BKMAX = 64;           // largest ku, kv
-constexpr int BP = 32;              // panel width (reflectors per panel)
-constexpr int PL = 8;               // lanes per panel column (QL) or row (LQ)
 constexpr int XC = 64;              // columns (QL) or rows (LQ) of C per GEMM chunk
 constexpr int XP = XC + 4;          // ld of the GEMM intermediate (>= kv, multiple of 4)
-constexpr int GP = BP + 1;          // ld of the Gram matrix and of T
 constexpr int SVP = BMAX;           // length of a broadcast reflector
 constexpr size_t kBlkSmemCap = 226 * 1024;
-static_assert(NT == 8 * BP, "the panel mapping puts 8 lanes on each of 32 columns (rows)");
 static_assert(XP >= BKMAX, "X holds Y V (32 x kv) in the V update");
 
 __host__ __device__ constexpr size_t sz4(size_t e) { return (e + 3) & ~size_t(3); }
 __host__ __device__ constexpr size_t zmax(size_t a, size_t b) { return a > b ? a : b; }
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-
 // shared-memory layout (elements of T), the same on host and device:
 //   D (m x n, ld LDD) | W: U (ld LDU) in the QL phase, the LQ panel (ld YP) in
 //   the LQ phase, the L1-inverse scratch at the end | V (n x kv, ld LDV) |
@@ -180,157 +174,12 @@ __device__ __forceinline__ void small_mm(T* Y, int ldy, T* Yg, const T* A, int l
   else small_mm_r<128>(Y, ldy, Yg, A, lda, B, bj, bl, rows, cols, K);
 }
 
-template <typename T>
-__device__ __forceinline__ T gsum8(T v, unsigned gm) {   // sum over the 8 lanes of a group
-  v += __shfl_xor_sync(gm, v, 4);
-  v += __shfl_xor_sync(gm, v, 2);
-  v += __shfl_xor_sync(gm, v, 1);
-  return v;
-}
-
-// xLARFG from alpha and the squared tail norm: the norm as sqrt(alpha^2 + ss)
-// (hypot only near overflow or underflow); FP32 with correctly rounded
-// reciprocals, FP64 with divisions.
-__device__ __forceinline__ void larfg_t(float alpha, float ss, float& beta, float& tau, float& scal) {
-  if (ss == 0.f) {
-    tau = 0.f;
-    beta = alpha;
-    scal = 1.f;
-    return;
-  }
-  const float t = fmaf(alpha, alpha, ss);
-  const float nrm = t <= 3.0e38f ? sqrtf(t) : hypotf(alpha, sqrtf(ss));
-  beta = -copysignf(nrm, alpha);
-  tau = (beta - alpha) * __frcp_rn(beta);
-  scal = __frcp_rn(alpha - beta);
-}
-__device__ __forceinline__ void larfg_t(double alpha, double ss, double& beta, double& tau, double& scal) {
-  // FP64 runs at 1/64 of the FP32 rate here: the norm as sqrt(alpha^2 + ss)
-  // (hypot only outside [1e-290, 1e290]), the two divisions independent
-  if (ss == 0.0) {
-    tau = 0.0;
-    beta = alpha;
-    scal = 1.0;
-    return;
-  }
-  const double t = fma(alpha, alpha, ss);
-  const double nrm = (t > 1e-290 && t < 1e290) ? sqrt(t) : hypot(alpha, sqrt(ss));
-  beta = -copysign(nrm, alpha);
-  tau = (beta - alpha) / beta;
-  scal = 1.0 / (alpha - beta);
-}
-
-
-// four consecutive elements, 16-byte aligned (FP32) or 32-byte aligned (FP64)
-__device__ __forceinline__ void ld4(float (&v)[4], const float* p) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-}
-__device__ __forceinline__ void ld4(double (&v)[4], const double* p) {
-  const double2 a = reinterpret_cast<const double2*>(p)[0];
-  const double2 b = reinterpret_cast<const double2*>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-}
-
-// acc += a . b over four entries as a chain of fused multiply-adds
-template <typename T>
-__device__ __forceinline__ void fma4(T& acc, const T (&a)[4], const T (&b)[4]) {
-  acc = fma_t(a[0], b[0], acc);
-  acc = fma_t(a[1], b[1], acc);
-  acc = fma_t(a[2], b[2], acc);
-  acc = fma_t(a[3], b[3], acc);
-}
-
 // Y of a QL panel read from U: column a of the panel has its pivot at row p;
 // rows above hold the reflector, the pivot an implicit 1, rows below zeros.
 template <typename T>
 __device__ __forceinline__ void ymask4(T (&y)[4], int r, int p) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) y[q] = r + q < p ? y[q] : (r + q == p ? T(1) : T(0));
-}
-
-// LU with partial pivoting of an m x m block in shared memory (ld).
-template <typename T>
-__device__ void lu_blk(T* A, int m, int ld, int32_t* piv, int32_t* err, T* bv, int* bi, int* prow) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int c = 0; c < m; ++c) {
-    T best = T(-1);
-    int idx = m;
-    for (int i = c + tid; i < m; i += NT) {
-      const T a = dabs(A[i + c * ld]);
-      if (a > best) { best = a; idx = i; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const T ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-      if (ob > best || (ob == best && oi < idx)) { best = ob; idx = oi; }
-    }
-    if (lane == 0) { bv[warp] = best; bi[warp] = idx; }
-    __syncthreads();
-    if (tid == 0) {
-      T b = bv[0];
-      int ix = bi[0];
-      for (int w = 1; w < NW; ++w)
-        if (bv[w] > b || (bv[w] == b && bi[w] < ix)) { b = bv[w]; ix = bi[w]; }
-      if (ix >= m) ix = c;
-      *prow = ix;
-      piv[c] = ix;
-      if (A[ix + c * ld] == T(0) && err != nullptr) atomicExch(err, DEV_SINGULAR);
-    }
-    __syncthreads();
-    const int p = *prow;
-    if (p != c)
-      for (int j = tid; j < m; j += NT) {
-        const T t = A[c + j * ld];
-        A[c + j * ld] = A[p + j * ld];
-        A[p + j * ld] = t;
-      }
-    __syncthreads();
-    const T d = A[c + c * ld];
-    if (d != T(0))
-      for (int i = c + 1 + tid; i < m; i += NT) A[i + c * ld] /= d;
-    __syncthreads();
-    const int rem = m - c - 1;
-    for (int e = tid; e < rem * rem; e += NT) {
-      const int i = c + 1 + e % rem, j = c + 1 + e / rem;
-      A[i + j * ld] -= A[i + c * ld] * A[c + j * ld];
-    }
-    __syncthreads();
-  }
-}
-
-// T = S^{-1} (S = diag(1/tau) + strictly upper G) by warp 0, one row of T per
-// lane in registers, columns in order (xLARFT's recurrence T(i,i) = tau_i,
-// T(0:i, i) = -tau_i T(0:i, 0:i) G(0:i, i)).  Tm row-major (ld GP, zero
-// outside the upper triangle), also written column-major to Tg (32 x 32).
-template <typename T>
-__device__ void blk_tmat(int nb, const T* G, const T* tau, T* Tm, T* Tg) {
-  if (threadIdx.x < 32) {
-    const int l = threadIdx.x;
-    T tr[BP];
-#pragma unroll
-    for (int q = 0; q < BP; ++q) tr[q] = T(0);
-#pragma unroll
-    for (int i = 0; i < BP; ++i) {
-      if (i < nb) {   // warp-uniform
-        T s0 = T(0), s1 = T(0);
-#pragma unroll
-        for (int q = 0; q < i; ++q) {
-          if (q & 1) s1 += tr[q] * G[q * GP + i];
-          else s0 += tr[q] * G[q * GP + i];
-        }
-        const T ti = tau[i];
-        tr[i] = l < i ? -ti * (s0 + s1) : (l == i ? ti : T(0));
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < BP; ++q) {
-      Tm[l * GP + q] = tr[q];
-      Tg[l + q * BP] = tr[q];
-    }
-  }
-  __syncthreads();
 }
 
 // Inverses of the 32 x 32 diagonal blocks of L1 (lower part of D[0:mk, 0:mk],

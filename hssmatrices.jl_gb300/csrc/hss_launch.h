@@ -121,6 +121,17 @@ size_t factor_blk_smem(int mmax, int nmax, int kumax, int kvmax, size_t extra);
 template <typename T>
 void launch_ulv_factor_blk(const Task* t, int64_t ntasks, const Slot* s, int mmax, int nmax, int kumax, int kvmax,
                            size_t extra, cudaStream_t st);
+// The reduction of one level by panels (hss_factor_pan.cu), FP32 or FP64, nodes up
+// to 512 x 512: largest sizes of the level's nodes (roots apart), and which kinds
+// it has.  *launches gets the number of kernels.
+struct FactorDims {
+  int mmax = 0, nmax = 0, kmax = 0, mkmax = 0, kvmax = 0, rootmax = 0;
+  bool leaves = false, branches = false;
+};
+bool factor_pan_fits(int mmax, int nmax);
+template <typename T>
+cudaError_t launch_ulv_factor_pan(const Task* t, int64_t nt, const Slot* s, const FactorDims& d, int sms, int* launches,
+                                  cudaStream_t st);
 // Blocked FP32 solve sweeps (hss_bsolve.cu) over factors of the blocked FP32
 // reduction: sizes are the level's largest node and children's ranks.
 bool bsolve_fits(int mmax, int nmax, int kmax, int kvmax);

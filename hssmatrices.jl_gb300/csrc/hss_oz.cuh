@@ -20,8 +20,8 @@
 // 10 K 2^-63 u; an FP64 sum of the same terms has the bound K 2^-53 M,
 // M = sum |a_k| |x_k|.  The tensor cores also form
 // S_abs = sum |top digit of a_k| |top digit of x_k|, and M >= S_abs 2^-14 u, so
-// S_abs >= 161 makes the first bound (with the final rounding, at K = 128; 320
-// at K = 2) the smaller one.  Outputs with S_abs below kAbsMin, and rows and
+// S_abs >= 161 makes the first bound (with the final rounding, at K = 128; 192 at
+// K = 6) the smaller one.  Outputs with S_abs below kAbsMin, and rows and
 // columns with infinities, NaN, or exponents near the ends of the range, are
 // summed in FP64 from the operands instead.
 #pragma once
@@ -36,7 +36,7 @@ namespace oz {
 constexpr int kDigits = 9;           // 7-bit digits per value
 constexpr int kSlices = kDigits + 1; // and |top digit|, for the check
 constexpr int kAcc = 9;              // accumulators S_0 .. S_8; S_abs follows them
-constexpr float kAbsMin = 512.f;
+constexpr float kAbsMin = 192.f;
 constexpr uint32_t kWaitLimit = 1u << 24;
 
 // Exponent codes of a row (column): its largest biased exponent, or one of
