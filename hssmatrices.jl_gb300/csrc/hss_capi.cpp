@@ -115,7 +115,63 @@ struct Seg {
   int64_t sv_stage = 0;                            // largest upward-solve staging need
   int mk_in = 0, rootmax = 0;                      // largest m - k of the nodes that are not roots; largest root
   bool leaves = false, branches = false;           // kinds of node in the list
+  std::vector<Seg> parts;                          // the list by size of node (empty: one size class)
 };
+
+// Size class of a node for the factor and solve kernels, whose registers and
+// shared memory are laid out for the largest node of a launch.
+inline int size_class(const Node& x) {
+  const int s = std::max(x.m, x.n);
+  return s <= 32 ? 0 : s <= 64 ? 1 : s <= 96 ? 2 : s <= 128 ? 3 : s <= 256 ? 4 : 5;
+}
+
+// Counts node x (children in `nodes`) into the largest sizes of a list.
+inline void seg_add(Seg& v, const Node& x, const Node* nodes) {
+  ++v.cnt;
+  v.mmax = std::max(v.mmax, x.m);
+  v.nmax = std::max(v.nmax, x.n);
+  v.kumax = std::max(v.kumax, x.ku);
+  v.kvmax = std::max(v.kvmax, x.kv);
+  v.kmax = std::max(v.kmax, x.root ? 0 : x.k);
+  v.mkmax = std::max(v.mkmax, x.mk);
+  if (x.root) v.rootmax = std::max(v.rootmax, x.m);
+  else v.mk_in = std::max(v.mk_in, x.mk);
+  (x.leaf ? v.leaves : v.branches) = true;
+  const Node* a = x.leaf ? nullptr : &nodes[x.left];
+  const Node* b = x.leaf ? nullptr : &nodes[x.right];
+  v.sv_stage = std::max(v.sv_stage, solve_up_stage_need(x.m, x.k, x.mk, x.nk, x.kv, x.leaf, x.root, a ? a->mr : 0,
+                                                        b ? b->mr : 0, a ? a->kv : 0, b ? b->kv : 0));
+  if (x.leaf) return;
+  v.c1u = std::max(v.c1u, a->ku);
+  v.c2u = std::max(v.c2u, b->ku);
+  v.c1v = std::max(v.c1v, a->kv);
+  v.c2v = std::max(v.c2v, b->kv);
+  v.c1mr = std::max(v.c1mr, a->mr);
+  v.c2mr = std::max(v.c2mr, b->mr);
+  v.c1nr = std::max(v.c1nr, a->nr);
+  v.c2nr = std::max(v.c2nr, b->nr);
+}
+
+// The list v (tasks off .. off + cnt of `tasks`) ordered by size class, with a part
+// per class where there are several; nodes(i): the node array of its i-th task.
+template <class F>
+void seg_split(Seg& v, std::vector<Task>& tasks, F&& nodes) {
+  v.parts.clear();
+  std::vector<std::pair<int, int64_t>> key((size_t)v.cnt);
+  for (int64_t i = 0; i < v.cnt; ++i) key[i] = {size_class(nodes(i)[tasks[v.off + i].node]), i};
+  std::stable_sort(key.begin(), key.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+  if (key.empty() || key.front().first == key.back().first) return;
+  const std::vector<Task> old(tasks.begin() + v.off, tasks.begin() + v.off + v.cnt);
+  for (int64_t i = 0; i < v.cnt; ++i) {
+    if (i == 0 || key[i].first != key[i - 1].first) {
+      v.parts.emplace_back();
+      v.parts.back().off = v.off + i;
+    }
+    tasks[v.off + i] = old[key[i].second];
+    const Node* nd = nodes(key[i].second);
+    seg_add(v.parts.back(), nd[old[key[i].second].node], nd);
+  }
+}
 
 inline int64_t align16(int64_t x) { return (x + 15) & ~int64_t(15); }
 
@@ -552,7 +608,7 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
   P->ws_sv = std::max<int64_t>(ws_sv, 1);
   P->fac_elems = std::max<int64_t>(fac, 1);
   // task lists
-  auto add_seg = [&](std::vector<Seg>& v, auto pred, int nlev, bool by_height) {
+  auto add_seg = [&](std::vector<Seg>& v, auto pred, int nlev, bool by_height, bool split) {
     v.assign(nlev + 1, Seg{});
     for (int lv = 0; lv <= nlev; ++lv) {
       v[lv].off = (int64_t)tasks.size();
@@ -560,43 +616,16 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
         const Node& x = P->nodes[i];
         if ((by_height ? x.height : x.depth) == lv && pred(x)) {
           tasks.push_back(Task{nullptr, (int32_t)i, x.tree});
-          v[lv].mmax = std::max(v[lv].mmax, x.m);
-          v[lv].nmax = std::max(v[lv].nmax, x.n);
-          v[lv].kumax = std::max(v[lv].kumax, x.ku);
-          v[lv].kvmax = std::max(v[lv].kvmax, x.kv);
-          v[lv].kmax = std::max(v[lv].kmax, x.root ? 0 : x.k);
-          v[lv].mkmax = std::max(v[lv].mkmax, x.mk);
-          if (x.root) v[lv].rootmax = std::max(v[lv].rootmax, x.m);
-          else v[lv].mk_in = std::max(v[lv].mk_in, x.mk);
-          (x.leaf ? v[lv].leaves : v[lv].branches) = true;
-          {
-            const Node* a = x.leaf ? nullptr : &P->nodes[x.left];
-            const Node* b = x.leaf ? nullptr : &P->nodes[x.right];
-            v[lv].sv_stage = std::max(v[lv].sv_stage,
-                                      solve_up_stage_need(x.m, x.k, x.mk, x.nk, x.kv, x.leaf, x.root, a ? a->mr : 0,
-                                                          b ? b->mr : 0, a ? a->kv : 0, b ? b->kv : 0));
-          }
-          if (!x.leaf) {
-            const Node& c1 = P->nodes[x.left];
-            const Node& c2 = P->nodes[x.right];
-            v[lv].c1u = std::max(v[lv].c1u, c1.ku);
-            v[lv].c2u = std::max(v[lv].c2u, c2.ku);
-            v[lv].c1v = std::max(v[lv].c1v, c1.kv);
-            v[lv].c2v = std::max(v[lv].c2v, c2.kv);
-            v[lv].c1mr = std::max(v[lv].c1mr, c1.mr);
-            v[lv].c2mr = std::max(v[lv].c2mr, c2.mr);
-            v[lv].c1nr = std::max(v[lv].c1nr, c1.nr);
-            v[lv].c2nr = std::max(v[lv].c2nr, c2.nr);
-          }
+          seg_add(v[lv], x, P->nodes.data());
         }
       }
-      v[lv].cnt = (int64_t)tasks.size() - v[lv].off;
+      if (split) seg_split(v[lv], tasks, [&](int64_t) { return P->nodes.data(); });
     }
   };
-  add_seg(P->by_h, [](const Node&) { return true; }, max_h, true);
-  add_seg(P->by_d, [](const Node&) { return true; }, max_d, false);
-  add_seg(P->mv_up, [](const Node& x) { return !x.leaf && !x.root; }, max_h, true);
-  add_seg(P->mv_dn, [](const Node& x) { return !x.leaf; }, max_d, false);
+  add_seg(P->by_h, [](const Node&) { return true; }, max_h, true, true);
+  add_seg(P->by_d, [](const Node&) { return true; }, max_d, false, true);
+  add_seg(P->mv_up, [](const Node& x) { return !x.leaf && !x.root; }, max_h, true, false);
+  add_seg(P->mv_dn, [](const Node& x) { return !x.leaf; }, max_d, false, false);
   P->leaves.off = (int64_t)tasks.size();
   for (int64_t i = 0; i < total_nodes; ++i)
     if (P->nodes[i].leaf) tasks.push_back(Task{nullptr, (int32_t)i, P->nodes[i].tree});
@@ -1022,32 +1051,51 @@ template <typename T>
 bool factor_level_pan(const Seg& g) {
   return factor_pan_fits(g.mmax, g.nmax) && (sizeof(T) == 8 || !factor_level_blk<T>(g));
 }
+// Levels of the one-block kernel, whose FP32 factors the blocked solve can read (it
+// needs the inverses of L1's diagonal blocks).
 template <typename T>
 bool factor_level_fast(const Seg& g) {
-  return !g_generic_factor && (factor_level_blk<T>(g) || factor_level_pan<T>(g));
+  return !g_generic_factor && factor_level_blk<T>(g) && !factor_level_pan<T>(g);
 }
 
-// One factor level (h = tree height); true when it ran one of the kernels whose
-// factors carry the panel T matrices and (FP32) the L1 block inverses.
+// Runs f on a level's list, or size class by size class where that is the shorter
+// schedule: a list of several times the SMs is bound by how many blocks fit (a
+// leaf level with 64-, 128- and 256-row leaves in one launch has the layout of the
+// largest; in a batch of 48 matrices 4.0 -> 3.5 ms for its factorization, 0.82 ->
+// 0.64 ms for its upward solve, 1.11 -> 0.86 ms for the first merges), a shorter one
+// by one block's latency, which each class would add.
+template <class F>
+void run_parts(const Levels& L, const Seg& g, F&& f) {
+  const int sms = sm_count(L.device);
+  if (g.parts.empty() || g.cnt <= 2 * sms) {
+    f(g);
+    return;
+  }
+  for (const Seg& p : g.parts) f(p);
+  add_launches((int64_t)g.parts.size() - 1);   // traced() counts one
+}
+
+// One factor level (h = tree height); true when it ran the one-block kernel alone.
 template <typename T>
 bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t st) {
-  const Seg& g = (*L.by_h)[h];
-  const bool fast = factor_level_fast<T>(g);
-  traced(h == 0 ? HSS_TRACE_FACTOR_LEAF : HSS_TRACE_FACTOR_MERGE, g.cnt, st, [&] {
-    if (fast && factor_level_pan<T>(g)) {
-      FactorDims d;
-      d.mmax = g.mmax; d.nmax = g.nmax; d.kmax = g.kmax; d.mkmax = g.mk_in; d.kvmax = g.kvmax; d.rootmax = g.rootmax;
-      d.leaves = g.leaves; d.branches = g.branches;
-      int launches = 0;
-      launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
-      add_launches(launches - 1);   // traced() counts one
-    } else if (fast) {
-      launch_ulv_factor_blk<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g), st);
-    } else {
-      launch_ulv_factor<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, st);
-    }
+  const Seg& all = (*L.by_h)[h];
+  traced(h == 0 ? HSS_TRACE_FACTOR_LEAF : HSS_TRACE_FACTOR_MERGE, all.cnt, st, [&] {
+    run_parts(L, all, [&](const Seg& g) {
+      if (!g_generic_factor && factor_level_pan<T>(g)) {
+        FactorDims d;
+        d.mmax = g.mmax; d.nmax = g.nmax; d.kmax = g.kmax; d.mkmax = g.mk_in; d.kvmax = g.kvmax; d.rootmax = g.rootmax;
+        d.leaves = g.leaves; d.branches = g.branches;
+        int launches = 0;
+        launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
+        add_launches(launches - 1);
+      } else if (factor_level_fast<T>(g)) {
+        launch_ulv_factor_blk<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g), st);
+      } else {
+        launch_ulv_factor<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, st);
+      }
+    });
   });
-  return fast;
+  return factor_level_fast<T>(all);
 }
 
 template <typename T>
@@ -1083,15 +1131,14 @@ inline bool pick_bsolve(bool blocked, const Seg& g, const std::vector<int8_t>* t
 template <typename T>
 void run_solve_up_level(const Levels& L, size_t h, const Slot* slots, int rmax, cudaStream_t st, bool blocked,
                         const std::vector<int8_t>* tup) {
-  const Seg& g = (*L.by_h)[h];
-  traced(HSS_TRACE_SOLVE_UP, g.cnt, st, [&] {
+  traced(HSS_TRACE_SOLVE_UP, (*L.by_h)[h].cnt, st, [&] { run_parts(L, (*L.by_h)[h], [&](const Seg& g) {
     if (pick_bsolve(blocked, g, tup, h))
       launch_bsolve_up(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g), rmax, st);
     else if (!g_generic_factor && solve_reg_fits(g.mmax, g.nmax))
       launch_ulv_solve_up_reg<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.sv_stage, rmax, st);
     else
       launch_ulv_solve_up<T>(L.d_tasks + g.off, g.cnt, slots, st);
-  });
+  }); });
 }
 
 template <typename T>
@@ -1111,15 +1158,14 @@ template <typename T>
 void run_solve_down(const Levels& L, const Slot* slots, int rmax, cudaStream_t st, bool blocked,
                     const std::vector<int8_t>* tdn) {
   for (size_t d = 0; d < L.by_d->size(); ++d) {
-    const Seg& g = (*L.by_d)[d];
-    traced(HSS_TRACE_SOLVE_DOWN, g.cnt, st, [&] {
+    traced(HSS_TRACE_SOLVE_DOWN, (*L.by_d)[d].cnt, st, [&] { run_parts(L, (*L.by_d)[d], [&](const Seg& g) {
       if (pick_bsolve(blocked, g, tdn, d))
         launch_bsolve_down(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g), rmax, st);
       else if (!g_generic_factor && solve_reg_fits(g.mmax, g.nmax))
         launch_ulv_solve_down_reg<T>(L.d_tasks + g.off, g.cnt, slots, g.nmax, g.mkmax, rmax, st);
       else
         launch_ulv_solve_down<T>(L.d_tasks + g.off, g.cnt, slots, st);
-    });
+    }); });
   }
 }
 
@@ -1151,25 +1197,9 @@ struct MergedLevels {
   }
 };
 
-Seg merge_seg_dims(Seg a, const Seg& b) {
-  a.mmax = std::max(a.mmax, b.mmax); a.nmax = std::max(a.nmax, b.nmax);
-  a.kumax = std::max(a.kumax, b.kumax); a.kvmax = std::max(a.kvmax, b.kvmax);
-  a.c1u = std::max(a.c1u, b.c1u); a.c2u = std::max(a.c2u, b.c2u);
-  a.c1v = std::max(a.c1v, b.c1v); a.c2v = std::max(a.c2v, b.c2v);
-  a.kmax = std::max(a.kmax, b.kmax); a.mkmax = std::max(a.mkmax, b.mkmax);
-  a.c1mr = std::max(a.c1mr, b.c1mr); a.c2mr = std::max(a.c2mr, b.c2mr);
-  a.c1nr = std::max(a.c1nr, b.c1nr); a.c2nr = std::max(a.c2nr, b.c2nr);
-  a.sv_stage = std::max(a.sv_stage, b.sv_stage);
-  a.mk_in = std::max(a.mk_in, b.mk_in);
-  a.rootmax = std::max(a.rootmax, b.rootmax);
-  a.leaves = a.leaves || b.leaves;
-  a.branches = a.branches || b.branches;
-  return a;
-}
-
 int merge_levels(const std::vector<hss_plan_s*>& plans, MergedLevels& M, cudaStream_t st) {
   M.h.clear();
-  auto merge = [&](std::vector<Seg>& out, std::vector<Seg> hss_plan_s::*field) {
+  auto merge = [&](std::vector<Seg>& out, std::vector<Seg> hss_plan_s::*field, bool split) {
     size_t nlev = 0;
     for (auto* P : plans) nlev = std::max(nlev, (P->*field).size());
     out.assign(nlev, Seg{});
@@ -1184,17 +1214,17 @@ int merge_levels(const std::vector<hss_plan_s*>& plans, MergedLevels& M, cudaStr
           Task x = P->h_tasks[s.off + t];
           x.slot = (int32_t)i;
           M.h.push_back(x);
+          seg_add(g, P->nodes[x.node], P->nodes.data());
         }
-        g = merge_seg_dims(g, s);
       }
-      g.cnt = (int64_t)M.h.size() - g.off;
-      out[lv] = g;
+      if (split) seg_split(g, M.h, [&](int64_t i) { return plans[M.h[g.off + i].slot]->nodes.data(); });
+      out[lv] = std::move(g);
     }
   };
-  merge(M.by_h, &hss_plan_s::by_h);
-  merge(M.by_d, &hss_plan_s::by_d);
-  merge(M.mv_up, &hss_plan_s::mv_up);
-  merge(M.mv_dn, &hss_plan_s::mv_dn);
+  merge(M.by_h, &hss_plan_s::by_h, true);
+  merge(M.by_d, &hss_plan_s::by_d, true);
+  merge(M.mv_up, &hss_plan_s::mv_up, false);
+  merge(M.mv_dn, &hss_plan_s::mv_dn, false);
   M.leaves = Seg{};
   M.leaves.off = (int64_t)M.h.size();
   for (size_t i = 0; i < plans.size(); ++i) {
