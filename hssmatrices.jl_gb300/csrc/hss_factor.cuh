@@ -119,53 +119,103 @@ __device__ __forceinline__ void fma4(T& acc, const T (&a)[4], const T (&b)[4]) {
   acc = fma_t(a[3], b[3], acc);
 }
 
-// LU with partial pivoting of an m x m block in shared memory (ld).
+// Index of the warp's largest magnitude (ties: the smallest index), by integer
+// reductions on the bits; lanes without an entry pass idx >= 2^30.
+__device__ __forceinline__ int warp_argmax(float x, int idx, bool& zero) {
+  const unsigned a = __float_as_uint(x) & 0x7FFFFFFFu;
+  const unsigned best = __reduce_max_sync(0xffffffffu, a);
+  zero = best == 0;
+  return (int)__reduce_min_sync(0xffffffffu, a == best ? (unsigned)idx : 1u << 30);
+}
+__device__ __forceinline__ int warp_argmax(double x, int idx, bool& zero) {
+  const unsigned long long a = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  const unsigned hi = (unsigned)(a >> 32), bh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lo = hi == bh ? (unsigned)a : 0u, bl = __reduce_max_sync(0xffffffffu, lo);
+  zero = bh == 0 && bl == 0;
+  return (int)__reduce_min_sync(0xffffffffu, hi == bh && lo == bl ? (unsigned)idx : 1u << 30);
+}
+__device__ __forceinline__ bool larger_mag(float a, float b) {
+  return (__float_as_uint(a) & 0x7FFFFFFFu) > (__float_as_uint(b) & 0x7FFFFFFFu);
+}
+__device__ __forceinline__ bool larger_mag(double a, double b) {
+  return ((unsigned long long)__double_as_longlong(a) << 1) > ((unsigned long long)__double_as_longlong(b) << 1);
+}
+__device__ __forceinline__ float recip(float d) { return 1.f / d; }
+__device__ __forceinline__ double recip(double d) {
+  const int e = (int)(__double_as_longlong(d) >> 52) & 0x7FF;
+  if (e < 64 || e > 1982) return 1.0 / d;
+  const double r = rcp_newton(__longlong_as_double(__double_as_longlong(d) & 0x7FFFFFFFFFFFFFFFll));
+  return copysign(r, d);
+}
+
+// LU with partial pivoting of an m x m block (ld), columns dealt to the warps in
+// turn.  One barrier per column: while the other warps apply column c, the owner
+// of column c + 1 applies it there first, finds the next pivot (first entry of
+// largest magnitude, compared on the bits: NaN counts as larger than any number)
+// and scales that column.  lv: 2 x m multipliers; pv: 2 pivots.  A root of 64 rows
+// with its assembly: FP64 215 -> 141 us (five barriers a column, FP64 comparisons
+// and a division per entry before), FP32 unchanged at 94; 32 rows 100 -> 55 and
+// 39 -> 35 us.
 template <typename T>
-__device__ void lu_blk(T* A, int m, int ld, int32_t* piv, int32_t* err, T* bv, int* bi, int* prow) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+__device__ void lu_blk(T* A, int m, int ld, int32_t* piv, int32_t* err, T* lv, int* pv) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // pivot and multipliers of column c, by the warp that owns it
+  auto next = [&](int c) {
+    T* col = A + (int64_t)c * ld;
+    T mine = T(0);
+    int at = 1 << 30;
+    for (int i = c + lane; i < m; i += 32)
+      if (at == 1 << 30 || larger_mag(col[i], mine)) { mine = col[i]; at = i; }
+    bool zero;
+    const int idx = warp_argmax(mine, at, zero);
+    if (lane == 0) {
+      piv[c] = idx;
+      pv[c & 1] = idx;
+      if (zero && err != nullptr) atomicExch(err, DEV_SINGULAR);
+      const T t = col[c];
+      col[c] = col[idx];
+      col[idx] = t;
+    }
+    __syncwarp();
+    const T r = zero ? T(1) : recip(col[c]);
+    T* l = lv + (c & 1) * m;
+    for (int i = c + 1 + lane; i < m; i += 32) {
+      const T x = col[i] * r;
+      col[i] = x;
+      l[i] = x;
+    }
+    __syncwarp();
+  };
+  if (m > 0 && warp == 0) next(0);
+  __syncthreads();
   for (int c = 0; c < m; ++c) {
-    T best = T(-1);
-    int idx = m;
-    for (int i = c + tid; i < m; i += NT) {
-      const T a = dabs(A[i + c * ld]);
-      if (a > best) { best = a; idx = i; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const T ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-      if (ob > best || (ob == best && oi < idx)) { best = ob; idx = oi; }
-    }
-    if (lane == 0) { bv[warp] = best; bi[warp] = idx; }
-    __syncthreads();
-    if (tid == 0) {
-      T b = bv[0];
-      int ix = bi[0];
-      for (int w = 1; w < NW; ++w)
-        if (bv[w] > b || (bv[w] == b && bi[w] < ix)) { b = bv[w]; ix = bi[w]; }
-      if (ix >= m) ix = c;
-      *prow = ix;
-      piv[c] = ix;
-      if (A[ix + c * ld] == T(0) && err != nullptr) atomicExch(err, DEV_SINGULAR);
-    }
-    __syncthreads();
-    const int p = *prow;
-    if (p != c)
-      for (int j = tid; j < m; j += NT) {
-        const T t = A[c + j * ld];
-        A[c + j * ld] = A[p + j * ld];
-        A[p + j * ld] = t;
+    const int p = pv[c & 1];
+    const T* l = lv + (c & 1) * m;
+    // this warp's columns, the next one first (its owner's first column is c + 1)
+    const int first = c + 1 + (warp + NW - (c + 1) % NW) % NW;
+    for (int q = 0; q * NW < m; ++q) {
+      const int j = (first + q * NW) < m ? first + q * NW : -1;
+      if (j < 0) break;
+      T* col = A + (int64_t)j * ld;
+      const T u = col[p];
+      __syncwarp();
+      if (lane == 0 && p != c) {
+        col[p] = col[c];
+        col[c] = u;
       }
-    __syncthreads();
-    const T d = A[c + c * ld];
-    if (d != T(0))
-      for (int i = c + 1 + tid; i < m; i += NT) A[i + c * ld] /= d;
-    __syncthreads();
-    const int rem = m - c - 1;
-    for (int e = tid; e < rem * rem; e += NT) {
-      const int i = c + 1 + e % rem, j = c + 1 + e / rem;
-      A[i + j * ld] -= A[i + c * ld] * A[c + j * ld];
+      __syncwarp();
+      for (int i = c + 1 + lane; i < m; i += 32) col[i] = fma_t(-l[i], u, col[i]);
+      __syncwarp();
+      if (j == c + 1) next(c + 1);
     }
+    // rows already eliminated: exchanged only
+    if (p != c)
+      for (int j = threadIdx.x; j < c; j += NT) {
+        T* col = A + (int64_t)j * ld;
+        const T t = col[c];
+        col[c] = col[p];
+        col[p] = t;
+      }
     __syncthreads();
   }
 }

@@ -548,9 +548,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
     ulv_factor_blk_kernel(const Task* __restrict__ tasks, const Slot* __restrict__ slots, int kumax, int kvmax,
                           int extra) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ T bvals[NW];
-  __shared__ int bidx[NW];
-  __shared__ int prow;
+  __shared__ int s_piv[2];
   const BlkLayout Lo(S, kumax, kvmax, (size_t)extra);
   const Task tk = tasks[blockIdx.x];
   const Node* nodes = tk.nodes;
@@ -662,7 +660,7 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
   __syncthreads();
 
   if (nd.root) {
-    lu_blk(sD, m, LDD, (int32_t*)(fb + nd.fpiv), sl.err, bvals, bidx, &prow);
+    lu_blk(sD, m, LDD, (int32_t*)(fb + nd.fpiv), sl.err, X, s_piv);   // X: BP x XP >= 2 m
     for (int e = tid; e < m * n; e += NT) gD[e] = sD[(e % m) + (e / m) * LDD];
     return;
   }

@@ -10,9 +10,10 @@
 //                       of U to its left (ormql!, :41);
 //   per LQ panel        panel_kernel: 32 rows of D[0:mk, :] reduced (gelqf!, :44), T;
 //                       apply_kernel: on the rows of D below and on V (ormlq!, :47, :50);
-//   finish_kernel       inverses of L1's diagonal blocks; the root's LU (:83).
-// The factor storage is that of ulv_factor_blk_kernel, for nodes of any rank and
-// up to 512 rows.
+//   root_kernel         the root's LU (:83).
+// The factor storage is that of ulv_factor_blk_kernel (without the inverses of L1's
+// diagonal blocks, which only its own solve reads), for nodes of any rank and up to
+// 512 rows.
 //
 // Why so: in one block per node the updates are FP64 multiply-adds at 2 per
 // clock and SM (2.9 of a leaf's 4 M at 128 x 128, k = 32) or, in FP32, one wave
@@ -719,66 +720,33 @@ __global__ void __launch_bounds__(AT, (sizeof(T) == 4 ? 2 : 1))
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(D::tmem));
 }
 
-// ---- last steps of a node ---------------------------------------------------------------
+// ---- roots ------------------------------------------------------------------------------
 
-// Inverses of L1's 32 x 32 diagonal blocks (one warp per block, lane b holds
-// column b); the root's LU with partial pivoting, in shared memory where it fits.
+// The roots' LU with partial pivoting, in shared memory where it fits.
 template <typename T>
-__global__ void __launch_bounds__(NT) finish_kernel(const Task* __restrict__ tasks, const Slot* __restrict__ slots,
-                                                    int smem_rows) {
+__global__ void __launch_bounds__(NT) root_kernel(const Task* __restrict__ tasks, const Slot* __restrict__ slots,
+                                                  int smem_rows) {
   extern __shared__ __align__(16) unsigned char fsm[];
-  __shared__ T bvals[NW];
-  __shared__ int bidx[NW];
-  __shared__ int prow;
+  __shared__ T s_l[2 * 512];
+  __shared__ int s_piv[2];
   const Task tk = tasks[blockIdx.x];
   const Node& nd = tk.nodes[tk.node];
+  if (!nd.root) return;
   const Slot& sl = slots[tk.slot];
   T* fb = (T*)sl.fbase;
   T* gD = fb + nd.fD;
   const int m = nd.m, tid = threadIdx.x;
-  if (nd.root) {
-    int32_t* piv = (int32_t*)(fb + nd.fpiv);
-    if (m > smem_rows) {
-      lu_blk(gD, m, m, piv, sl.err, bvals, bidx, &prow);
-      return;
-    }
-    T* sD = (T*)fsm;
-    const int ld = m | 1;
-    for (int e = tid; e < m * m; e += NT) sD[(e % m) + (e / m) * ld] = gD[e];
-    __syncthreads();
-    lu_blk(sD, m, ld, piv, sl.err, bvals, bidx, &prow);
-    for (int e = tid; e < m * m; e += NT) gD[e] = sD[(e % m) + (e / m) * ld];
+  int32_t* piv = (int32_t*)(fb + nd.fpiv);
+  if (m > smem_rows) {
+    lu_blk(gD, m, m, piv, sl.err, s_l, s_piv);
     return;
   }
-  if (sizeof(T) == 8) return;
-  const int warp = tid >> 5, b = tid & 31;
-  for (int w = warp; w * BP < nd.mk; w += NW) {
-    const int i0 = w * BP, nb = min(BP, nd.mk - i0);
-    const T* L = gD + i0 + (int64_t)i0 * m;
-    T lc[BP], xc[BP];
-#pragma unroll
-    for (int a = 0; a < BP; ++a) xc[a] = T(0);
-    // column by column: x(a) for a > b from the rows above it
-    T r[BP];
-#pragma unroll
-    for (int q = 0; q < BP; ++q) lc[q] = (b < nb && q < nb && q <= b) ? L[b + (int64_t)q * m] : T(0);   // row b of L
-#pragma unroll
-    for (int a = 0; a < BP; ++a) {
-      T s0 = T(0), s1 = T(0);
-#pragma unroll
-      for (int q = 0; q < a; ++q) {
-        const T l = __shfl_sync(0xffffffffu, lc[q], a);
-        if (q & 1) s1 = fma_t(l, xc[q], s1);
-        else s0 = fma_t(l, xc[q], s0);
-      }
-      const T d = __shfl_sync(0xffffffffu, lc[a], a);
-      r[a] = a < nb ? T(1) / d : T(0);
-      xc[a] = a < nb ? (a == b ? r[a] : (a > b ? -(s0 + s1) * r[a] : T(0))) : T(0);
-    }
-    T* out = fb + nd.fLi + (int64_t)w * 1024 + b * BP;
-#pragma unroll
-    for (int a = 0; a < BP; ++a) out[a] = xc[a];
-  }
+  T* sD = (T*)fsm;
+  const int ld = m | 1;
+  for (int e = tid; e < m * m; e += NT) sD[(e % m) + (e / m) * ld] = gD[e];
+  __syncthreads();
+  lu_blk(sD, m, ld, piv, sl.err, s_l, s_piv);
+  for (int e = tid; e < m * m; e += NT) gD[e] = sD[(e % m) + (e / m) * ld];
 }
 
 template <typename T, int S, bool QL, int PL>
@@ -853,18 +821,15 @@ cudaError_t launch_ulv_factor_pan(const Task* t, int64_t nt, const Slot* s, cons
     count(panel<T, false>(t, nt, s, p, d.nmax, sms, st));
     count(apply<T, false>(t, nt, s, p, d.mmax + d.kvmax, st));
   }
-  const int cap = (int)((sizeof(T) == 4 ? 100 : 200) * 1024 / sizeof(T));
-  int rows = 0;
-  if (d.rootmax > 0 && d.rootmax * (d.rootmax | 1) <= cap) rows = d.rootmax;
-  const size_t smem = (size_t)rows * (rows | 1) * sizeof(T);
-  static bool attr_set = false;
-  if (!attr_set) {
-    count(cudaFuncSetAttribute(finish_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cap * sizeof(T))));
-    --*launches;
-    attr_set = true;
-  }
-  if (sizeof(T) == 4 || d.rootmax > 0) {   // the FP64 solve does not use the inverses
-    finish_kernel<T><<<(unsigned)nt, NT, smem, st>>>(t, s, rows);
+  if (d.rootmax > 0) {
+    const int cap = (int)(200 * 1024 / sizeof(T));
+    const int rows = d.rootmax * (d.rootmax | 1) <= cap ? d.rootmax : 0;
+    static bool attr_set = false;
+    if (!attr_set && e == cudaSuccess) {
+      e = cudaFuncSetAttribute(root_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cap * sizeof(T)));
+      attr_set = e == cudaSuccess;
+    }
+    root_kernel<T><<<(unsigned)nt, NT, (size_t)rows * (rows | 1) * sizeof(T), st>>>(t, s, rows);
     count(cudaGetLastError());
   }
   return e;
