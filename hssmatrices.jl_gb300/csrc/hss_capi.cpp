@@ -1126,16 +1126,20 @@ inline bool pick_bsolve(bool blocked, const Seg& g, const std::vector<int8_t>* t
   return use_bsolve(blocked, g);
 }
 
+// pdl: the level's launches may start while the one before them on the stream ends
+// (not the first level's, which may follow the factorization, and not where the
+// level waits for its own factorization on another stream).
 // blocked: the factors come from the blocked FP32 reduction (T = float only);
 // tf: the factor whose tuned choices apply (the plan's own task lists), or null.
 template <typename T>
 void run_solve_up_level(const Levels& L, size_t h, const Slot* slots, int rmax, cudaStream_t st, bool blocked,
-                        const std::vector<int8_t>* tup) {
+                        const std::vector<int8_t>* tup, bool pdl) {
   traced(HSS_TRACE_SOLVE_UP, (*L.by_h)[h].cnt, st, [&] { run_parts(L, (*L.by_h)[h], [&](const Seg& g) {
     if (pick_bsolve(blocked, g, tup, h))
       launch_bsolve_up(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g), rmax, st);
     else if (!g_generic_factor && solve_reg_fits(g.mmax, g.nmax))
-      launch_ulv_solve_up_reg<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.sv_stage, rmax, st);
+      launch_ulv_solve_up_reg<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.sv_stage, g.c1v + g.c2v, rmax,
+                                 sm_count(L.device), st, pdl);
     else
       launch_ulv_solve_up<T>(L.d_tasks + g.off, g.cnt, slots, st);
   }); });
@@ -1150,7 +1154,7 @@ void run_solve(const Levels& L, const Slot* slots, int rmax, cudaStream_t st, bo
                const hss_factor_s* tf = nullptr) {
   const std::vector<int8_t>* tup = tf ? &tf->tune_up : nullptr;
   const std::vector<int8_t>* tdn = tf ? &tf->tune_down : nullptr;
-  for (size_t h = 0; h < L.by_h->size(); ++h) run_solve_up_level<T>(L, h, slots, rmax, st, blocked, tup);
+  for (size_t h = 0; h < L.by_h->size(); ++h) run_solve_up_level<T>(L, h, slots, rmax, st, blocked, tup, h > 0);
   run_solve_down<T>(L, slots, rmax, st, blocked, tdn);
 }
 
@@ -1162,7 +1166,8 @@ void run_solve_down(const Levels& L, const Slot* slots, int rmax, cudaStream_t s
       if (pick_bsolve(blocked, g, tdn, d))
         launch_bsolve_down(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g), rmax, st);
       else if (!g_generic_factor && solve_reg_fits(g.mmax, g.nmax))
-        launch_ulv_solve_down_reg<T>(L.d_tasks + g.off, g.cnt, slots, g.nmax, g.mkmax, rmax, st);
+        launch_ulv_solve_down_reg<T>(L.d_tasks + g.off, g.cnt, slots, g.nmax, g.mkmax, rmax, sm_count(L.device), st,
+                                     d > 0);
       else
         launch_ulv_solve_down<T>(L.d_tasks + g.off, g.cnt, slots, st);
     }); });
@@ -1580,7 +1585,7 @@ cudaError_t factsolve_issue(hss_factor_s* f, const Levels& L, const SlotTable& t
     run_factor_level<T>(L, h, f->fac_slots.dev.p, sf);
     chk(cudaEventRecord(f->pipe_ev[4 + h], sf));
     chk(cudaStreamWaitEvent(s2, f->pipe_ev[4 + h], 0));
-    run_solve_up_level<T>(L, h, table.dev.p, (int)pp.rmax, s2, pp.blocked, &f->tune_up);
+    run_solve_up_level<T>(L, h, table.dev.p, (int)pp.rmax, s2, pp.blocked, &f->tune_up, false);
   }
   chk(cudaEventRecord(f->pipe_ev[2], sf));
   chk(cudaEventRecord(f->pipe_ev[1], s2));

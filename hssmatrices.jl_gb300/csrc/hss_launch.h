@@ -141,15 +141,17 @@ void launch_bsolve_down(const Task* t, int64_t ntasks, const Slot* s, int mmax, 
                         cudaStream_t st);
 // Register-resident solve sweeps for nodes with m, n <= 256 (hss_solve.cu).
 bool solve_reg_fits(int mmax, int nmax);
+// kvs: largest sum of the children's column ranks; pdl: a programmatic dependent of
+// the launch before it (which must itself come after the factorization).
 template <typename T>
-void launch_ulv_solve_up_reg(const Task* t, int64_t ntasks, const Slot* s, int mmax, int64_t stage, int r,
-                             cudaStream_t st);
+void launch_ulv_solve_up_reg(const Task* t, int64_t nt, const Slot* s, int mmax, int64_t stage, int kvs, int r, int sms,
+                             cudaStream_t st, bool pdl);
 // Shared-memory elements the upward solve stages for one node.
 int64_t solve_up_stage_need(int m, int k, int mk, int nk, int kv, bool leaf, bool root, int mr1, int mr2, int kv1,
                             int kv2);
 template <typename T>
-void launch_ulv_solve_down_reg(const Task* t, int64_t ntasks, const Slot* s, int nmax, int mkmax, int r,
-                               cudaStream_t st);
+void launch_ulv_solve_down_reg(const Task* t, int64_t nt, const Slot* s, int nmax, int mkmax, int r, int sms,
+                               cudaStream_t st, bool pdl);
 template <typename T>
 void launch_ulv_solve_up(const Task* t, int64_t ntasks, const Slot* s, cudaStream_t st);
 template <typename T>

@@ -7,6 +7,23 @@
 // solves broadcast each solved entry from its owner lane.  No block-wide
 // barrier sits inside the sequential sweeps.
 //
+// A level is bound by one block's chain, a list of many blocks by the FP64 pipe:
+// * a division is about forty FP64 instructions of 64 clocks on the chain of every
+//   row of a substitution; the diagonal's reciprocals are formed once per block
+//   instead, and a quotient is a product and one correction;
+// * 8 lanes per right-hand side (four per warp) spend 20 FP64 instructions on a
+//   reflector of 64 rows for four right-hand sides, 32 lanes 10 for one: FP64
+//   lists longer than two rounds of the SMs take 8 lanes, shorter ones 32;
+// * a launch after the first of a sweep starts while the level before it ends
+//   (programmatic dependent launch) and copies its factor blocks meanwhile.
+// Measured (one GB300, CUDA events around each launch): n = 65536, k = 32, 32
+// right-hand sides in FP64, leaf level upward 2540 -> 1225 us and downward 1565 ->
+// 983, 256-node level upward 541 -> 295, root 72 -> 45; 1200 unknowns, k = 16 in
+// FP64, a level upward 50 -> 34 us.  FP32, 64 x 64 nodes: upward 26.6 -> 20.5 us a
+// level (16-byte-stride copies without index divisions, no transposed stores), with
+// the overlap of consecutive levels a resident solve of n = 16384 with 4
+// right-hand sides 1020 -> 773 us.
+//
 // Upward pass per node (reference src/ulvfactor.jl:22-57, :74, :89):
 //   b = rhs rows (leaf) or [b1; b2] - [T12 u2; T21 u1] (branch)
 //   b <- Q_ql^T b;  zloc = L1 \ b[0:mk];  b_red = b[mk:m] - L2 zloc;
@@ -17,6 +34,7 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include "hss_factor.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
 
@@ -25,7 +43,15 @@ namespace hss {
 namespace {
 
 constexpr int ST = 256;
-constexpr int LDS = 257;   // odd leading dimension of the shared staging block
+
+// The launch's dependents may be scheduled; wait for the launch it depends on.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// dst (ld ldd) = rows x cols block of src (ld lds), a column per warp; tril: rows
+// from the diagonal on only.
+template <typename T>
+__device__ __forceinline__ void stage_block(T* dst, int ldd, const T* src, int64_t lds, int rows, int cols, bool tril = false);
 
 // Asynchronous element copy global -> shared (cp.async, 4 or 8 bytes): the
 // staging copies of a block are all in flight at once; cpa_wait() waits for
@@ -40,6 +66,23 @@ __device__ __forceinline__ void cpa(T* s, const T* g) {
 }
 __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+template <typename T>
+__device__ __forceinline__ void stage_block(T* dst, int ldd, const T* src, int64_t lds, int rows, int cols, bool tril) {
+  const int lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < cols; c += ST / 32)
+    for (int i = lane + (tril ? c & ~31 : 0); i < rows; i += 32) cpa(dst + i + c * ldd, src + i + (int64_t)c * lds);
+}
+
+// b / d from r = 1 / d: the product and one correction.
+__device__ __forceinline__ float quot(float b, float d, float r) {
+  const float x = b * r;
+  return fmaf(r, fmaf(-d, x, b), x);
+}
+__device__ __forceinline__ double quot(double b, double d, double r) {
+  const double x = b * r;
+  return fma(r, fma(-d, x, b), x);
+}
+
 template <int TPC, typename T>
 __device__ __forceinline__ T gsum(T v) {
 #pragma unroll
@@ -47,9 +90,10 @@ __device__ __forceinline__ T gsum(T v) {
   return v;
 }
 
-// Forward substitution L x = b in registers (L lower, ld ldl, size nr).
+// Forward substitution L x = b in registers (L lower, ld ldl, size nr; rd: the
+// reciprocals of its diagonal).
 template <typename T, int TPC, int RPT, bool UNIT>
-__device__ __forceinline__ void lower_solve(T (&b)[RPT], const T* __restrict__ L, int ldl, int nr, int gl) {
+__device__ __forceinline__ void lower_solve(T (&b)[RPT], const T* __restrict__ L, int ldl, int nr, int gl, const T* rd) {
 #pragma unroll
   for (int s = 0; s < RPT; ++s) {
     if (s * TPC >= nr) break;
@@ -57,7 +101,7 @@ __device__ __forceinline__ void lower_solve(T (&b)[RPT], const T* __restrict__ L
       const int c = s * TPC + o;
       if (c >= nr) break;
       const T bc = __shfl_sync(0xffffffffu, b[s], o, TPC);
-      const T xc = UNIT ? bc : bc / L[c + (int64_t)c * ldl];
+      const T xc = UNIT ? bc : quot(bc, L[c + (int64_t)c * ldl], rd[c]);
       if (gl == o) b[s] = xc;
 #pragma unroll
       for (int s2 = s; s2 < RPT; ++s2) {
@@ -70,7 +114,7 @@ __device__ __forceinline__ void lower_solve(T (&b)[RPT], const T* __restrict__ L
 
 // Backward substitution U x = b (U upper, non-unit).
 template <typename T, int TPC, int RPT>
-__device__ __forceinline__ void upper_solve(T (&b)[RPT], const T* __restrict__ A, int lda, int nr, int gl) {
+__device__ __forceinline__ void upper_solve(T (&b)[RPT], const T* __restrict__ A, int lda, int nr, int gl, const T* rd) {
 #pragma unroll
   for (int s = RPT - 1; s >= 0; --s) {
     if (s * TPC >= nr) continue;
@@ -78,7 +122,7 @@ __device__ __forceinline__ void upper_solve(T (&b)[RPT], const T* __restrict__ A
       const int c = s * TPC + o;
       if (c >= nr) continue;
       const T bc = __shfl_sync(0xffffffffu, b[s], o, TPC);
-      const T xc = bc / A[c + (int64_t)c * lda];
+      const T xc = quot(bc, A[c + (int64_t)c * lda], rd[c]);
       if (gl == o) b[s] = xc;
 #pragma unroll
       for (int s2 = 0; s2 <= s; ++s2) {
@@ -90,16 +134,15 @@ __device__ __forceinline__ void upper_solve(T (&b)[RPT], const T* __restrict__ A
 }
 
 // Elements of shared memory the upward kernel stages for one node (beyond the
-// LDS x CPB right-hand-side block); the host sizes launches with the level's
-// largest value.
+// right-hand sides); the host sizes launches with the level's largest value.
 __host__ __device__ inline int64_t solve_up_stage_elems(int m, int k, int mk, int nk, int kv, bool leaf, bool root,
                                                        int mr1, int mr2, int kv1, int kv2, int cpb) {
   int64_t e = 0;
   if (root) e += (int64_t)m * m;
-  else if (mk > 0) e += (int64_t)m * k + (int64_t)mk * mk + (int64_t)k * nk + (int64_t)nk * kv;
+  else if (mk > 0) e += (int64_t)m * k + (int64_t)mk * mk + (int64_t)k * nk + (int64_t)(nk | 1) * kv;
   if (!leaf) {
     e += (int64_t)mr1 * kv2 + (int64_t)mr2 * kv1 + (int64_t)(kv1 + kv2) * cpb;
-    if (!root) e += (int64_t)(kv1 + kv2) * kv;
+    if (!root) e += (int64_t)((kv1 | 1) + (kv2 | 1)) * kv;
   }
   return e;
 }
@@ -110,9 +153,12 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
                                                        int nchunk) {
   constexpr int RPT = MR / TPC;
   constexpr int CPB = ST / TPC;
+  constexpr int LDS = MR + 1;
   extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ T s_rd[MR];      // reciprocals of the diagonal that is solved with
   T* sb = (T*)smraw;          // LDS x CPB right-hand sides
   T* sx = sb + LDS * CPB;     // staged operands
+  pdl_trigger();
   const Task tk = tasks[blockIdx.x / nchunk];
   const int jchunk = (blockIdx.x % nchunk) * CPB;   // this block's columns: jchunk .. jchunk+CPB-1
   const Node* nodes = tk.nodes;
@@ -122,7 +168,10 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
   const int64_t ld = sl.ldws;
   const T* fb = (const T*)sl.fbase;
   const int m = nd.m, n = nd.n, kv = nd.kv, r = sl.r;
-  if (jchunk >= r) return;
+  if (jchunk >= r) {
+    pdl_wait();
+    return;
+  }
   const int tid = threadIdx.x, g = tid / TPC, gl = tid % TPC;
   const int k = nd.k, mk = nd.mk, nk = nd.nk;
   T* u = ws + nd.wu;
@@ -141,53 +190,56 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
   const T* T12p = nd.leaf ? nullptr : fb + nd.fT12;   // mr1 x kv2
   const T* T21p = nd.leaf ? nullptr : fb + nd.fT21;   // mr2 x kv1
   T* sW1 = nullptr;  T* sW2 = nullptr;  T* su1 = nullptr;  T* su2 = nullptr;
+  int ldW1 = 0, ldW2 = 0;
   if (staged) {
     T* p = sx;
     if (nd.root) {
-      for (int e = tid; e < m * m; e += ST) cpa(p + e, Lp + e);
+      stage_block(p, m, Lp, m, m, m);
       Lp = p; ldL = m; p += m * m;
     } else if (mk > 0) {
-      T* q = p;
-      for (int e = tid; e < m * k; e += ST) cpa(q + e, Up + e);
-      Up = q; ldU = m; q += m * k;
-      for (int e = tid; e < mk * mk; e += ST) cpa(q + e, Lp + (e % mk) + (int64_t)(e / mk) * m);
-      Lp = q; ldL = mk; q += mk * mk;
-      for (int e = tid; e < k * nk; e += ST) cpa(q + e, L2p + (e % k) + (int64_t)(e / k) * m);
-      L2p = q; ldL2 = k; q += k * nk;
-      // V[0:nk, :] transposed (element (l, c) at c + l*kv): consecutive threads read consecutive c
-      for (int e = tid; e < nk * kv; e += ST) cpa(q + (e / nk) + (e % nk) * kv, Vap + (e % nk) + (int64_t)(e / nk) * n);
-      Vap = q; ldVa = -1; q += nk * kv;
-      p = q;
+      stage_block(p, m, Up, m, m, k);
+      Up = p; ldU = m; p += m * k;
+      stage_block(p, mk, Lp, m, mk, mk, true);
+      Lp = p; ldL = mk; p += mk * mk;
+      stage_block(p, k, L2p, m, k, nk);
+      L2p = p; ldL2 = k; p += k * nk;
+      ldVa = nk | 1;   // odd: consecutive threads read consecutive columns
+      stage_block(p, ldVa, Vap, n, nk, kv);
+      Vap = p; p += ldVa * kv;
     }
     if (!nd.leaf) {
-      for (int e = tid; e < mr1 * kv2; e += ST) cpa(p + e, T12p + e);
+      stage_block(p, mr1, T12p, mr1, mr1, kv2);
       T12p = p; p += mr1 * kv2;
-      for (int e = tid; e < mr2 * kv1; e += ST) cpa(p + e, T21p + e);
+      stage_block(p, mr2, T21p, mr2, mr2, kv1);
       T21p = p; p += mr2 * kv1;
       if (!nd.root) {
-        sW1 = p; p += kv1 * kv;
-        sW2 = p; p += kv2 * kv;
-        // W1, W2 transposed (element (l, c) at c + l*kv)
-        // (converted from the FP64 generators: register loads, four in flight per thread)
-        auto stage_w = [&](T* dst, const double* src, int kc) {
-          for (int e0 = tid; e0 < kc * kv; e0 += 4 * ST) {
-            double w[4];
+        ldW1 = kv1 | 1; ldW2 = kv2 | 1;
+        sW1 = p; p += ldW1 * kv;
+        sW2 = p; p += ldW2 * kv;
+        // (converted from the FP64 generators: register loads, eight in flight per lane)
+        auto stage_w = [&](T* dst, int ldd, const double* src, int kc) {
+          const int lane = tid & 31;
+          for (int c0 = tid >> 5; c0 < kv; c0 += 8 * (ST / 32))
+            for (int i = lane; i < kc; i += 32) {
+              double w[8];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) w[q] = e0 + q * ST < kc * kv ? __ldg(src + e0 + q * ST) : 0.0;
+              for (int q = 0; q < 8; ++q)
+                w[q] = c0 + q * (ST / 32) < kv ? __ldg(src + i + (int64_t)(c0 + q * (ST / 32)) * kc) : 0.0;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int e = e0 + q * ST;
-              if (e < kc * kv) dst[(e / kc) + (e % kc) * kv] = (T)w[q];
+              for (int q = 0; q < 8; ++q)
+                if (c0 + q * (ST / 32) < kv) dst[i + (c0 + q * (ST / 32)) * ldd] = (T)w[q];
             }
-          }
         };
-        stage_w(sW1, nd.W1, kv1);
-        stage_w(sW2, nd.W2, kv2);
+        stage_w(sW1, ldW1, nd.W1, kv1);
+        stage_w(sW2, ldW2, nd.W2, kv2);
       }
       su1 = p; p += kv1 * CPB;
       su2 = p; p += kv2 * CPB;
     }
   }
+  // (from the factor storage itself: the staged copy is still on its way)
+  for (int i = tid; i < (nd.root ? m : mk); i += ST) s_rd[i] = fac::recip(fb[nd.fD + i + (int64_t)i * m]);
+  pdl_wait();   // what follows reads the level before
   for (int j0 = jchunk; j0 < jchunk + CPB && j0 < r; j0 += CPB) {
     const int ncol = min(CPB, r - j0);
     // ---- gather b for this chunk of columns into shared memory
@@ -255,8 +307,8 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
           T s = T(0);
           if (staged) {
             T s1 = T(0);
-            for (int l = 0; l < kv1; ++l) s += sW1[c + l * kv] * a1[l];
-            for (int l = 0; l < kv2; ++l) s1 += sW2[c + l * kv] * a2[l];
+            for (int l = 0; l < kv1; ++l) s += sW1[l + c * ldW1] * a1[l];
+            for (int l = 0; l < kv2; ++l) s1 += sW2[l + c * ldW2] * a2[l];
             s += s1;
           } else {
             for (int l = 0; l < kv1; ++l) s += (T)nd.W1[l + (int64_t)c * kv1] * a1[l];
@@ -286,8 +338,8 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
         const int row = gl + s * TPC;
         b[s] = row < m ? sb[row + g * LDS] : T(0);
       }
-      lower_solve<T, TPC, RPT, true>(b, A, ldL, m, gl);
-      upper_solve<T, TPC, RPT>(b, A, ldL, m, gl);
+      lower_solve<T, TPC, RPT, true>(b, A, ldL, m, gl, s_rd);
+      upper_solve<T, TPC, RPT>(b, A, ldL, m, gl, s_rd);
       if (j < r) {
         T* x = ws + nd.wx + (int64_t)j * ld;
 #pragma unroll
@@ -309,8 +361,7 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
       }
       // b <- Q_ql^T b (src/ulvfactor.jl:42), reflectors in generation order
       for (int c = k - 1; c >= 0; --c) {
-        const T tau = tq[c];
-        if (tau == T(0)) continue;
+        const T tau = tq[c];   // 0: the reflector leaves b as it is
         const int p = mk + c;
         const T* v = Up + (int64_t)c * ldU;
         T d0 = T(0), d1 = T(0);
@@ -330,7 +381,7 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
         }
       }
       // zloc = L1 \ b[0:mk] (trsm, src/ulvfactor.jl:48)
-      lower_solve<T, TPC, RPT, false>(b, Lp, ldL, mk, gl);
+      lower_solve<T, TPC, RPT, false>(b, Lp, ldL, mk, gl, s_rd);
 #pragma unroll
       for (int s = 0; s < RPT; ++s) {
         const int row = gl + s * TPC;
@@ -355,16 +406,12 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
       const int c = e % kv, gg = e / kv;
       const T* bb = sb + gg * LDS;
       T s0 = nd.leaf ? T(0) : u[c + (int64_t)(j0 + gg) * ld], s1 = T(0);
-      if (ldVa < 0) {   // staged transposed
-        int l = 0;
-        for (; l + 1 < nk; l += 2) {
-          s0 += Vap[c + l * kv] * bb[l];
-          s1 += Vap[c + (l + 1) * kv] * bb[l + 1];
-        }
-        if (l < nk) s0 += Vap[c + l * kv] * bb[l];
-      } else {
-        for (int l = 0; l < nk; ++l) s0 += Vap[l + c * ldVa] * bb[l];
+      int l = 0;
+      for (; l + 1 < nk; l += 2) {
+        s0 += Vap[l + c * ldVa] * bb[l];
+        s1 += Vap[l + 1 + c * ldVa] * bb[l + 1];
       }
+      if (l < nk) s0 += Vap[l + c * ldVa] * bb[l];
       u[c + (int64_t)(j0 + gg) * ld] = s0 + s1;
     }
     for (int e = tid; e < mk * ncol; e += ST) {
@@ -392,7 +439,11 @@ __global__ void __launch_bounds__(ST) ulv_solve_down_reg(const Task* __restrict_
   const int64_t ld = sl.ldws;
   const T* fb = (const T*)sl.fbase;
   const int n = nd.n, r = sl.r;
-  if (jchunk >= r) return;
+  pdl_trigger();
+  if (jchunk >= r) {
+    pdl_wait();
+    return;
+  }
   const int tid = threadIdx.x, g = tid / TPC, gl = tid % TPC;
   const T* x = ws + nd.wx;
   const T* Qt = fb + nd.fQt;
@@ -402,6 +453,7 @@ __global__ void __launch_bounds__(ST) ulv_solve_down_reg(const Task* __restrict_
     cpa_wait();
     __syncthreads();
   }
+  pdl_wait();   // what follows reads the level before
   for (int j0 = jchunk; j0 < jchunk + CPB && j0 < r; j0 += CPB) {
     const int j = j0 + g;
     const bool act = j < r;
@@ -416,8 +468,7 @@ __global__ void __launch_bounds__(ST) ulv_solve_down_reg(const Task* __restrict_
       const T* tl = fb + nd.ftl;
       const int nl = min(nd.mk, n);
       for (int i = nl - 1; i >= 0; --i) {
-        const T tau = tl[i];
-        if (tau == T(0)) continue;
+        const T tau = tl[i];   // 0: the reflector leaves b as it is
         const T* v = Qt + (int64_t)i * n;
         T d0 = T(0), d1 = T(0);
 #pragma unroll
@@ -464,9 +515,26 @@ __global__ void __launch_bounds__(ST) ulv_solve_down_reg(const Task* __restrict_
 
 constexpr size_t kSolveSmemCap = 200 * 1024;
 
+// A launch of ST threads per block, as a programmatic dependent of the one before
+// it on the stream where pdl is set.
+template <typename K, typename... A>
+void launch_st(K kernel, int64_t blocks, size_t smem, cudaStream_t st, bool pdl, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(ST);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 template <typename T, int TPC, int MR>
-void up_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, cudaStream_t st) {
-  const size_t base = (size_t)LDS * (ST / TPC) * sizeof(T);
+void up_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, cudaStream_t st, bool pdl) {
+  const size_t base = (size_t)(MR + 1) * (ST / TPC) * sizeof(T);
   size_t smem = base + want * sizeof(T);
   if (smem > kSolveSmemCap) smem = base;   // operands stay in global memory
   static bool set = false;
@@ -476,12 +544,11 @@ void up_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, 
     set = true;
   }
   const int nchunk = (rmax + ST / TPC - 1) / (ST / TPC);
-  ulv_solve_up_reg<T, TPC, MR><<<(unsigned)(nt * nchunk), ST, smem, st>>>(t, s, (int64_t)((smem - base) / sizeof(T)),
-                                                                          nchunk);
+  launch_st(ulv_solve_up_reg<T, TPC, MR>, nt * nchunk, smem, st, pdl, t, s, (int64_t)((smem - base) / sizeof(T)), nchunk);
 }
 
 template <typename T, int TPC, int MR>
-void down_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, cudaStream_t st) {
+void down_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, cudaStream_t st, bool pdl) {
   size_t smem = want * sizeof(T);
   if (smem > kSolveSmemCap) smem = 0;
   static bool set = false;
@@ -491,7 +558,14 @@ void down_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax
     set = true;
   }
   const int nchunk = (rmax + ST / TPC - 1) / (ST / TPC);
-  ulv_solve_down_reg<T, TPC, MR><<<(unsigned)(nt * nchunk), ST, smem, st>>>(t, s, (int)(smem / sizeof(T)), nchunk);
+  launch_st(ulv_solve_down_reg<T, TPC, MR>, nt * nchunk, smem, st, pdl, t, s, (int)(smem / sizeof(T)), nchunk);
+}
+
+// 8 lanes per right-hand side: FP64 lists longer than two rounds of the SMs with
+// at least 16 right-hand sides (32 to a block).
+template <typename T>
+bool narrow_groups(int64_t nt, int r, int sms) {
+  return sizeof(T) == 8 && r >= 16 && nt * ((r + 7) / 8) > 2 * sms;
 }
 
 }  // namespace
@@ -503,31 +577,48 @@ int64_t solve_up_stage_need(int m, int k, int mk, int nk, int kv, bool leaf, boo
   return solve_up_stage_elems(m, k, mk, nk, kv, leaf, root, mr1, mr2, kv1, kv2, ST / 32);
 }
 
-// One warp per right-hand-side column, 8 columns per thread block; the grid
-// covers (node, column chunk) pairs so that few-node levels still fill SMs.
+// One warp (or a quarter of one) per right-hand-side column; the grid covers
+// (node, column chunk) pairs so that few-node levels still fill SMs.
 template <typename T>
-void launch_ulv_solve_up_reg(const Task* t, int64_t nt, const Slot* s, int mmax, int64_t stage, int r,
-                             cudaStream_t st) {
+void launch_ulv_solve_up_reg(const Task* t, int64_t nt, const Slot* s, int mmax, int64_t stage, int kvs, int r, int sms,
+                             cudaStream_t st, bool pdl) {
   if (nt <= 0 || r <= 0) return;
   const size_t want = (size_t)stage;
-  if (mmax <= 64) up_launch<T, 32, 64>(t, nt, s, want, r, st);
-  else if (mmax <= 128) up_launch<T, 32, 128>(t, nt, s, want, r, st);
-  else up_launch<T, 32, 256>(t, nt, s, want, r, st);
+  if constexpr (sizeof(T) == 8) {
+    if (narrow_groups<T>(nt, r, sms) && mmax <= 128) {
+      const size_t more = want + (size_t)kvs * (ST / 8 - ST / 32);   // the children's u of 32 columns
+      if (mmax <= 64) up_launch<T, 8, 64>(t, nt, s, more, r, st, pdl);
+      else up_launch<T, 8, 128>(t, nt, s, more, r, st, pdl);
+      return;
+    }
+  }
+  if (mmax <= 64) up_launch<T, 32, 64>(t, nt, s, want, r, st, pdl);
+  else if (mmax <= 128) up_launch<T, 32, 128>(t, nt, s, want, r, st, pdl);
+  else up_launch<T, 32, 256>(t, nt, s, want, r, st, pdl);
 }
 
 template <typename T>
-void launch_ulv_solve_down_reg(const Task* t, int64_t nt, const Slot* s, int nmax, int mkmax, int r,
-                               cudaStream_t st) {
+void launch_ulv_solve_down_reg(const Task* t, int64_t nt, const Slot* s, int nmax, int mkmax, int r, int sms,
+                               cudaStream_t st, bool pdl) {
   if (nt <= 0 || r <= 0) return;
   const size_t want = (size_t)nmax * mkmax;
-  if (nmax <= 64) down_launch<T, 32, 64>(t, nt, s, want, r, st);
-  else if (nmax <= 128) down_launch<T, 32, 128>(t, nt, s, want, r, st);
-  else down_launch<T, 32, 256>(t, nt, s, want, r, st);
+  if constexpr (sizeof(T) == 8) {
+    if (narrow_groups<T>(nt, r, sms) && nmax <= 128) {
+      if (nmax <= 64) down_launch<T, 8, 64>(t, nt, s, want, r, st, pdl);
+      else down_launch<T, 8, 128>(t, nt, s, want, r, st, pdl);
+      return;
+    }
+  }
+  if (nmax <= 64) down_launch<T, 32, 64>(t, nt, s, want, r, st, pdl);
+  else if (nmax <= 128) down_launch<T, 32, 128>(t, nt, s, want, r, st, pdl);
+  else down_launch<T, 32, 256>(t, nt, s, want, r, st, pdl);
 }
 
-template void launch_ulv_solve_up_reg<double>(const Task*, int64_t, const Slot*, int, int64_t, int, cudaStream_t);
-template void launch_ulv_solve_up_reg<float>(const Task*, int64_t, const Slot*, int, int64_t, int, cudaStream_t);
-template void launch_ulv_solve_down_reg<double>(const Task*, int64_t, const Slot*, int, int, int, cudaStream_t);
-template void launch_ulv_solve_down_reg<float>(const Task*, int64_t, const Slot*, int, int, int, cudaStream_t);
+template void launch_ulv_solve_up_reg<double>(const Task*, int64_t, const Slot*, int, int64_t, int, int, int, cudaStream_t,
+                                              bool);
+template void launch_ulv_solve_up_reg<float>(const Task*, int64_t, const Slot*, int, int64_t, int, int, int, cudaStream_t,
+                                             bool);
+template void launch_ulv_solve_down_reg<double>(const Task*, int64_t, const Slot*, int, int, int, int, cudaStream_t, bool);
+template void launch_ulv_solve_down_reg<float>(const Task*, int64_t, const Slot*, int, int, int, int, cudaStream_t, bool);
 
 }  // namespace hss
