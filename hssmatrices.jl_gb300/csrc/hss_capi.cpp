@@ -114,6 +114,7 @@ struct Seg {
   int c1mr = 0, c2mr = 0, c1nr = 0, c2nr = 0;      // largest children's reduced sizes
   int64_t sv_stage = 0;                            // largest upward-solve staging need
   int mk_in = 0, rootmax = 0;                      // largest m - k of the nodes that are not roots; largest root
+  int smin = INT32_MAX;                            // smallest node: its larger side
   bool leaves = false, branches = false;           // kinds of node in the list
   std::vector<Seg> parts;                          // the list by size of node (empty: one size class)
 };
@@ -128,6 +129,7 @@ inline int size_class(const Node& x) {
 // Counts node x (children in `nodes`) into the largest sizes of a list.
 inline void seg_add(Seg& v, const Node& x, const Node* nodes) {
   ++v.cnt;
+  v.smin = std::min(v.smin, std::max(x.m, x.n));
   v.mmax = std::max(v.mmax, x.m);
   v.nmax = std::max(v.nmax, x.n);
   v.kumax = std::max(v.kumax, x.ku);
@@ -1040,7 +1042,7 @@ inline size_t factor_extra(const Seg& g) {
 
 template <typename T>
 bool factor_level_blk(const Seg& g) {
-  return factor_blk_fits<T>(g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g));
+  return sizeof(T) == 4 && factor_blk_fits<float>(g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g));
 }
 // Levels reduced by panels with the block updates on the tensor cores.  FP64: all
 // that fit (n = 65536, k = 32: 12.6 -> 5.8 ms; 256-row leaves, k = 40: 10.2 -> 5.9;
@@ -1063,11 +1065,11 @@ bool factor_level_fast(const Seg& g) {
 // leaf level with 64-, 128- and 256-row leaves in one launch has the layout of the
 // largest; in a batch of 48 matrices 4.0 -> 3.5 ms for its factorization, 0.82 ->
 // 0.64 ms for its upward solve, 1.11 -> 0.86 ms for the first merges), a shorter one
-// by one block's latency, which each class would add.
+// by one block's latency, which each class would add.  split: by class in any case.
 template <class F>
-void run_parts(const Levels& L, const Seg& g, F&& f) {
+void run_parts(const Levels& L, const Seg& g, F&& f, bool split = false) {
   const int sms = sm_count(L.device);
-  if (g.parts.empty() || g.cnt <= 2 * sms) {
+  if (g.parts.empty() || (!split && g.cnt <= 2 * sms)) {
     f(g);
     return;
   }
@@ -1089,7 +1091,8 @@ bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t
         launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
         add_launches(launches - 1);
       } else if (factor_level_fast<T>(g)) {
-        launch_ulv_factor_blk<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g), st);
+        launch_ulv_factor_blk<float>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax,
+                                     factor_extra(g), st, h > 0);
       } else {
         launch_ulv_factor<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, st);
       }
@@ -1111,19 +1114,25 @@ inline int seg_kvmax(const Seg& g) { return std::max({g.kvmax, g.c1v, g.c2v, 1})
 
 // The blocked solve (GEMM steps, one block per 32 right-hand sides) wins on
 // levels of large nodes; the register kernels (one warp per right-hand side)
-// win on levels of small nodes (64 x 64 merges, the root).
+// win on levels of small nodes (64 x 64 merges, the root), whose factors do not
+// carry what the blocked one reads: a list that has both is run by size class
+// (a class never crosses 64 rows).
 inline bool use_bsolve(bool blocked, const Seg& g) {
-  return blocked && std::max(g.mmax, g.nmax) > 64 && bsolve_fits(g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g));
+  return blocked && g.smin > 64 && bsolve_fits(g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g));
 }
 
 // Kernel of one solve level: the autotuner's forced choice, else the factor's
 // tuned choice (tuned[level] of the plan's own lists), else the rule above.
 inline bool pick_bsolve(bool blocked, const Seg& g, const std::vector<int8_t>* tuned, size_t level) {
-  const bool eligible = blocked && bsolve_fits(g.mmax, g.nmax, seg_kmax(g), seg_kvmax(g));
+  const bool eligible = use_bsolve(blocked, g);
   if (!eligible) return false;
   if (g_pick_force >= 0) return g_pick_force == 1;
   if (tuned && level < tuned->size() && (*tuned)[level] >= 0) return (*tuned)[level] == 1;
   return use_bsolve(blocked, g);
+}
+
+inline bool solve_split(bool blocked, const Seg& g) {
+  return blocked && g.smin <= 64 && std::max(g.mmax, g.nmax) > 64;
 }
 
 // pdl: the level's launches may start while the one before them on the stream ends
@@ -1142,7 +1151,7 @@ void run_solve_up_level(const Levels& L, size_t h, const Slot* slots, int rmax, 
                                  sm_count(L.device), st, pdl);
     else
       launch_ulv_solve_up<T>(L.d_tasks + g.off, g.cnt, slots, st);
-  }); });
+  }, solve_split(blocked, (*L.by_h)[h])); });
 }
 
 template <typename T>
@@ -1170,7 +1179,7 @@ void run_solve_down(const Levels& L, const Slot* slots, int rmax, cudaStream_t s
                                      d > 0);
       else
         launch_ulv_solve_down<T>(L.d_tasks + g.off, g.cnt, slots, st);
-    }); });
+    }, solve_split(blocked, (*L.by_d)[d])); });
   }
 }
 

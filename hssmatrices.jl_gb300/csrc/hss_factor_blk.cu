@@ -1,9 +1,9 @@
-// Blocked ULV reduction of one node per thread block, FP32 or FP64, for nodes
+// Blocked ULV reduction of one node per thread block, FP32, for nodes
 // up to 128 x 128 with ranks up to 64 (every node of the leafsize-128 and
 // leafsize-64 workloads).  Restated from src/ulvfactor.jl:22-57 (the leaf
 // reduction) and :74-79 (the merge), with the reference's reflector order:
 //
-//   P0  load the leaf's D and U (FP64 -> T) or assemble the merged block of the
+//   P0  load the leaf's D and U (FP64 -> FP32) or assemble the merged block of the
 //       children (D, U in shared memory; V = [V1 W1; V2 W2], T12, T21 to global);
 //   P1  QL of U (geqlf!, :39) by panels of 32 columns from the last: inside a
 //       panel every reflector is generated and applied one at a time (8 lanes per
@@ -15,23 +15,24 @@
 //       to the rows below it, C <- C - (C Y^T) T Y (ormlq!, :47), and to V,
 //       V <- V - Y^T T^T Y V (ormlq!('L', 'N'), :50).
 //
-// FP32 nodes of at most 64 x 64 with a single QL and a single LQ panel (the
-// merges of rank-32 children) skip the block updates instead: each reflector
-// is applied to D (QL) or to D's trailing rows and V (LQ) in the panel loop
-// itself, as it is generated; T and the L1 inverses are still stored.
+// Launches whose nodes are all at most 64 x 64 (the merges of rank-32 children)
+// skip the block updates: each reflector is applied to D (QL) or to D's
+// trailing rows and V (LQ) in the panel loop itself, as soon as the barrier of
+// that reflector opens, and neither T nor the L1 inverses are formed (the
+// register solves, which run such nodes, read neither).
 //
 // Y is never copied for the QL panels: it is read from the panel's columns of
 // U (entries above the pivot, an implicit 1 at the pivot, zeros below); the LQ
 // panel is copied reflector-major (rows of D are strided in shared memory).
 // Each GEMM streams C in chunks of 64 columns (rows), so that an FP32 leaf
-// needs about 110 KB of shared memory and two leaves run on an SM at once
-// (FP64: about 220 KB, one per SM).  Global loads (the leaf's generators, the
+// needs about 110 KB of shared memory and two leaves run on an SM at once.  Global loads (the leaf's generators, the
 // children's reduced blocks of a merge) are issued 16 per thread at a time.
 //
 // Outputs (factor storage, precision T): D (L1, LQ reflectors, L2, reduced D),
 // U (QL reflectors + reduced U), V, the two tau vectors, the LQ reflectors
-// transposed (Qt, n x mk), per panel the compact-WY T (32 x 32) of the QL and
-// LQ reflectors, and the inverses of L1's 32 x 32 diagonal blocks.  The root
+// transposed (Qt, n x mk) and, above 64 rows, per panel the compact-WY T (32 x
+// 32) of the QL and LQ reflectors, and the inverses of L1's 32 x 32 diagonal
+// blocks.  The root
 // gets an LU with partial pivoting in shared memory (src/ulvfactor.jl:83).
 #include <cuda_runtime.h>
 
@@ -43,6 +44,7 @@
 #include "hss_factor.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_oz.cuh"
 
 namespace hss {
 
@@ -549,6 +551,8 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
                           int extra) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ int s_piv[2];
+  __shared__ __align__(8) uint64_t s_bar[2][BP];
+  __shared__ T s_tau[2][BP];
   const BlkLayout Lo(S, kumax, kvmax, (size_t)extra);
   const Task tk = tasks[blockIdx.x];
   const Node* nodes = tk.nodes;
@@ -572,9 +576,11 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
   T* gU = fb + nd.fU;
   T* gV = fb + nd.fV;
   const int tid = threadIdx.x, lane = tid & 31;
+  asm volatile("griddepcontrol.launch_dependents;");
 
   // ---- P0: load or assemble ---------------------------------------------------
   if (nd.leaf) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     stage_cols(sD, LDD, nd.D, m, m, n);
     if (!nd.root) {
       stage_cols(sW, LDU, nd.U, m, m, ku);
@@ -616,6 +622,8 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
         default: break;
       }
       if (w < 6) stage_warp(sm, G64);
+      // the generators do not depend on the level below, which may still run
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       CopyJob<T> J{nullptr, 0, 0, 0, 0, 0, 0};
       const int wc = (w + 6) % NW;   // warps 6 and 7 take the first of these, the others follow
       switch (wc) {
@@ -678,30 +686,65 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
   const int g = tid >> 3, l8 = tid & 7;            // panel column / row g, lane l8 of its group
   const unsigned gm = 0xFFu << (lane & 24);        // the group's 8 lanes
 
-  if constexpr (S == 64 && sizeof(T) == sizeof(float)) {
+  if constexpr (S <= 64) {
     if (k <= BP && ku <= BP && mk <= BP && m - mk <= BP && kv <= BP) {
-      // FP32 nodes of at most 64 x 64 with one QL and one LQ panel (the merges
-      // of rank-32 children; FP64 keeps the block updates, measured faster on
-      // its slower FMA pipe): every reflector is applied, as soon as it is
-      // generated, to everything it acts on, each column (row) held in
-      // registers by a group of 8 lanes, one barrier per reflector.  QL: the
-      // U panel and D's columns (two per group); LQ: the panel rows, D's rows
-      // below them and V's columns (one each per group).  This replaces the
-      // panels' block updates (shared-memory GEMMs after the panel loops); the
-      // panels' T matrices and the L1 block inverses are still formed and
-      // stored for the blocked solve, so the factor storage is the same.
+      // Nodes of at most 64 x 64 with one QL and one LQ panel (the merges of children
+      // of rank up to 32): every reflector is applied, as soon as it is there, to
+      // everything it acts on, each column (row) held in registers by a group of 8
+      // lanes.  QL: the U panel and D's columns (two per group); LQ: the panel rows,
+      // D's rows below them and V's columns (one each per group).  A reflector is
+      // published in shared memory with an mbarrier of its own: the chain is its
+      // owner's apply and generate, 32 times, and the other warps follow at their own
+      // pace (a block barrier per reflector held the owner back for D and V: 98
+      // against 75 us a level of 64 x 64 nodes, 57 against 35 of 32 x 32).  The panels' T matrices and L1's block
+      // inverses are not formed: the solve of such nodes is the register kernel.
+      if (tid < 2 * BP) oz::mbar_init(&s_bar[tid / BP][tid % BP]);
+      asm volatile("fence.mbarrier_init.release.cluster;");
+      __syncthreads();
+      const int w0 = tid / 32 * 4;   // the warp's first group
+      bool ok = true;
       auto refl = [&](T(&x)[PE], const T(&vv)[PE], T tau) {
-        T w0 = T(0), w1 = T(0);
+        T a0 = T(0), a1 = T(0);
 #pragma unroll
         for (int t = 0; t < PE; t += 2) {
-          w0 = fma_t(vv[t], x[t], w0);
-          w1 = fma_t(vv[t + 1], x[t + 1], w1);
+          a0 = fma_t(vv[t], x[t], a0);
+          a1 = fma_t(vv[t + 1], x[t + 1], a1);
         }
-        const T w = gsum8(w0 + w1, gm) * tau;
+        const T w = gsum8(a0 + a1, gm) * -tau;
 #pragma unroll
-        for (int t = 0; t < PE; ++t) x[t] = fma_t(-w, vv[t], x[t]);
+        for (int t = 0; t < PE; ++t) x[t] = fma_t(w, vv[t], x[t]);
       };
-      // ---- QL of U (geqlf!, :39), applied to D (ormql!, :41) ----
+      // the group that holds reflector a makes it: pivot entry pv, the tail before it
+      // (QL, ph = 0) or behind it (LQ, ph = 1)
+      auto gen = [&](T(&x)[PE], int a, int pv, int ph, T* Y, T* taus) {
+        auto in = [&](int i) { return ph == 0 ? i < pv : i > pv; };
+        T sq[4] = {T(0), T(0), T(0), T(0)}, mine = T(0);
+#pragma unroll
+        for (int t = 0; t < PE; ++t) {
+          const int i = l8 + PL * t;
+          if (in(i)) sq[t & 3] = fma_t(x[t], x[t], sq[t & 3]);
+          if (i == pv) mine = x[t];
+        }
+        const T ss = gsum8((sq[0] + sq[1]) + (sq[2] + sq[3]), gm);
+        const T alpha = __shfl_sync(gm, mine, (lane & 24) | (pv & 7));
+        T beta, tau, sc;
+        larfg_t(alpha, ss, beta, tau, sc);
+#pragma unroll
+        for (int t = 0; t < PE; ++t) {
+          const int i = l8 + PL * t;
+          if (in(i)) x[t] *= sc;   // 1 where tau is 0
+          Y[i] = in(i) ? x[t] : (i == pv ? T(1) : T(0));
+          if (i == pv) x[t] = beta;
+        }
+        if (l8 == 0) {
+          s_tau[ph][a] = tau;
+          taus[a] = tau;
+        }
+        __syncwarp(gm);
+        if (l8 == 0)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(oz::smem_u32(&s_bar[ph][a])) : "memory");
+      };
+      // ---- QL of U (geqlf!, :39), applied to D (ormql!, :41); reflectors in X ----
       {
         T u[PE], dq0[PE], dq1[PE];
 #pragma unroll
@@ -711,66 +754,43 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
           dq0[t] = (g < n && row < m) ? sD[row + g * LDD] : T(0);
           dq1[t] = (g + BP < n && row < m) ? sD[row + (g + BP) * LDD] : T(0);
         }
-        auto gen = [&](int c, int buf) {   // the 8 lanes of column c
-          const int p = mk + c;
-          T sq[4] = {T(0), T(0), T(0), T(0)}, mine = T(0);
-#pragma unroll
-          for (int t = 0; t < PE; ++t) {
-            const int row = l8 + PL * t;
-            if (row < p) sq[t & 3] = fma_t(u[t], u[t], sq[t & 3]);
-            if (row == p) mine = u[t];
-          }
-          const T ss = gsum8((sq[0] + sq[1]) + (sq[2] + sq[3]), gm);
-          const T alpha = __shfl_sync(gm, mine, (lane & 24) | (p & 7));
-          T beta, tau, sc;
-          larfg_t(alpha, ss, beta, tau, sc);
-#pragma unroll
-          for (int t = 0; t < PE; ++t) {
-            const int row = l8 + PL * t;
-            if (row < p && tau != T(0)) u[t] *= sc;
-            if (row == p) u[t] = beta;
-            sv[buf * SVP + row] = row < p ? u[t] : (row == p ? T(1) : T(0));
-          }
-          if (l8 == 0) {
-            stau[buf] = tau;
-            ptau[c] = tau;
-            tq[c] = tau;
-          }
+        auto make = [&](int c) {
+          gen(u, c, mk + c, 0, X + c * XP, tq);
         };
-        if (g == k - 1) gen(k - 1, 0);
-        __syncthreads();
+        if (g == k - 1) make(k - 1);
+        __syncwarp();
         for (int c = k - 1; c >= 0; --c) {
-          const int cur = (k - 1 - c) & 1;
-          const T tau = stau[cur];
-          const T* v = sv + cur * SVP;
+          ok = oz::mbar_wait(&s_bar[0][c], 0) && ok;
+          __syncwarp();
+          const T tau = s_tau[0][c];
           T vv[PE];
 #pragma unroll
-          for (int t = 0; t < PE; ++t) vv[t] = v[l8 + PL * t];
-          if (g < c && tau != T(0)) refl(u, vv, tau);
-          if (c > 0 && g == c - 1) gen(c - 1, cur ^ 1);   // the next reflector first: it is on the critical path
-          if (tau != T(0)) {
-            if (g < n) refl(dq0, vv, tau);
-            if (g + BP < n) refl(dq1, vv, tau);
+          for (int t = 0; t < PE; ++t) vv[t] = X[c * XP + l8 + PL * t];
+          if (w0 < c) {   // uniform over the warp
+            if (g < c) refl(u, vv, tau);
+            if (c > 0 && g == c - 1) make(c - 1);   // the next reflector first: it is on the critical path
+            __syncwarp();
           }
-          __syncthreads();
+          if (w0 < n) refl(dq0, vv, tau);
+          if (w0 + BP < n) refl(dq1, vv, tau);
         }
+        __syncthreads();   // every warp has read its columns of U
 #pragma unroll
         for (int t = 0; t < PE; ++t) {
           const int row = l8 + PL * t;
           if (row < m) {
-            if (g < k) sW[row + g * LDU] = u[t];
+            if (g < k) gU[row + (int64_t)g * m] = u[t];
             if (g < n) sD[row + g * LDD] = dq0[t];
             if (g + BP < n) sD[row + (g + BP) * LDD] = dq1[t];
           }
         }
+        // columns of U beyond the reflectors (k < ku) pass unchanged
+        for (int e = tid; e < m * (ku - k); e += NT) gU[e + (int64_t)k * m] = sW[(e % m) + (k + e / m) * LDU];
       }
       __syncthreads();
-      ql_gram(sW, LDU, 0, k, mk, G);
-      blk_tmat(k, G, ptau, Tm, fb + nd.fTq);
-      for (int e = tid; e < m * ku; e += NT) gU[e] = sW[(e % m) + (e / m) * LDU];
-      __syncthreads();
-      // ---- LQ of D[0:mk, :] (gelqf!, :44), applied to the rows below (:47) and to V (:50) ----
+      // ---- LQ of D[0:mk, :] (gelqf!, :44), applied to the rows below (:47) and to V (:50); reflectors in W ----
       {
+        T* Yc = sW;   // U is in global memory now
         T d[PE], dt[PE], vc[PE];
 #pragma unroll
         for (int t = 0; t < PE; ++t) {
@@ -779,73 +799,42 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
           dt[t] = (mk + g < m && col < n) ? sD[(mk + g) + col * LDD] : T(0);
           vc[t] = (g < kv && col < n) ? sV[col + g * LDV] : T(0);
         }
-        auto gen = [&](int i, int buf) {   // the 8 lanes of row i
-          T sq[4] = {T(0), T(0), T(0), T(0)}, mine = T(0);
-#pragma unroll
-          for (int t = 0; t < PE; ++t) {
-            const int col = l8 + PL * t;
-            if (col > i) sq[t & 3] = fma_t(d[t], d[t], sq[t & 3]);
-            if (col == i) mine = d[t];
-          }
-          const T ss = gsum8((sq[0] + sq[1]) + (sq[2] + sq[3]), gm);
-          const T alpha = __shfl_sync(gm, mine, (lane & 24) | (i & 7));
-          T beta, tau, sc;
-          larfg_t(alpha, ss, beta, tau, sc);
-#pragma unroll
-          for (int t = 0; t < PE; ++t) {
-            const int col = l8 + PL * t;
-            if (col > i && tau != T(0)) d[t] *= sc;
-            if (col == i) d[t] = beta;
-            sv[buf * SVP + col] = col < i ? T(0) : (col == i ? T(1) : d[t]);
-          }
-          if (l8 == 0) {
-            stau[buf] = tau;
-            ptau[i] = tau;
-            tl[i] = tau;
-          }
-        };
-        if (g == 0) gen(0, 0);
-        __syncthreads();
+        __syncthreads();   // sW is overwritten
+        auto make = [&](int i) { gen(d, i, i, 1, Yc + i * YP, tl); };
+        if (g == 0) make(0);
+        __syncwarp();
         for (int i = 0; i < mk; ++i) {
-          const int cur = i & 1;
-          const T tau = stau[cur];
-          const T* v = sv + cur * SVP;
+          ok = oz::mbar_wait(&s_bar[1][i], 0) && ok;
+          __syncwarp();
+          const T tau = s_tau[1][i];
           T vv[PE];
 #pragma unroll
-          for (int t = 0; t < PE; ++t) vv[t] = v[l8 + PL * t];
-          if (g > i && g < mk && tau != T(0)) refl(d, vv, tau);
-          if (i + 1 < mk && g == i + 1) gen(i + 1, cur ^ 1);
-          if (tau != T(0)) {
-            if (mk + g < m) refl(dt, vv, tau);
-            if (g < kv) refl(vc, vv, tau);
+          for (int t = 0; t < PE; ++t) vv[t] = Yc[i * YP + l8 + PL * t];
+          if (w0 + 3 > i && w0 < mk) {   // uniform over the warp
+            if (g > i && g < mk) refl(d, vv, tau);
+            if (i + 1 < mk && g == i + 1) make(i + 1);
+            __syncwarp();
           }
-          __syncthreads();
+          if (mk + w0 < m) refl(dt, vv, tau);
+          if (w0 < kv) refl(vc, vv, tau);
         }
-        // write back; the reflectors also reflector-major (zero-padded to YP - 4
-        // columns) for the Gram matrix, and transposed to global memory
+        if (!ok && sl.err) atomicCAS(sl.err, DEV_OK, DEV_TIMEOUT);
         T* gQt = fb + nd.fQt;
-        T* Yc = sW;   // U is in global memory now
 #pragma unroll
         for (int t = 0; t < PE; ++t) {
           const int col = l8 + PL * t;
-          const T y = col < g ? T(0) : (col == g ? T(1) : d[t]);
           if (col < n) {
             if (g < mk) {
               sD[g + col * LDD] = d[t];
-              gQt[col + (int64_t)g * n] = y;
+              gQt[col + (int64_t)g * n] = col < g ? T(0) : (col == g ? T(1) : d[t]);
             }
             if (mk + g < m) sD[(mk + g) + col * LDD] = dt[t];
-            if (g < kv) sV[col + g * LDV] = vc[t];
+            if (g < kv) gV[col + (int64_t)g * n] = vc[t];
           }
-          if (g < mk && col < YP - 4) Yc[g * YP + col] = col < n ? y : T(0);
         }
         __syncthreads();
-        lq_gram(Yc, YP, n, mk, G);
-        blk_tmat(mk, G, ptau, Tm, fb + nd.fTl);
       }
-      blk_linv(mk, sD, LDD, sW, fb + nd.fLi);
       for (int e = tid; e < m * n; e += NT) gD[e] = sD[(e % m) + (e / m) * LDD];
-      for (int e = tid; e < n * kv; e += NT) gV[e] = sV[(e % n) + (e / n) * LDV];
       return;
     }
   }
@@ -1005,8 +994,8 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
     if (i1 < m) lq_apply_right(sD, LDD, i1, m, n, Yc, YP, nb, Tm, X);
     if (kv > 0) lq_apply_v(sV, LDV, n, kv, Yc, YP, nb, Tm, X);   // V <- Q V (ormlq!('L', 'N'), :50)
   }
-  // inverses of L1's diagonal blocks for the solve (the panel buffer is free)
-  blk_linv(mk, sD, LDD, sW, fb + nd.fLi);
+  // inverses of L1's diagonal blocks for the blocked solve (the panel buffer is free)
+  if constexpr (S > 64) blk_linv(mk, sD, LDD, sW, fb + nd.fLi);
   for (int e = tid; e < m * n; e += NT) gD[e] = sD[(e % m) + (e / m) * LDD];
   for (int e = tid; e < n * kv; e += NT) gV[e] = sV[(e % n) + (e / n) * LDV];
 }
@@ -1027,36 +1016,42 @@ bool factor_blk_fits(int mmax, int nmax, int kumax, int kvmax, size_t extra) {
 namespace {
 template <typename T, int S>
 void launch_blk_sized(const Task* t, int64_t nt, const Slot* s, int kumax, int kvmax, size_t extra, size_t smem,
-                      cudaStream_t st) {
+                      cudaStream_t st, bool pdl) {
   static bool attr_set = false;
   if (!attr_set) {
     cudaFuncSetAttribute(ulv_factor_blk_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlkSmemCap);
     attr_set = true;
   }
-  ulv_factor_blk_kernel<T, S><<<(unsigned)nt, NT, smem, st>>>(t, s, kumax, kvmax, (int)extra);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)nt);
+  cfg.blockDim = dim3(NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, ulv_factor_blk_kernel<T, S>, t, s, kumax, kvmax, (int)extra);
 }
 }  // namespace
 
 template <typename T>
 void launch_ulv_factor_blk(const Task* t, int64_t nt, const Slot* s, int mmax, int nmax, int kumax, int kvmax,
-                           size_t extra, cudaStream_t st) {
+                           size_t extra, cudaStream_t st, bool pdl) {
   if (nt <= 0) return;
   const size_t smem = factor_blk_smem<T>(mmax, nmax, kumax, kvmax, extra);
   switch (size_bucket(mmax, nmax)) {
-    case 32: launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st); break;
-    case 64: launch_blk_sized<T, 64>(t, nt, s, kumax, kvmax, extra, smem, st); break;
-    case 96: launch_blk_sized<T, 96>(t, nt, s, kumax, kvmax, extra, smem, st); break;
-    default: launch_blk_sized<T, 128>(t, nt, s, kumax, kvmax, extra, smem, st); break;
+    case 32: launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+    case 64: launch_blk_sized<T, 64>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+    case 96: launch_blk_sized<T, 96>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+    default: launch_blk_sized<T, 128>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
   }
 }
 
-template bool factor_blk_fits<double>(int, int, int, int, size_t);
 template bool factor_blk_fits<float>(int, int, int, int, size_t);
-template size_t factor_blk_smem<double>(int, int, int, int, size_t);
 template size_t factor_blk_smem<float>(int, int, int, int, size_t);
-template void launch_ulv_factor_blk<double>(const Task*, int64_t, const Slot*, int, int, int, int, size_t,
-                                            cudaStream_t);
 template void launch_ulv_factor_blk<float>(const Task*, int64_t, const Slot*, int, int, int, int, size_t,
-                                           cudaStream_t);
+                                           cudaStream_t, bool);
 
 }  // namespace hss

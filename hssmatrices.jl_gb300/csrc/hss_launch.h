@@ -112,15 +112,16 @@ void launch_pqr(const PqrTask* tasks, int64_t count, int qmax, int kmax, cudaStr
 template <typename T>
 void launch_ulv_factor(const Task* t, int64_t ntasks, const Slot* s, int max_m, int max_n,
                        cudaStream_t st);
-// Blocked on-chip factor kernel (hss_factor_blk.cu), FP32 (two blocks per SM)
-// or FP64; `extra` = merge staging elements.
+// Blocked on-chip factor kernel (hss_factor_blk.cu), T = float: two blocks per SM;
+// `extra` = merge staging elements; pdl: a programmatic dependent of the launch
+// before it (the level below).
 template <typename T>
 bool factor_blk_fits(int mmax, int nmax, int kumax, int kvmax, size_t extra);
 template <typename T>
 size_t factor_blk_smem(int mmax, int nmax, int kumax, int kvmax, size_t extra);
 template <typename T>
-void launch_ulv_factor_blk(const Task* t, int64_t ntasks, const Slot* s, int mmax, int nmax, int kumax, int kvmax,
-                           size_t extra, cudaStream_t st);
+void launch_ulv_factor_blk(const Task* t, int64_t nt, const Slot* s, int mmax, int nmax, int kumax, int kvmax,
+                           size_t extra, cudaStream_t st, bool pdl);
 // The reduction of one level by panels (hss_factor_pan.cu), FP32 or FP64, nodes up
 // to 512 x 512: largest sizes of the level's nodes (roots apart), and which kinds
 // it has.  *launches gets the number of kernels.
