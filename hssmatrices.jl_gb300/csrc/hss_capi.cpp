@@ -268,12 +268,9 @@ struct hss_plan_s {
   int pmv_nleaf = 0, pmv_mleaf = 0, pmv_kmax = 0;   // largest leaf columns / rows, largest rank
   int64_t pmv_ninner = 0;                           // branches that are not roots
   int64_t tr_lo = 0, tr_hi = 0;         // element range of d_gen holding every translator (B, R, W)
-  // flat product tables (flat_dep = 0: it does not apply): per-node links,
-  // per-leaf ancestor paths (flat_dep entries each), the non-root branches
-  FlatLink* d_links = nullptr;
-  int32_t* d_paths = nullptr;
-  int32_t flat_dep = 0;
-  Seg branches;
+  FlatTables flat;                      // flat product tables in one allocation (dep = 0: it does not apply)
+  unsigned char* d_flat = nullptr;
+  int64_t flat_bytes = 0;
   std::vector<Task> h_tasks;            // host copy of the task lists (merged batches)
   std::vector<int64_t> h_table;         // node table of a single-tree plan (hss_export)
   int64_t h_npacked = 0;                // its packed generator length
@@ -348,8 +345,7 @@ hss_plan_s::~hss_plan_s() {
   if (d_tasks) cudaFree(d_tasks);
   if (d_err) cudaFree(d_err);
   if (d_sync) cudaFree(d_sync);
-  if (d_links) cudaFree(d_links);
-  if (d_paths) cudaFree(d_paths);
+  if (d_flat) cudaFree(d_flat);
 }
 
 
@@ -639,19 +635,22 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
 // so caches keyed on plans use these instead of pointers.
 std::atomic<uint64_t> g_plan_serial{0};
 
-// Tables of the flat product: the edge of every non-root node to its parent,
-// and every leaf's ancestors by depth.  It applies when each subtree's leaves
-// are contiguous in the leaf list (pre-order node numbering gives that) and
-// the trees are not deeper than kFlatDep - 1.
+// Tables of the flat product.  It applies when each subtree's leaves are contiguous
+// in the leaf list (pre-order node numbering gives that) and the trees are not
+// deeper than kFlatDep - 1.
 int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
   const std::vector<Node>& N = P->nodes;
-  const int64_t nn = (int64_t)N.size();
-  std::vector<int32_t> lo(nn, INT32_MAX), hi(nn, -1), cnt(nn, 0);
+  const int64_t nn = (int64_t)N.size(), nl = P->leaves.cnt;
+  std::vector<int32_t> lo(nn, INT32_MAX), hi(nn, -1), cnt(nn, 0), up(nn), height(nn);
   int maxd = 0;
-  for (int64_t t = 0; t < P->leaves.cnt; ++t) {
-    const int32_t i = tasks[P->leaves.off + t].node;
+  for (int64_t i = 0; i < nn; ++i) {
+    up[i] = N[i].root ? -1 : N[i].parent;
+    height[i] = N[i].height;
     maxd = std::max(maxd, N[i].depth);
-    for (int32_t y = i; y >= 0; y = N[y].parent) {
+  }
+  auto leaf_node = [&](int64_t t) { return tasks[P->leaves.off + t].node; };
+  for (int64_t t = 0; t < nl; ++t) {
+    for (int32_t y = leaf_node(t); y >= 0; y = up[y]) {
       lo[y] = std::min<int32_t>(lo[y], (int32_t)t);
       hi[y] = std::max<int32_t>(hi[y], (int32_t)t);
       ++cnt[y];
@@ -661,8 +660,26 @@ int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
     if (cnt[i] > 0 && hi[i] - lo[i] + 1 != cnt[i]) return HSS_OK;
   const int dep = maxd + 1;
   if (dep < 2 || dep > kFlatDep) return HSS_OK;
-  std::vector<FlatLink> links(nn);
-  std::memset(links.data(), 0, links.size() * sizeof(FlatLink));
+  // one image: the links; per level the groups and the branches
+  int32_t ng[kFlatLevels] = {}, nbr[kFlatLevels] = {};
+  auto is_root = [&](int32_t i, int gmax) {   // of a group
+    return up[i] >= 0 && cnt[i] <= gmax && (up[up[i]] < 0 || cnt[up[i]] > gmax);
+  };
+  for (int level = 0; level < kFlatLevels; ++level)
+    for (int64_t i = 0; i < nn; ++i) {
+      ng[level] += is_root((int32_t)i, 1 << level);
+      nbr[level] += up[i] >= 0 && cnt[i] > 1 << level;
+    }
+  size_t bytes = (size_t)nn * sizeof(FlatLink), at[kFlatLevels][2];
+  for (int level = 0; level < kFlatLevels; ++level) {
+    at[level][0] = bytes;
+    bytes += (size_t)ng[level] * sizeof(FlatGroup);
+    at[level][1] = bytes;
+    bytes += (size_t)nbr[level] * sizeof(FlatBranch);
+  }
+  static_assert(sizeof(FlatLink) % 16 == 0 && sizeof(FlatGroup) % 16 == 0 && sizeof(FlatBranch) % 16 == 0, "aligned");
+  std::vector<unsigned char> img(bytes);
+  FlatLink* links = (FlatLink*)img.data();
   for (int64_t i = 0; i < nn; ++i) {
     const Node& x = N[i];
     if (x.root) continue;
@@ -681,20 +698,66 @@ int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
     L.kpv = p.kv;
     L.sku = sib.ku;
     L.depth = x.depth;
-    L.lf0 = lo[i];
-    L.lfn = cnt[i];
   }
-  std::vector<int32_t> paths((size_t)std::max<int64_t>(P->leaves.cnt, 1) * dep, 0);
-  for (int64_t t = 0; t < P->leaves.cnt; ++t)
-    for (int32_t y = tasks[P->leaves.off + t].node; !N[y].root; y = N[y].parent) paths[t * dep + N[y].depth] = y;
-  CUDA_TRY(dev_alloc((void**)&P->d_links, std::max<size_t>(links.size(), 1) * sizeof(FlatLink)));
-  CUDA_TRY(cudaMemcpy(P->d_links, links.data(), links.size() * sizeof(FlatLink), cudaMemcpyHostToDevice));
-  CUDA_TRY(dev_alloc((void**)&P->d_paths, paths.size() * sizeof(int32_t)));
-  CUDA_TRY(cudaMemcpy(P->d_paths, paths.data(), paths.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  P->branches.off = P->mv_up.empty() ? 0 : P->mv_up.front().off;
-  P->branches.cnt = 0;
-  for (const Seg& g : P->mv_up) P->branches.cnt += g.cnt;
-  P->flat_dep = dep;
+  std::vector<int32_t> gof(nl + 1);   // groups that start before leaf t
+  for (int level = 0; level < kFlatLevels; ++level) {
+    const int gmax = 1 << level;
+    FlatGroup* groups = (FlatGroup*)(img.data() + at[level][0]);
+    FlatBranch* branches = (FlatBranch*)(img.data() + at[level][1]);
+    int32_t n = 0;
+    for (int64_t t = 0; t < nl;) {
+      int32_t y = leaf_node(t);
+      gof[t] = n;
+      while (up[y] >= 0 && !is_root(y, gmax)) y = up[y];
+      if (up[y] < 0) {   // a single-leaf tree
+        ++t;
+        continue;
+      }
+      FlatGroup& g = groups[n++];
+      g.slot = N[y].tree;
+      g.nl = cnt[y];
+      g.t0 = (int32_t)t;
+      g.depth = N[y].depth;
+      for (; g.nn < g.nl; ++g.nn) {
+        gof[t] = n - 1;
+        g.node[g.nn] = leaf_node(t++);
+      }
+      // branches, once both children are numbered, lowest first
+      int32_t in[kFlatGroup - 1], nb = 0;
+      for (int k = 0; k < g.nl; ++k)
+        for (int32_t i = up[g.node[k]]; k + 1 < g.nl && lo[i] == g.t0 + k && cnt[i] <= g.nl; i = up[i]) {
+          int b = nb++;
+          for (; b > 0 && height[in[b - 1]] > height[i]; --b) in[b] = in[b - 1];
+          in[b] = i;
+          if (i == y) break;
+        }
+      for (int b = 0; b < nb; ++b) {
+        const Node& x = N[in[b]];
+        for (int k = 0; k < g.nn; ++k) {
+          if (g.node[k] == x.left) g.left[b] = k;
+          if (g.node[k] == x.right) g.right[b] = k;
+        }
+        g.level[b] = b == 0 || height[in[b - 1]] != height[in[b]];
+        g.node[g.nn++] = in[b];
+      }
+      for (int32_t i = y, d = g.depth; d > 0; i = up[i]) g.path[--d] = i;
+    }
+    gof[nl] = n;
+    n = 0;
+    for (int64_t i = 0; i < nn; ++i)
+      if (up[i] >= 0 && cnt[i] > gmax)
+        branches[n++] = FlatBranch{(int32_t)i, N[i].tree, gof[lo[i]], gof[hi[i] + 1] - gof[lo[i]]};
+  }
+  CUDA_TRY(dev_alloc((void**)&P->d_flat, img.size()));
+  CUDA_TRY(cudaMemcpy(P->d_flat, img.data(), img.size(), cudaMemcpyHostToDevice));
+  P->flat_bytes = (int64_t)img.size();
+  FlatTables& f = P->flat;
+  for (int level = 0; level < kFlatLevels; ++level)
+    f.lev[level] = FlatLevel{(const FlatGroup*)(P->d_flat + at[level][0]), (const FlatBranch*)(P->d_flat + at[level][1]),
+                             ng[level], nbr[level]};
+  f.nodes = P->d_nodes;
+  f.links = (const FlatLink*)P->d_flat;
+  f.dep = dep;
   return HSS_OK;
 }
 
@@ -797,11 +860,8 @@ struct Levels {
   int64_t nodes_max = 0, nslots = 0;   // largest node array of a slot's plan; slots
   int64_t ninner = 0;                  // non-root branches
   int device = 0;
-  // flat product tables (flat_dep = 0: not available)
-  const FlatLink* links = nullptr;
-  const int32_t* paths = nullptr;
-  int flat_dep = 0;
-  Seg branches;
+  FlatTables flat;   // flat product tables (dep = 0: not available)
+  int64_t gen_len = 0;
   // translators to prefetch into L2 (FP64 and pair copies; null: none)
   const double* pf64 = nullptr;
   const float2* pfdf = nullptr;
@@ -824,10 +884,8 @@ Levels plan_levels(const hss_plan_s* P) {
   L.nslots = P->ntrees;
   L.ninner = P->pmv_ninner;
   L.device = P->device;
-  L.links = P->d_links;
-  L.paths = P->d_paths;
-  L.flat_dep = P->flat_dep;
-  L.branches = P->branches;
+  L.flat = P->flat;
+  L.gen_len = P->gen_len;
   if (P->tr_hi > P->tr_lo) {
     L.pf64 = P->d_gen + P->tr_lo;
     L.pfdf = P->d_gen_df ? P->d_gen_df + P->tr_lo : nullptr;
@@ -843,21 +901,27 @@ bool use_pmv(const Levels& L, const SlotTable* pm, bool pairs, int rmax) {
          pmv_chunks(pairs, rmax) > 0 && pmv_queue_fits(L.nodes_max, L.nslots);
 }
 
+int sm_count(int device);
+
 // The flat product takes FP64 products of few columns on plans that have its tables.
 bool use_flat(const Levels& L, bool pairs, int rmax) {
-  return !pairs && g_flat_product && L.flat_dep > 0 && pmv_flat_fits(L.nleaf, L.kmax, L.flat_dep, rmax);
+  return !pairs && g_flat_product && L.flat.dep > 0 && pmv_flat_fits(L.flat, L.gen_len, L.nleaf, L.kmax, rmax, sm_count(L.device));
+}
+
+cudaError_t ensure_flat(const Levels& L, int rmax, SlotTable& pm, cudaStream_t st) {
+  int64_t ctb = 0, counters = 0;
+  pmv_flat_space(L.flat, L.leaves.cnt, L.kmax, rmax, sm_count(L.device), &ctb, &counters);
+  return pm.ensure_flat(ctb, counters, st);
 }
 
 int run_pmv(const Levels& L, const Slot* slots, int rmax, bool pairs, SlotTable& pm, cudaStream_t st) {
   if (use_flat(L, pairs, rmax)) {
     CUDA_TRY(pm.ensure_pmv(1, st));
-    CUDA_TRY(pm.ensure_flat(pmv_flat_ctb_elems(L.leaves.cnt, L.flat_dep, L.kmax, rmax),
-                            L.leaves.cnt * pmv_flat_chunks(rmax), st));
+    CUDA_TRY(ensure_flat(L, rmax, pm, st));
     cudaError_t e = cudaSuccess;
     traced(HSS_TRACE_MV_LEAF, L.leaves.cnt, st, [&] {
-      e = launch_pmv_flat(L.d_tasks + L.leaves.off, L.leaves.cnt, L.d_tasks + L.branches.off, L.branches.cnt,
-                          L.links, L.paths, L.flat_dep, slots, rmax, L.nleaf, L.mleaf, L.kmax, pm.pstate.p,
-                          pm.ctb.p, pm.dcnt.p, L.device, st);
+      e = launch_pmv_flat(L.flat, L.d_tasks + L.leaves.off, L.leaves.cnt, slots, rmax, L.nleaf, L.mleaf, L.kmax,
+                          pm.pstate.p, pm.ctb.p, pm.dcnt.p, L.device, sm_count(L.device), pmv_poll_limit(), st);
     });
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -890,9 +954,7 @@ cudaError_t pmv_prepare(const Levels& L, bool pairs, int rmax, SlotTable& pm, cu
   cudaError_t e = cudaSuccess;
   if (use_flat(L, pairs, rmax)) {
     e = pm.ensure_pmv(1, st);
-    if (e == cudaSuccess)
-      e = pm.ensure_flat(pmv_flat_ctb_elems(L.leaves.cnt, L.flat_dep, L.kmax, rmax),
-                         L.leaves.cnt * pmv_flat_chunks(rmax), st);
+    if (e == cudaSuccess) e = ensure_flat(L, rmax, pm, st);
   } else {
     e = pm.ensure_pmv(pmv_queue_entries(L.ntasks, L.ninner, pmv_chunks(pairs, rmax)), st);
   }
@@ -1296,17 +1358,28 @@ int check_cols(hss_plan_s* P, const std::vector<Cols>& io, bool solve) {
 }
 
 // Whether the tensor-core product takes a product of r columns.  It needs one
-// launch per tree level (about 5 us each) and, once per plan, the digit slices
-// (100-400 us with their allocation), and then hardly depends on r up to 32,
-// where the FP64 products grow with entries x columns at the FP64 pipe's rate:
-// n = 65536, k = 32 (15.7 M entries) 276 -> 194 us at r = 6, 938 -> 287 at 32,
-// 1838 -> 422 at 64; n = 16384 166 -> 103 at r = 6; n = 4096 (0.98 M) 105 -> 79
-// at r = 16, 87 -> 69 at 6; n = 10007, leaves of 39, k = 20 (1.3 M) 123 -> 115 at
-// r = 6, 155 -> 130 at 16; n = 2000, k = 16 (0.2 M) 88 -> 76 at r = 64.  The line is
-// where the gain repays the slices within a few products.  Up to 5 columns one
-// launch of the flat or the queued product is as fast (r = 4, n = 65536: 221).
+// launch per tree level and, once per plan, the digit slices (100-400 us with their
+// allocation), and then hardly depends on r up to 32, where the FP64 products grow
+// with entries x columns at the FP64 pipe's rate: n = 65536, k = 32 (15.7 M entries)
+// 286 -> 200 us at r = 6, 948 -> 293 at 32, 1838 -> 422 at 64.  Where the flat product
+// applies, the line is its estimate against the tensor-core product's (launches,
+// slices, blocks; fitted as the flat product's), with a tenth for the slices; both
+// sides measured, flat / tensor cores in us: n = 32768 r = 4 110 / 143, r = 5 155 /
+// 143; n = 16384 r = 8 110 / 110, r = 10 155 / 114; n = 8192 r = 12 85 / 93, r = 16
+// 111 / 100; n = 10007, leaves of 39 rows, r = 16 108 / 136, r = 20 179 / 154; n = 4000,
+// leaves of 250 rows, r = 8 61 / 79, r = 10 104 / 81; n = 2048 r = 32 60 / 72.  Elsewhere
+// the line is where the gain over the queued product repays the slices within a few
+// products (n = 16384 171 -> 107 at r = 6, n = 4096 98 -> 87 at r = 16), later at low
+// ranks, whose small blocks fill the tensor cores' tiles less (n = 18944, k = 8: 148
+// against 152 at r = 17, 221 against 156 at 32).
 bool oz_product_pays(const hss_plan_s* P, int64_t r) {
-  return !g_level_product && r >= 6 && P->gen_len * r >= 16000000;
+  if (g_level_product || r < 5) return false;
+  const Levels L = plan_levels(P);
+  if (!use_flat(L, false, (int)std::min<int64_t>(r, INT32_MAX)))
+    return P->gen_len * r >= (P->pmv_kmax >= 16 ? 16000000 : 45000000);
+  const double launches = 2.0 * (double)P->by_d.size() - 1.0, gen = (double)P->gen_len;
+  const double oz = (6.3 * launches + 2.6e-6 * gen + 0.086 * (double)P->leaves.cnt) * (1.0 + (double)r / 128.0);
+  return pmv_flat_estimate(P->flat, P->leaves.cnt, P->gen_len, (int)r, sm_count(P->device)) > 1.1 * oz;
 }
 
 int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double beta,
@@ -2604,7 +2677,7 @@ int hss_device_bytes(hss_handle h, hss_factor f, int64_t* bytes) {
     if (h->d_gen_df) b += h->gen_len * 8;
     if (h->d_oz) b += h->oz_bytes;
     // node descriptors, task lists, flat-product links, paths and counters
-    b += nn * (int64_t)(sizeof(Node) + 4 * sizeof(Task) + sizeof(FlatLink) + 4 * (h->flat_dep + 1));
+    b += nn * (int64_t)(sizeof(Node) + 4 * sizeof(Task)) + h->flat_bytes;
     b += (int64_t)(h->mv_ws.cap + h->hB.cap + h->hC.cap) * 8 + slots(h->mv_slots);
   }
   if (f) {

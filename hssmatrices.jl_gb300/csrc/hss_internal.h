@@ -52,17 +52,37 @@ struct Node {
 static_assert(sizeof(Node) % 8 == 0, "Node is copied as 8-byte words");
 
 // The edge from a non-root node x to its parent p, as the flat product reads
-// it (one chain of small products per leaf): the translators of p that act on
-// x, the F slots of x and of its sibling, the ranks involved and x's leaves.
+// it: the translators of p that act on x, the F slots of x and of its sibling,
+// and the ranks involved.
 struct FlatLink {
   const double* W;      // W1 or W2 of p (kv x kpv, ld kv): Z_p += W^T Z_x
   const double* R;      // R1 or R2 of p (ku x kpu, ld ku): F_x = G_x + R F_p
   const double* B;      // B21 (x left) or B12 (x right) of p (sku x kv, ld sku): G_sibling = B Z_x
   int64_t wf, swf;      // product workspace rows of F_x and of F_sibling
   int32_t ku, kv, kpu, kpv, sku, depth;
-  int32_t lf0, lfn;     // x's leaves: positions lf0 .. lf0 + lfn - 1 of the leaf list
 };
 static_assert(sizeof(FlatLink) % 8 == 0, "FlatLink is copied as 8-byte words");
+
+// A group of the flat product: a subtree (not a whole tree) of at most kFlatGroup
+// leaves.  Its nodes are numbered leaves first, from left to right, then branches
+// by height; the last one is its root.
+constexpr int kFlatGroup = 8;
+constexpr int kFlatDep = 32;       // deepest tree, and one
+struct FlatGroup {
+  int32_t slot, nl, nn;            // nl leaves, nn nodes
+  int32_t t0;                      // position of the first leaf in the leaf list
+  int32_t depth;                   // of the group's root
+  int32_t left[kFlatGroup - 1], right[kFlatGroup - 1];   // children of branch nl + b
+  int32_t level[kFlatGroup - 1];   // 1: branch nl + b is the first of its height
+  int32_t node[2 * kFlatGroup - 1];
+  int32_t path[kFlatDep - 1];      // the root's ancestors and itself: depths 1 .. depth
+};
+static_assert(sizeof(FlatGroup) % 8 == 0, "FlatGroup is copied as 8-byte words");
+
+// A non-root branch above the groups: the groups below it are g0 .. g0 + gn - 1.
+struct FlatBranch {
+  int32_t node, slot, g0, gn;
+};
 
 struct Task {
   const Node* nodes;   // node array the index refers to

@@ -69,24 +69,34 @@ cudaError_t launch_ozmv_prep(int kind, const Task* t, int64_t nt, int rows, int 
                              cudaStream_t st);
 cudaError_t launch_ozmv(int kind, const Task* t, int64_t nt, const Slot* s, int rmax, int rows, int sms, cudaStream_t st);
 
-// Flat persistent product (hss_pmv.cu), FP64 with few right-hand sides: every
-// leaf carries its own chain of small products up to the root and back, so
-// the launch has two grid barriers instead of the tree's dependency chain.
-// links: one per node of the plan (roots unused); paths: for leaf position t
-// of `leaves`, paths[t * dep + d] is its ancestor at depth d (1 <= d <= its
-// depth), dep > every leaf depth; branches: the non-root branches.  ctb holds
-// pmv_flat_ctb_elems doubles of contributions; dcnt one counter per (leaf,
-// chunk), zero before the first launch (the kernel leaves them zero).  The
-// state words are those of launch_pmv (zero between launches).
-constexpr int kFlatDep = 32;
-size_t pmv_flat_smem_elems(int nleaf, int kmax, int dep);
-bool pmv_flat_fits(int nleaf, int kmax, int dep, int rmax);
-int64_t pmv_flat_ctb_elems(int64_t nleaves, int dep, int kmax, int rmax);
-int64_t pmv_flat_chunks(int rmax);
-cudaError_t launch_pmv_flat(const Task* leaves, int64_t nleaves, const Task* branches, int64_t nbranch,
-                            const FlatLink* links, const int32_t* paths, int dep, const Slot* slots, int rmax,
-                            int nleaf, int mleaf, int kmax, uint32_t* state, double* ctb, uint32_t* dcnt,
-                            int device, cudaStream_t st);
+// Flat persistent product (hss_flat.cu), FP64 with few right-hand sides: one block
+// takes a group of leaves through the tree, so that the launch has two waits for
+// all blocks instead of the tree's chain of hand-offs.  The tables hold, per node of
+// the plan, the link to its parent (roots: unused), and the groups of at most 1, 2, 4
+// and 8 leaves with the branches above them; dep > every leaf's depth.
+// pmv_flat_space: doubles of contributions (ctb) and counters (dcnt, one per leaf
+// and chunk, zero before the first launch; the kernel leaves them zero).  The state
+// words are those of launch_pmv (zero between launches).
+constexpr int kFlatCols = 32;   // most columns
+constexpr int kFlatLevels = 4;  // groups of at most 1 << level leaves
+static_assert(kFlatGroup == 1 << (kFlatLevels - 1), "the largest groups");
+struct FlatLevel {
+  const FlatGroup* groups = nullptr;
+  const FlatBranch* branches = nullptr;
+  int32_t ngroup = 0, nbranch = 0;
+};
+struct FlatTables {
+  const Node* nodes = nullptr;
+  const FlatLink* links = nullptr;
+  FlatLevel lev[kFlatLevels];
+  int32_t dep = 0;   // 0: the product does not apply to the plan
+};
+bool pmv_flat_fits(const FlatTables& f, int64_t gen, int nleaf, int kmax, int rmax, int sms);
+double pmv_flat_estimate(const FlatTables& f, int64_t nleaves, int64_t gen, int rmax, int sms);
+void pmv_flat_space(const FlatTables& f, int64_t nleaves, int kmax, int rmax, int sms, int64_t* ctb, int64_t* counters);
+cudaError_t launch_pmv_flat(const FlatTables& f, const Task* leaves, int64_t nleaves, const Slot* slots, int rmax,
+                            int nleaf, int mleaf, int kmax, uint32_t* state, double* ctb, uint32_t* dcnt, int device,
+                            int sms, uint32_t idle_limit, cudaStream_t st);
 
 // Entry extraction (hss_getindex.cu): basis pass for one list of nodes (one
 // tree height), the off-diagonal tiles, the diagonal leaf blocks.  R / C are
