@@ -159,10 +159,14 @@ inline void seg_add(Seg& v, const Node& x, const Node* nodes) {
 template <class F>
 void seg_split(Seg& v, std::vector<Task>& tasks, F&& nodes) {
   v.parts.clear();
+  bool one = true;
   std::vector<std::pair<int, int64_t>> key((size_t)v.cnt);
-  for (int64_t i = 0; i < v.cnt; ++i) key[i] = {size_class(nodes(i)[tasks[v.off + i].node]), i};
+  for (int64_t i = 0; i < v.cnt; ++i) {
+    key[i] = {size_class(nodes(i)[tasks[v.off + i].node]), i};
+    one = one && key[i].first == key[0].first;
+  }
+  if (one) return;
   std::stable_sort(key.begin(), key.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-  if (key.empty() || key.front().first == key.back().first) return;
   const std::vector<Task> old(tasks.begin() + v.off, tasks.begin() + v.off + v.cnt);
   for (int64_t i = 0; i < v.cnt; ++i) {
     if (i == 0 || key[i].first != key[i - 1].first) {
@@ -606,14 +610,20 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
   P->ws_sv = std::max<int64_t>(ws_sv, 1);
   P->fac_elems = std::max<int64_t>(fac, 1);
   // task lists
+  // nodes by height and by depth, in index order (one pass each over the descriptors)
+  std::vector<std::vector<int32_t>> at_h(max_h + 1), at_d(max_d + 1);
+  for (int64_t i = 0; i < total_nodes; ++i) {
+    at_h[P->nodes[i].height].push_back((int32_t)i);
+    at_d[P->nodes[i].depth].push_back((int32_t)i);
+  }
   auto add_seg = [&](std::vector<Seg>& v, auto pred, int nlev, bool by_height, bool split) {
     v.assign(nlev + 1, Seg{});
     for (int lv = 0; lv <= nlev; ++lv) {
       v[lv].off = (int64_t)tasks.size();
-      for (int64_t i = 0; i < total_nodes; ++i) {
+      for (int32_t i : (by_height ? at_h : at_d)[lv]) {
         const Node& x = P->nodes[i];
-        if ((by_height ? x.height : x.depth) == lv && pred(x)) {
-          tasks.push_back(Task{nullptr, (int32_t)i, x.tree});
+        if (pred(x)) {
+          tasks.push_back(Task{nullptr, i, x.tree});
           seg_add(v[lv], x, P->nodes.data());
         }
       }
