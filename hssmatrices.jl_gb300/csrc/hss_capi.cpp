@@ -1112,18 +1112,24 @@ inline size_t factor_extra(const Seg& g) {
          (size_t)g.c1nr * g.c1v + (size_t)g.c2nr * g.c2v + (size_t)g.c1mr * g.c2v + (size_t)g.c2mr * g.c1v;
 }
 
+// Levels of the one-block kernel: FP32 nodes up to 128 x 128, FP64 up to 40 x 40
+// (merges of rank 16 167 -> 105 us a level, rank 8 122 -> 50; 60000 unknowns in
+// leaves of 15 rows 1926 -> 540; leaves of 38 rows, k = 16 194 -> 145; but leaves of 47
+// rows, k = 12 271 against 328, 64 x 64 merges 300 against 385: the panels' updates on
+// the tensor cores).  Above 32 rows only what its one-panel path takes.
 template <typename T>
 bool factor_level_blk(const Seg& g) {
-  return sizeof(T) == 4 && factor_blk_fits<float>(g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g));
+  if (sizeof(T) == 8 && std::max(g.mmax, g.nmax) > 32 && std::max({g.mkmax, g.kumax, g.kvmax}) > 32) return false;
+  return factor_blk_fits<T>(g.mmax, g.nmax, g.kumax, g.kvmax, factor_extra(g));
 }
 // Levels reduced by panels with the block updates on the tensor cores.  FP64: all
-// that fit (n = 65536, k = 32: 12.6 -> 5.8 ms; 256-row leaves, k = 40: 10.2 -> 5.9;
-// 1200 unknowns, k = 16: 1.18 -> 0.95).  FP32: levels whose nodes the one-block kernel
+// others that fit (n = 65536, k = 32: 12.6 -> 5.8 ms; 256-row leaves, k = 40: 10.2 ->
+// 5.9).  FP32: levels whose nodes the one-block kernel
 // does not take (156-row leaves, k = 40: 1.47 -> 0.63 ms); where it fits it is faster
 // (n = 65536: 1.45 against 1.83 ms).
 template <typename T>
 bool factor_level_pan(const Seg& g) {
-  return factor_pan_fits(g.mmax, g.nmax) && (sizeof(T) == 8 || !factor_level_blk<T>(g));
+  return factor_pan_fits(g.mmax, g.nmax) && !factor_level_blk<T>(g);
 }
 // Levels of the one-block kernel, whose FP32 factors the blocked solve can read (it
 // needs the inverses of L1's diagonal blocks).
@@ -1163,14 +1169,14 @@ bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t
         launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
         add_launches(launches - 1);
       } else if (factor_level_fast<T>(g)) {
-        launch_ulv_factor_blk<float>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax,
-                                     factor_extra(g), st, h > 0);
+        launch_ulv_factor_blk<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax,
+                                 factor_extra(g), st, h > 0);
       } else {
         launch_ulv_factor<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, st);
       }
     });
   });
-  return factor_level_fast<T>(all);
+  return sizeof(T) == 4 && factor_level_fast<T>(all);
 }
 
 template <typename T>

@@ -1,9 +1,9 @@
-// Blocked ULV reduction of one node per thread block, FP32, for nodes
+// Blocked ULV reduction of one node per thread block, for FP32 nodes
 // up to 128 x 128 with ranks up to 64 (every node of the leafsize-128 and
 // leafsize-64 workloads).  Restated from src/ulvfactor.jl:22-57 (the leaf
 // reduction) and :74-79 (the merge), with the reference's reflector order:
 //
-//   P0  load the leaf's D and U (FP64 -> FP32) or assemble the merged block of the
+//   P0  load the leaf's D and U (FP64 -> T) or assemble the merged block of the
 //       children (D, U in shared memory; V = [V1 W1; V2 W2], T12, T21 to global);
 //   P1  QL of U (geqlf!, :39) by panels of 32 columns from the last: inside a
 //       panel every reflector is generated and applied one at a time (8 lanes per
@@ -15,8 +15,10 @@
 //       to the rows below it, C <- C - (C Y^T) T Y (ormlq!, :47), and to V,
 //       V <- V - Y^T T^T Y V (ormlq!('L', 'N'), :50).
 //
-// Launches whose nodes are all at most 64 x 64 (the merges of rank-32 children)
-// skip the block updates: each reflector is applied to D (QL) or to D's
+// Launches whose nodes are all at most 64 x 64 (the merges of rank-32 children) skip
+// the block updates (FP64 nodes of at most 40 rows are all of this kind: the FP64
+// pipe takes 64 clocks an instruction, so that larger ones gain more from the panels'
+// updates on the tensor cores): each reflector is applied to D (QL) or to D's
 // trailing rows and V (LQ) in the panel loop itself, as soon as the barrier of
 // that reflector opens, and neither T nor the L1 inverses are formed (the
 // register solves, which run such nodes, read neither).
@@ -58,6 +60,7 @@ constexpr int XC = 64;              // columns (QL) or rows (LQ) of C per GEMM c
 constexpr int XP = XC + 4;          // ld of the GEMM intermediate (>= kv, multiple of 4)
 constexpr int SVP = BMAX;           // length of a broadcast reflector
 constexpr size_t kBlkSmemCap = 226 * 1024;
+constexpr size_t kBlkSmemCap64 = 112 * 1024;   // FP64 (nodes of at most 40 rows): two blocks per SM
 static_assert(XP >= BKMAX, "X holds Y V (32 x kv) in the V update");
 
 __host__ __device__ constexpr size_t sz4(size_t e) { return (e + 3) & ~size_t(3); }
@@ -90,8 +93,10 @@ struct BlkLayout {
     total = oX + zmax(tail, sz4(extra));
   }
 };
-__host__ __device__ constexpr int size_bucket(int mmax, int nmax) {
-  return (((mmax > nmax ? mmax : nmax) + 31) / 32) * 32;
+template <typename T>
+constexpr int size_bucket(int mmax, int nmax) {
+  const int s = mmax > nmax ? mmax : nmax;
+  return sizeof(T) == 8 && s > 32 ? 48 : (s + 31) / 32 * 32;
 }
 static_assert(BP * GP + 4 + 2 * SVP <= BP * XP, "the Gram matrix and the broadcast reflectors fit in X");
 
@@ -546,7 +551,7 @@ __device__ __forceinline__ void lq_apply_v(T* V, int LDV, int n, int kv, const T
 }
 
 template <typename T, int S>
-__global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
+__global__ void __launch_bounds__(NT, 2)
     ulv_factor_blk_kernel(const Task* __restrict__ tasks, const Slot* __restrict__ slots, int kumax, int kvmax,
                           int extra) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -703,14 +708,14 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
       __syncthreads();
       const int w0 = tid / 32 * 4;   // the warp's first group
       bool ok = true;
+      // sums in one FP64 accumulator: the pipe takes an instruction every 64 clocks, so
+      // that a second one only adds an addition; two in FP32
+      constexpr int NA = sizeof(T) == 8 ? 1 : 2;
       auto refl = [&](T(&x)[PE], const T(&vv)[PE], T tau) {
-        T a0 = T(0), a1 = T(0);
+        T a[NA];
 #pragma unroll
-        for (int t = 0; t < PE; t += 2) {
-          a0 = fma_t(vv[t], x[t], a0);
-          a1 = fma_t(vv[t + 1], x[t + 1], a1);
-        }
-        const T w = gsum8(a0 + a1, gm) * -tau;
+        for (int t = 0; t < PE; ++t) a[t % NA] = t < NA ? vv[t] * x[t] : fma_t(vv[t], x[t], a[t % NA]);
+        const T w = gsum8(NA == 1 ? a[0] : a[0] + a[NA - 1], gm) * -tau;
 #pragma unroll
         for (int t = 0; t < PE; ++t) x[t] = fma_t(w, vv[t], x[t]);
       };
@@ -718,14 +723,18 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
       // (QL, ph = 0) or behind it (LQ, ph = 1)
       auto gen = [&](T(&x)[PE], int a, int pv, int ph, T* Y, T* taus) {
         auto in = [&](int i) { return ph == 0 ? i < pv : i > pv; };
-        T sq[4] = {T(0), T(0), T(0), T(0)}, mine = T(0);
+        constexpr int NS = NA == 1 ? 1 : 4;
+        T sq[NS], mine = T(0);
 #pragma unroll
         for (int t = 0; t < PE; ++t) {
           const int i = l8 + PL * t;
-          if (in(i)) sq[t & 3] = fma_t(x[t], x[t], sq[t & 3]);
+          const T z = in(i) ? x[t] : T(0);
+          sq[t % NS] = t < NS ? z * z : fma_t(z, z, sq[t % NS]);
           if (i == pv) mine = x[t];
         }
-        const T ss = gsum8((sq[0] + sq[1]) + (sq[2] + sq[3]), gm);
+        T ss = sq[0];
+        if constexpr (NS == 4) ss = (sq[0] + sq[1]) + (sq[2] + sq[3]);
+        ss = gsum8(ss, gm);
         const T alpha = __shfl_sync(gm, mine, (lane & 24) | (pv & 7));
         T beta, tau, sc;
         larfg_t(alpha, ss, beta, tau, sc);
@@ -1004,13 +1013,13 @@ __global__ void __launch_bounds__(NT, (sizeof(T) == 4 ? 2 : 1))
 
 template <typename T>
 size_t factor_blk_smem(int mmax, int nmax, int kumax, int kvmax, size_t extra) {
-  return BlkLayout(size_bucket(mmax, nmax), kumax, kvmax, extra).total * sizeof(T);
+  return BlkLayout(size_bucket<T>(mmax, nmax), kumax, kvmax, extra).total * sizeof(T);
 }
 
 template <typename T>
 bool factor_blk_fits(int mmax, int nmax, int kumax, int kvmax, size_t extra) {
-  return mmax <= BMAX && nmax <= BMAX && kumax <= BKMAX && kvmax <= BKMAX &&
-         factor_blk_smem<T>(mmax, nmax, kumax, kvmax, extra) <= kBlkSmemCap;
+  return mmax <= (sizeof(T) == 4 ? BMAX : 40) && nmax <= (sizeof(T) == 4 ? BMAX : 40) && kumax <= BKMAX && kvmax <= BKMAX &&
+         factor_blk_smem<T>(mmax, nmax, kumax, kvmax, extra) <= (sizeof(T) == 4 ? kBlkSmemCap : kBlkSmemCap64);
 }
 
 namespace {
@@ -1019,7 +1028,8 @@ void launch_blk_sized(const Task* t, int64_t nt, const Slot* s, int kumax, int k
                       cudaStream_t st, bool pdl) {
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute(ulv_factor_blk_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBlkSmemCap);
+    cudaFuncSetAttribute(ulv_factor_blk_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(T) == 4 ? kBlkSmemCap : kBlkSmemCap64));
     attr_set = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -1041,11 +1051,17 @@ void launch_ulv_factor_blk(const Task* t, int64_t nt, const Slot* s, int mmax, i
                            size_t extra, cudaStream_t st, bool pdl) {
   if (nt <= 0) return;
   const size_t smem = factor_blk_smem<T>(mmax, nmax, kumax, kvmax, extra);
-  switch (size_bucket(mmax, nmax)) {
-    case 32: launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
-    case 64: launch_blk_sized<T, 64>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
-    case 96: launch_blk_sized<T, 96>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
-    default: launch_blk_sized<T, 128>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+  const int bucket = size_bucket<T>(mmax, nmax);
+  if constexpr (sizeof(T) == 8) {
+    if (bucket == 32) launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st, pdl);
+    else launch_blk_sized<T, 48>(t, nt, s, kumax, kvmax, extra, smem, st, pdl);
+  } else {
+    switch (bucket) {
+      case 32: launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+      case 64: launch_blk_sized<T, 64>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+      case 96: launch_blk_sized<T, 96>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+      default: launch_blk_sized<T, 128>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+    }
   }
 }
 
@@ -1053,5 +1069,8 @@ template bool factor_blk_fits<float>(int, int, int, int, size_t);
 template size_t factor_blk_smem<float>(int, int, int, int, size_t);
 template void launch_ulv_factor_blk<float>(const Task*, int64_t, const Slot*, int, int, int, int, size_t,
                                            cudaStream_t, bool);
+template bool factor_blk_fits<double>(int, int, int, int, size_t);
+template void launch_ulv_factor_blk<double>(const Task*, int64_t, const Slot*, int, int, int, int, size_t,
+                                            cudaStream_t, bool);
 
 }  // namespace hss

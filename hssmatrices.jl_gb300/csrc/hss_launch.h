@@ -122,7 +122,8 @@ void launch_pqr(const PqrTask* tasks, int64_t count, int qmax, int kmax, cudaStr
 template <typename T>
 void launch_ulv_factor(const Task* t, int64_t ntasks, const Slot* s, int max_m, int max_n,
                        cudaStream_t st);
-// Blocked on-chip factor kernel (hss_factor_blk.cu), T = float: two blocks per SM;
+// Blocked on-chip factor kernel (hss_factor_blk.cu), FP32 up to 128 x 128, FP64 up to
+// 40 x 40: two blocks per SM;
 // `extra` = merge staging elements; pdl: a programmatic dependent of the launch
 // before it (the level below).
 template <typename T>

@@ -1,5 +1,6 @@
-"""The FP32 reduction of levels of at most 64 x 64 nodes (``hss_factor_blk.cu``), one
-mbarrier per reflector, and solve lists that hold nodes on both sides of 64 rows.
+"""The reduction of FP32 levels of at most 64 x 64 nodes and FP64 levels of at most
+40 x 40 (``hss_factor_blk.cu``), one mbarrier per reflector, and solve lists that hold
+nodes on both sides of 64 rows.
 
 Ranks at the edges of the 32-reflector panel and of the 8-lane groups (a rank of 33
 takes the general path), nodes of 62 to 66 rows, and forests of trees of different
@@ -27,6 +28,21 @@ def test_merges(pkg, orc, n, ls, k):
     F = pkg.ulvfactor(pkg.HssMatrix.from_tree(h), "fp32")
     for _ in range(2):
         assert rel(F.solve(b, tol=1e-10, maxit=3), ref) <= 1e-8   # raises unless it converged
+        F.refactor()
+
+
+@pytest.mark.parametrize("n,ls,k", [(512, 64, 16), (600, 50, 7), (260, 32, 1), (320, 20, 16), (512, 64, 17),
+                                    (320, 40, 8), (320, 40, 7), (328, 41, 9), (320, 40, 33)])
+def test_merges_fp64(pkg, orc, n, ls, k):
+    """FP64 levels of at most 40 x 40 nodes (ranks of 7 and 33 at 40 rows have more than
+    one panel and go to the panel kernels, as do 41 rows): 1e-12."""
+    rng = np.random.default_rng(n + k)
+    h = orc.synthetic_hss(n, ls, k, rng)
+    b = rng.standard_normal((n, 3))
+    ref = orc.ulvfactsolve(h, b)
+    F = pkg.ulvfactor(pkg.HssMatrix.from_tree(h), "fp64")
+    for _ in range(2):
+        assert rel(F.solve(b), ref) <= 1e-12
         F.refactor()
 
 
