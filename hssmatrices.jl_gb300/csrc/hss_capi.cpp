@@ -766,6 +766,7 @@ int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
     f.lev[level] = FlatLevel{(const FlatGroup*)(P->d_flat + at[level][0]), (const FlatBranch*)(P->d_flat + at[level][1]),
                              ng[level], nbr[level]};
   f.nodes = P->d_nodes;
+  for (int64_t t = 0; t < nl; ++t) f.leaf_elems += (int64_t)N[leaf_node(t)].gm * N[leaf_node(t)].gn;
   f.links = (const FlatLink*)P->d_flat;
   f.dep = dep;
   return HSS_OK;
@@ -1379,8 +1380,9 @@ int check_cols(hss_plan_s* P, const std::vector<Cols>& io, bool solve) {
 // with entries x columns at the FP64 pipe's rate: n = 65536, k = 32 (15.7 M entries)
 // 286 -> 200 us at r = 6, 948 -> 293 at 32, 1838 -> 422 at 64.  Where the flat product
 // applies, the line is its estimate against the tensor-core product's (launches,
-// slices, blocks; fitted as the flat product's), with a tenth for the slices; both
-// sides measured, flat / tensor cores in us: n = 32768 r = 4 110 / 143, r = 5 155 /
+// slices, blocks; fitted as the flat product's) and an eighth of what making the
+// slices takes (545 us at 15.7 M entries, 140 at 2 M); both sides measured, flat /
+// tensor cores in us: n = 32768 r = 4 110 / 143, r = 5 155 /
 // 143; n = 16384 r = 8 110 / 110, r = 10 155 / 114; n = 8192 r = 12 85 / 93, r = 16
 // 111 / 100; n = 10007, leaves of 39 rows, r = 16 108 / 136, r = 20 179 / 154; n = 4000,
 // leaves of 250 rows, r = 8 61 / 79, r = 10 104 / 81; n = 2048 r = 32 60 / 72.  Elsewhere
@@ -1395,7 +1397,8 @@ bool oz_product_pays(const hss_plan_s* P, int64_t r) {
     return P->gen_len * r >= (P->pmv_kmax >= 16 ? 16000000 : 45000000);
   const double launches = 2.0 * (double)P->by_d.size() - 1.0, gen = (double)P->gen_len;
   const double oz = (6.3 * launches + 2.6e-6 * gen + 0.086 * (double)P->leaves.cnt) * (1.0 + (double)r / 128.0);
-  return pmv_flat_estimate(P->flat, P->leaves.cnt, P->gen_len, (int)r, sm_count(P->device)) > 1.1 * oz;
+  const double slices = 80.0 + 30e-6 * gen;
+  return pmv_flat_estimate(P->flat, P->leaves.cnt, P->gen_len, (int)r, sm_count(P->device)) > oz + slices / 8;
 }
 
 int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double beta,

@@ -749,12 +749,14 @@ bool pmv_flat_fits(const FlatTables& f, int64_t gen, int nleaf, int kmax, int rm
 }
 
 // Estimated time in us: the chain's latency per pass over the groups, and 0.34 ns per
-// multiply-add of the group that one SM carries (both fitted to trees of 8 to 1024
-// leaves of 64 to 250 rows at 1 to 32 columns, within 20 %).
+// multiply-add of an SM, its groups' tree part and its share of the leaf products
+// (fitted to trees of 8 to 1024 leaves of 15 to 250 rows at 1 to 32 columns, within
+// 25 %).
 double pmv_flat_estimate(const FlatTables& f, int64_t nleaves, int64_t gen, int rmax, int sms) {
   const FlatShape s = flat_shape(f, rmax, sms);
   const double passes = std::ceil((double)f.lev[s.level].ngroup * s.nchunk / sms);
-  return passes * (35.0 + 0.34e-3 * (1 << s.level) * s.nc * ((double)gen / (double)nleaves));
+  const double tree = passes * (1 << s.level) * s.nc * (double)(gen - f.leaf_elems) / (double)nleaves;
+  return 50.0 * passes - 15.0 + 0.34e-3 * (tree + (double)f.leaf_elems * rmax / sms);
 }
 
 void pmv_flat_space(const FlatTables& f, int64_t nleaves, int kmax, int rmax, int sms, int64_t* ctb, int64_t* counters) {

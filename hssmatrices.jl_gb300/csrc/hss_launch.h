@@ -90,6 +90,7 @@ struct FlatTables {
   const FlatLink* links = nullptr;
   FlatLevel lev[kFlatLevels];
   int32_t dep = 0;   // 0: the product does not apply to the plan
+  int64_t leaf_elems = 0;   // entries of the leaves' D
 };
 bool pmv_flat_fits(const FlatTables& f, int64_t gen, int nleaf, int kmax, int rmax, int sms);
 double pmv_flat_estimate(const FlatTables& f, int64_t nleaves, int64_t gen, int rmax, int sms);
