@@ -240,6 +240,9 @@ def randcompress_adaptive(A, rcl, ccl, opts=None, kest=10, rng=None, stats=None,
     comp = Compressor(rcl, ccl)
     k, r, bs = kest, opts.noversampling, opts.stepsize
     sp = _SamplePrecision(Ad, sample_precision)
+    # the library's calls below are on the default stream, the tensor operations
+    # between them on the caller's current one
+    mine, lib = torch.cuda.current_stream(Ad.t.device), torch.cuda.default_stream(Ad.t.device)
     # Columns are drawn (1.6 ms for 20 of 16384, and as much again to transpose and
     # copy them) while the sample product before them runs, in the order of their use.
     with sp:
@@ -258,6 +261,7 @@ def randcompress_adaptive(A, rcl, ccl, opts=None, kest=10, rng=None, stats=None,
             Scol_t = comp.sample(Ad, Ocol_t)
         nrm = math.sqrt(1.0 / bs) * math.sqrt(sumsq(Scol_t))
         E = Scol_t.clone()
+        lib.wait_stream(mine)
         dev.matmul_device(Ocol_t, n, bs, E, m, alpha=-1.0, beta=1.0)
         nrm_est = math.sqrt(1.0 / bs) * math.sqrt(sumsq(E))
         failed = nrm_est > opts.atol and nrm_est > opts.rtol * nrm
@@ -270,10 +274,12 @@ def randcompress_adaptive(A, rcl, ccl, opts=None, kest=10, rng=None, stats=None,
             Orow_t = _cols_to_device(Orow_t)
             with sp:
                 Srow_t = comp.sample(Ad, Orow_t, trans=True)
+            mine.wait_stream(lib)
             Ocol = torch.cat([Ocol, Ocol_t], dim=0)
             Orow = torch.cat([Orow, Orow_t], dim=0)
             Scol = torch.cat([Scol, Scol_t], dim=0)
             Srow = torch.cat([Srow, Srow_t], dim=0)
+            lib.wait_stream(mine)
             k += bs
     if dev is None:   # kest >= n: the block diagonal alone (hss_blkdiag, :447-475)
         z = torch.zeros((0, m), dtype=torch.float64, device=Ad.t.device)
