@@ -926,7 +926,7 @@ def run_matvec_workload(args):
                 lib.hss_set_option(3, 0)
         diff = float(np.linalg.norm(res.pop("C") - res.pop("C_level")))
         out[r] = dict(res, algorithmic_bytes=alg, paths_rel_diff=diff / max(1e-300, float(torch.linalg.norm(dC))),
-                      kernel="pmv_flat_kernel" if r <= 4 else "pmv_kernel<PF64>")
+                      kernel="pmv_flat_kernel" if r <= 4 else "ozmv_kernel (tensor cores, one launch per level)")
     clk = clocks.stop()
     g1 = out[1]["persistent"]["gbs"]
     # full(hssA) on the device (src/hssmatrix.jl:270-305) for an n = 16384 tree
@@ -1001,7 +1001,7 @@ def run_matvec_workload(args):
                      "frac": g1 / peak, "peak_source": peak_src,
                      "traffic": MATVEC_R1_TRAFFIC.get((n, args.leafsize, args.rank)),
                      "traffic_source": "ncu capture of one r = 1 launch at this size",
-                     "note": "FP64 products of <= 4 columns run the flat persistent kernel, wider ones pmv_kernel<PF64>"},
+                     "note": "FP64 products of <= 4 columns run the flat persistent kernel, wide ones the tensor-core product"},
         "by_rhs": {str(r): v for r, v in out.items()}, "clocks": clk,
         "full_n16384": {"ms": full_ms, "written_gbs": nf * nf * 8 / (full_ms * 1e-3) / 1e9,
                         "fp64_tflops": 2.0 * nf * nf * args.rank / (full_ms * 1e-3) / 1e12},

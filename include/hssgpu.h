@@ -291,9 +291,10 @@ int64_t hss_launch_counter(void);
  * kernel against it); 0 (default) picks the on-chip kernel where it fits.
  * HSS_OPT_RESIDUAL_FP64 = 1 forms the refinement residual of an FP32 factor
  * with the product on the FP64 pipe instead of the default tensor-core product.
- * HSS_OPT_LEVEL_PRODUCT = 1 runs every product with one kernel launch per
- * tree level instead of the default single persistent launch (leaves up to
- * 512 columns, ranks up to 64); used to test the two against each other.
+ * HSS_OPT_LEVEL_PRODUCT = 1 runs every product with one FP64 kernel launch per
+ * tree level instead of the default (a single persistent launch for leaves up
+ * to 512 columns and ranks up to 64, or one tensor-core launch per level);
+ * used to test them against each other.
  * HSS_OPT_GRAPHS = 1 replays the per-level launch sequences of factorizations
  * and solve passes issued on a non-default stream as CUDA graphs: the second
  * call with unchanged task lists, buffers and sizes is captured, later ones
@@ -308,10 +309,10 @@ int64_t hss_launch_counter(void);
  * within float's exponent range): the mixed-precision form of the sampling
  * in randcompress.  0 (default): FP64.
  * HSS_OPT_FLAT_PRODUCT = 0 turns off the flat form of the persistent FP64
- * product (1, default: FP64 products of at most 4 columns run it, with every
- * leaf carrying its own chain of translator products and two grid barriers
- * in place of the tree's dependency chain); used to test the two forms
- * against each other.
+ * product (1, default: FP64 products of at most 4 columns run it, and of up to
+ * 32 where the multiply-adds are few enough; a block takes a group of leaves
+ * through the tree, with two waits for all blocks in place of the tree's
+ * dependency chain); used to test the two forms against each other.
  * HSS_OPT_POLL_LIMIT = p sets how many times a block of the persistent
  * products polls for ready work before it gives up, records a device status
  * and exits (0: the default, 2^22 polls, i.e. seconds).  The next
