@@ -21,7 +21,7 @@
 // What bounds it now: cutting A into digits, about 45 integer instructions per
 // entry (ALU pipe 52 % busy, tensor pipe 20 %, DRAM 17 %); per chunk of 128 x 128
 // about 12 us.  Measured (one GB300, L2 cold): 8192 x 8192, 30 columns 3750 ->
-// 425 us; 16384 x 16384, 20 columns 9500 -> 1380 us (1.55 TB/s of A); 4096 x
+// 444 us; 16384 x 16384, 20 columns 9500 -> 1380 us (1.55 TB/s of A); 4096 x
 // 4096, 20 columns 604 -> 122 us.  Error against exact sums, relative to
 // 2^-53 (|A| |X|), root mean square: 0.46 -> 0.17 (Cauchy kernel, 2048 points),
 // 0.13 -> 0.05 (normal entries); leaving out the products with d = 8 gave 0.91
