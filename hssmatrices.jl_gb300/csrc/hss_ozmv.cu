@@ -24,7 +24,8 @@
 // The 200 KB ring leaves one block per SM.  A launch after the first of a product
 // starts while the one before it ends (programmatic dependent launch): its set-up
 // and its first copies of A's slices, which no launch writes, come before the
-// wait for the previous step's outputs.  Waits
+// wait for the previous step's outputs; every block waits for that step before it
+// ends, so that the chain of launches stays whole where a level has no units.  Waits
 // are bounded: one that runs out records DEV_TIMEOUT and the block ends once
 // its copies and MMAs have.
 //
@@ -591,6 +592,9 @@ __global__ void __launch_bounds__(OT, 1) ozmv_kernel(const Task* __restrict__ ta
       }
     }
   }
+  // in every block, units or not: the launch after this one waits for this grid only,
+  // so a grid of empty units (a level of rank 0) must not end before the one before it
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(R::tmem));
