@@ -18,6 +18,7 @@
 #include "hss_host.h"
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_levels.h"
 #include "hss_sample.h"
 
 using namespace hss;
@@ -105,79 +106,6 @@ struct SlotTable {
     return e;
   }
 };
-
-struct Seg {
-  int64_t off = 0, cnt = 0;
-  int mmax = 0, nmax = 0, kumax = 0, kvmax = 0;   // largest node of the list
-  int c1u = 0, c2u = 0, c1v = 0, c2v = 0;          // largest children's ranks (branches)
-  int kmax = 0, mkmax = 0;                         // largest ULV k and m - k
-  int c1mr = 0, c2mr = 0, c1nr = 0, c2nr = 0;      // largest children's reduced sizes
-  int64_t sv_stage = 0;                            // largest upward-solve staging need
-  int mk_in = 0, rootmax = 0;                      // largest m - k of the nodes that are not roots; largest root
-  int smin = INT32_MAX;                            // smallest node: its larger side
-  bool leaves = false, branches = false;           // kinds of node in the list
-  std::vector<Seg> parts;                          // the list by size of node (empty: one size class)
-};
-
-// Size class of a node for the factor and solve kernels, whose registers and
-// shared memory are laid out for the largest node of a launch.
-inline int size_class(const Node& x) {
-  const int s = std::max(x.m, x.n);
-  return s <= 32 ? 0 : s <= 64 ? 1 : s <= 96 ? 2 : s <= 128 ? 3 : s <= 256 ? 4 : 5;
-}
-
-// Counts node x (children in `nodes`) into the largest sizes of a list.
-inline void seg_add(Seg& v, const Node& x, const Node* nodes) {
-  ++v.cnt;
-  v.smin = std::min(v.smin, std::max(x.m, x.n));
-  v.mmax = std::max(v.mmax, x.m);
-  v.nmax = std::max(v.nmax, x.n);
-  v.kumax = std::max(v.kumax, x.ku);
-  v.kvmax = std::max(v.kvmax, x.kv);
-  v.kmax = std::max(v.kmax, x.root ? 0 : x.k);
-  v.mkmax = std::max(v.mkmax, x.mk);
-  if (x.root) v.rootmax = std::max(v.rootmax, x.m);
-  else v.mk_in = std::max(v.mk_in, x.mk);
-  (x.leaf ? v.leaves : v.branches) = true;
-  const Node* a = x.leaf ? nullptr : &nodes[x.left];
-  const Node* b = x.leaf ? nullptr : &nodes[x.right];
-  v.sv_stage = std::max(v.sv_stage, solve_up_stage_need(x.m, x.k, x.mk, x.nk, x.kv, x.leaf, x.root, a ? a->mr : 0,
-                                                        b ? b->mr : 0, a ? a->kv : 0, b ? b->kv : 0));
-  if (x.leaf) return;
-  v.c1u = std::max(v.c1u, a->ku);
-  v.c2u = std::max(v.c2u, b->ku);
-  v.c1v = std::max(v.c1v, a->kv);
-  v.c2v = std::max(v.c2v, b->kv);
-  v.c1mr = std::max(v.c1mr, a->mr);
-  v.c2mr = std::max(v.c2mr, b->mr);
-  v.c1nr = std::max(v.c1nr, a->nr);
-  v.c2nr = std::max(v.c2nr, b->nr);
-}
-
-// The list v (tasks off .. off + cnt of `tasks`) ordered by size class, with a part
-// per class where there are several; nodes(i): the node array of its i-th task.
-template <class F>
-void seg_split(Seg& v, std::vector<Task>& tasks, F&& nodes) {
-  v.parts.clear();
-  bool one = true;
-  std::vector<std::pair<int, int64_t>> key((size_t)v.cnt);
-  for (int64_t i = 0; i < v.cnt; ++i) {
-    key[i] = {size_class(nodes(i)[tasks[v.off + i].node]), i};
-    one = one && key[i].first == key[0].first;
-  }
-  if (one) return;
-  std::stable_sort(key.begin(), key.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-  const std::vector<Task> old(tasks.begin() + v.off, tasks.begin() + v.off + v.cnt);
-  for (int64_t i = 0; i < v.cnt; ++i) {
-    if (i == 0 || key[i].first != key[i - 1].first) {
-      v.parts.emplace_back();
-      v.parts.back().off = v.off + i;
-    }
-    tasks[v.off + i] = old[key[i].second];
-    const Node* nd = nodes(key[i].second);
-    seg_add(v.parts.back(), nd[old[key[i].second].node], nd);
-  }
-}
 
 inline int64_t align16(int64_t x) { return (x + 15) & ~int64_t(15); }
 
@@ -856,29 +784,6 @@ int build_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, bool device_fill
 // launch sequences
 // ---------------------------------------------------------------------------
 
-// The task lists one launch sequence walks: a plan's own (slot = tree of the
-// forest) or lists merged over several single-tree plans (slot = item).
-struct Levels {
-  const Task* d_tasks = nullptr;
-  const std::vector<Seg>* by_h = nullptr;
-  const std::vector<Seg>* by_d = nullptr;
-  const std::vector<Seg>* mv_up = nullptr;
-  const std::vector<Seg>* mv_dn = nullptr;
-  Seg leaves;
-  // persistent product: largest leaf columns / rows, largest rank, non-root nodes
-  int nleaf = 0, mleaf = 0, kmax = 0;
-  int64_t ntasks = 0;
-  int64_t nodes_max = 0, nslots = 0;   // largest node array of a slot's plan; slots
-  int64_t ninner = 0;                  // non-root branches
-  int device = 0;
-  FlatTables flat;   // flat product tables (dep = 0: not available)
-  int64_t gen_len = 0;
-  // translators to prefetch into L2 (FP64 and pair copies; null: none)
-  const double* pf64 = nullptr;
-  const float2* pfdf = nullptr;
-  int64_t pf_elems = 0;
-};
-
 Levels plan_levels(const hss_plan_s* P) {
   Levels L;
   L.d_tasks = P->d_tasks;
@@ -1432,29 +1337,6 @@ int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double
   if (rc) return rc;
   CUDA_TRY(cudaGetLastError());
   return HSS_OK;
-}
-
-inline uint64_t fnv(uint64_t h, uint64_t v) {
-  for (int i = 0; i < 8; ++i) {
-    h ^= (v >> (8 * i)) & 0xffu;
-    h *= 1099511628211ull;
-  }
-  return h;
-}
-
-// Key of a launch sequence over task lists L with the device slot table `slots`.
-uint64_t levels_key(const Levels& L, const void* slots, int64_t extra) {
-  uint64_t h = 1469598103934665603ull;
-  h = fnv(h, (uint64_t)(uintptr_t)L.d_tasks);
-  h = fnv(h, (uint64_t)(uintptr_t)slots);
-  h = fnv(h, (uint64_t)extra);
-  for (const std::vector<Seg>* v : {L.by_h, L.by_d})
-    for (const Seg& g : *v) {
-      const int64_t f[] = {g.off, g.cnt, g.mmax, g.nmax, g.kumax, g.kvmax, g.c1u, g.c2u, g.c1v, g.c2v,
-                           g.kmax, g.mkmax, g.c1mr, g.c2mr, g.c1nr, g.c2nr, g.sv_stage};
-      for (int64_t x : f) h = fnv(h, (uint64_t)x);
-    }
-  return h;
 }
 
 // Runs `launch` (which issues kernels on st and returns a flag) directly or,
