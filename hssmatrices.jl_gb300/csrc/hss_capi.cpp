@@ -1454,7 +1454,7 @@ int solve_prep(const std::vector<Item>& items, const Levels& L, const double* sc
   uint64_t key = levels_key(L, table.dev.p, rmax * 64 + (blocked ? 1 : 0) + (sizeof(T) == 4 ? 2 : 0));
   if (tf)
     for (const std::vector<int8_t>* v : {&tf->tune_up, &tf->tune_down})
-      for (int8_t c : *v) key = fnv(key, (uint64_t)(c + 2));
+      for (int8_t c : *v) key = mix(key, (uint64_t)(c + 2));
   pp.key = key;
   return HSS_OK;
 }
@@ -1534,10 +1534,10 @@ int factsolve_prep(hss_factor_s* f, const std::vector<Item>& items, const Levels
     CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     f->pipe_ev.push_back(e);
   }
-  uint64_t key = fnv(levels_key(L, f->fac_slots.dev.p, (int64_t)sizeof(T) + (g_generic_factor ? 16 : 0)),
+  uint64_t key = mix(levels_key(L, f->fac_slots.dev.p, (int64_t)sizeof(T) + (g_generic_factor ? 16 : 0)),
                      levels_key(L, table.dev.p, rmax * 64 + (pp.blocked ? 1 : 0) + (sizeof(T) == 4 ? 2 : 0)));
   for (const std::vector<int8_t>* v : {&f->tune_up, &f->tune_down})
-    for (int8_t c : *v) key = fnv(key, (uint64_t)(c + 2));
+    for (int8_t c : *v) key = mix(key, (uint64_t)(c + 2));
   pp.key = key;
   // the solves that follow (and the correction passes of a refinement) read
   // this factorization's kind
@@ -1852,11 +1852,11 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
     CUDA_TRY(B.status.ensure(4));
     CUDA_TRY(B.h_status.ensure(4));
     // every address and choice the recorded launches hold
-    uint64_t key = fnv(fnv(p0.key, p1.key), levels_key(L, B.mv.dev.p, rmax));
+    uint64_t key = mix(mix(p0.key, p1.key), levels_key(L, B.mv.dev.p, rmax));
     for (const Item& it : items)
       for (uint64_t v : {(uint64_t)(uintptr_t)it.f, (uint64_t)it.tree, (uint64_t)(uintptr_t)it.io.B,
                          (uint64_t)it.io.ldb, (uint64_t)(uintptr_t)it.io.C, (uint64_t)it.io.ldc, (uint64_t)it.io.r})
-        key = fnv(key, v);
+        key = mix(key, v);
     double tolv = tol;
     uint64_t tolbits = 0;
     std::memcpy(&tolbits, &tolv, sizeof(tolbits));
@@ -1869,7 +1869,7 @@ int solve_items(const std::vector<Item>& items, const Levels& L, SolveBufs& B, d
                        (uint64_t)(uintptr_t)B.bn2.p, (uint64_t)(uintptr_t)B.rn2.p, (uint64_t)(uintptr_t)B.scale.p,
                        (uint64_t)(uintptr_t)B.R.p, (uint64_t)(uintptr_t)B.xs.p, (uint64_t)(uintptr_t)B.tmp.p,
                        (uint64_t)(uintptr_t)B.status.p})
-      key = fnv(key, v);
+      key = mix(key, v);
     GraphCache& gc = B.loop;
     RefineStatus* dst = (RefineStatus*)B.status.p;
     auto issue_check = [&](cudaGraphConditionalHandle cond) {

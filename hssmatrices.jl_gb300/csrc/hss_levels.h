@@ -12,7 +12,8 @@
 
 namespace hss {
 
-// A list of tasks, with the largest sizes of its nodes.
+// A list of tasks, with the largest sizes of its nodes.  Every field shapes launches:
+// a new one also goes into seg_key.
 struct Seg {
   int64_t off = 0, cnt = 0;
   int mmax = 0, nmax = 0, kumax = 0, kvmax = 0;   // largest node of the list
@@ -115,26 +116,40 @@ struct Levels {
   int64_t pf_elems = 0;
 };
 
-inline uint64_t fnv(uint64_t h, uint64_t v) {
-  for (int i = 0; i < 8; ++i) {
-    h ^= (v >> (8 * i)) & 0xffu;
-    h *= 1099511628211ull;
-  }
+// A word mixed into a key.
+inline uint64_t mix(uint64_t h, uint64_t v) {
+  h = (h ^ v) * 0x9E3779B97F4A7C15ull;
+  return h ^ (h >> 29);
+}
+
+// A list's share of a key: the list, its sizes, and its parts.
+inline uint64_t seg_key(uint64_t h, const Seg& g) {
+  for (int64_t x : {g.off, g.cnt, g.sv_stage}) h = mix(h, (uint64_t)x);
+  for (int x : {g.mmax, g.nmax, g.kumax, g.kvmax, g.c1u, g.c2u, g.c1v, g.c2v, g.kmax, g.mkmax, g.c1mr, g.c2mr, g.c1nr,
+                g.c2nr, g.mk_in, g.rootmax, g.smin, (int)g.leaves, (int)g.branches})
+    h = mix(h, (uint64_t)(int64_t)x);
+  h = mix(h, g.parts.size());
+  for (const Seg& p : g.parts) h = seg_key(h, p);
   return h;
 }
 
-// Key of a launch sequence over task lists L with the device slot table `slots`.
+// Key of a launch sequence over task lists L with the device slot table `slots`: all
+// that the launches take from L.  (The task buffer's contents are read when a recorded
+// sequence runs, its lists' offsets and sizes are part of the recording: a batcher
+// keeps its buffers' addresses from one batch to the next.)
 inline uint64_t levels_key(const Levels& L, const void* slots, int64_t extra) {
   uint64_t h = 1469598103934665603ull;
-  h = fnv(h, (uint64_t)(uintptr_t)L.d_tasks);
-  h = fnv(h, (uint64_t)(uintptr_t)slots);
-  h = fnv(h, (uint64_t)extra);
-  for (const std::vector<Seg>* v : {L.by_h, L.by_d})
-    for (const Seg& g : *v) {
-      const int64_t f[] = {g.off, g.cnt, g.mmax, g.nmax, g.kumax, g.kvmax, g.c1u, g.c2u, g.c1v, g.c2v,
-                           g.kmax, g.mkmax, g.c1mr, g.c2mr, g.c1nr, g.c2nr, g.sv_stage};
-      for (int64_t x : f) h = fnv(h, (uint64_t)x);
-    }
+  for (const void* p : {(const void*)L.d_tasks, slots, (const void*)L.pf64, (const void*)L.pfdf,
+                        (const void*)L.flat.links})
+    h = mix(h, (uint64_t)(uintptr_t)p);
+  for (int64_t x : {extra, (int64_t)L.nleaf, (int64_t)L.mleaf, (int64_t)L.kmax, L.ntasks, L.nodes_max, L.nslots,
+                    L.ninner, (int64_t)L.device, L.gen_len, L.pf_elems, (int64_t)L.flat.dep, L.flat.leaf_elems})
+    h = mix(h, (uint64_t)x);
+  h = seg_key(h, L.leaves);
+  for (const std::vector<Seg>* v : {L.by_h, L.by_d, L.mv_up, L.mv_dn}) {
+    h = mix(h, v->size());
+    for (const Seg& g : *v) h = seg_key(h, g);
+  }
   return h;
 }
 

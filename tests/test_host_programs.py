@@ -25,6 +25,6 @@ def run(tmp_path, name, link):
     assert out.returncode == 0 and out.stdout == "", out.stdout + out.stderr
 
 
-@pytest.mark.parametrize("name", ["levels_split"])
+@pytest.mark.parametrize("name", ["levels_split", "levels_key"])
 def test_linked(lib, tmp_path, name):
     run(tmp_path, name, link=True)
