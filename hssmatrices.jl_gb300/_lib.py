@@ -39,6 +39,7 @@ HSS_OPT_FLAT_PRODUCT = 6
 HSS_OPT_POLL_LIMIT = 7
 HSS_OPT_FAIL_ALLOC = 8
 HSS_OPT_TENSOR_RESIDUAL = 9
+HSS_OPT_FAIL_LAUNCH = 10
 
 NODE_FIELDS = 16
 CLUSTER_FIELDS = 6

@@ -51,7 +51,6 @@ struct GraphCache {
   uint64_t key = 0, seen = 0;     // seen: key of the last uncaptured run
   cudaGraphExec_t exec = nullptr;
   int64_t launches = 0;           // kernel launches inside the graph
-  bool flag = false;              // a result of the captured run (factor: every level fast)
   GraphCache() = default;
   GraphCache(const GraphCache&) = delete;
   GraphCache& operator=(const GraphCache&) = delete;
@@ -1061,9 +1060,11 @@ void run_parts(const Levels& L, const Seg& g, F&& f, bool split = false) {
   add_launches((int64_t)g.parts.size() - 1);   // traced() counts one
 }
 
-// One factor level (h = tree height); true when it ran the one-block kernel alone.
+// One factor level (h = tree height): the first error of its launches that is not left
+// to cudaGetLastError().
 template <typename T>
-bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t st) {
+cudaError_t run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
   const Seg& all = (*L.by_h)[h];
   traced(h == 0 ? HSS_TRACE_FACTOR_LEAF : HSS_TRACE_FACTOR_MERGE, all.cnt, st, [&] {
     run_parts(L, all, [&](const Seg& g) {
@@ -1072,7 +1073,9 @@ bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t
         d.mmax = g.mmax; d.nmax = g.nmax; d.kmax = g.kmax; d.mkmax = g.mk_in; d.kvmax = g.kvmax; d.rootmax = g.rootmax;
         d.leaves = g.leaves; d.branches = g.branches;
         int launches = 0;
-        launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
+        const cudaError_t le =
+            launch_ulv_factor_pan<T>(L.d_tasks + g.off, g.cnt, slots, d, sm_count(L.device), &launches, st);
+        if (e == cudaSuccess) e = le;
         add_launches(launches - 1);
       } else if (factor_level_fast<T>(g)) {
         launch_ulv_factor_blk<T>(L.d_tasks + g.off, g.cnt, slots, g.mmax, g.nmax, g.kumax, g.kvmax,
@@ -1082,14 +1085,22 @@ bool run_factor_level(const Levels& L, size_t h, const Slot* slots, cudaStream_t
       }
     });
   });
-  return sizeof(T) == 4 && factor_level_fast<T>(all);
+  return e;
 }
 
 template <typename T>
-bool run_factor(const Levels& L, const Slot* slots, cudaStream_t st) {
-  bool all_fast = true;
-  for (size_t h = 0; h < L.by_h->size(); ++h) all_fast = run_factor_level<T>(L, h, slots, st) && all_fast;
-  return all_fast;
+cudaError_t run_factor(const Levels& L, const Slot* slots, cudaStream_t st) {
+  cudaError_t e = cudaSuccess;
+  for (size_t h = 0; h < L.by_h->size() && e == cudaSuccess; ++h) e = run_factor_level<T>(L, h, slots, st);
+  return e;
+}
+
+// Whether the blocked solve can read the factors: FP32, every level of the one-block kernel.
+template <typename T>
+bool factor_blocked(const Levels& L) {
+  bool all = sizeof(T) == sizeof(float);
+  for (const Seg& g : *L.by_h) all = all && factor_level_fast<T>(g);
+  return all;
 }
 
 // Largest rank a level's blocked solve stages (its own and its children's).
@@ -1339,15 +1350,21 @@ int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double
   return HSS_OK;
 }
 
-// Runs `launch` (which issues kernels on st and returns a flag) directly or,
-// with graphs enabled on a non-default stream, as a replayed CUDA graph: the
-// second run with an unchanged key is captured and every later one replays it.
+// Runs `launch` (which issues kernels on st) directly or, with graphs enabled on a
+// non-default stream, as a replayed CUDA graph: the second run with an unchanged key
+// is captured and every later one replays it.  A sequence with a failed launch is not
+// kept.
 template <typename F>
-int graphed(GraphCache& gc, uint64_t key, cudaStream_t st, bool& flag, F&& launch, unsigned inst_flags = 0) {
+int graphed(GraphCache& gc, uint64_t key, cudaStream_t st, const char* what, F&& launch, unsigned inst_flags = 0) {
   const bool can = g_graphs && st != nullptr && g_trace.kind < 0 && g_pick_force < 0;
+  auto issue = [&]() -> cudaError_t {
+    const cudaError_t e = launch(), l = cudaGetLastError();
+    return e != cudaSuccess ? e : l;
+  };
   if (!can || (gc.key != key && gc.seen != key)) {
+    const cudaError_t e = issue();
+    if (e != cudaSuccess) return cuda_fail(e, what);
     if (can) gc.seen = key;
-    flag = launch();
     return HSS_OK;
   }
   if (gc.key != key) {
@@ -1356,9 +1373,14 @@ int graphed(GraphCache& gc, uint64_t key, cudaStream_t st, bool& flag, F&& launc
     CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     int64_t captured = 0;
     t_capture = &captured;
-    const bool fl = launch();
+    const cudaError_t le = issue();
     t_capture = nullptr;
     const cudaError_t e = cudaStreamEndCapture(st, &g);
+    if (le != cudaSuccess) {
+      if (e == cudaSuccess) cudaGraphDestroy(g);
+      cudaGetLastError();
+      return cuda_fail(le, what);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
     const cudaError_t ie = cudaGraphInstantiate(&gc.exec, g, inst_flags);
     cudaGraphDestroy(g);
@@ -1368,11 +1390,9 @@ int graphed(GraphCache& gc, uint64_t key, cudaStream_t st, bool& flag, F&& launc
     }
     gc.key = key;
     gc.launches = captured;
-    gc.flag = fl;
   }
   CUDA_TRY(cudaGraphLaunch(gc.exec, st));
   add_launches(gc.launches);
-  flag = gc.flag;
   return HSS_OK;
 }
 
@@ -1387,12 +1407,11 @@ int factor_items(const std::vector<hss_factor_s*>& fs, const Levels& L, SlotTabl
     x.err = fs[i]->plan->d_err;
   }
   CUDA_TRY(table.upload(s, st));
-  bool fast = false;
   const uint64_t key = levels_key(L, table.dev.p, (int64_t)sizeof(T) + (g_generic_factor ? 16 : 0));
-  int rc = graphed(table.graph, key, st, fast, [&] { return run_factor<T>(L, table.dev.p, st); });
+  int rc = graphed(table.graph, key, st, "factorization launch", [&] { return run_factor<T>(L, table.dev.p, st); });
   if (rc) return rc;
-  for (auto* f : fs) f->blocked = fast && sizeof(T) == sizeof(float);
-  CUDA_TRY(cudaGetLastError());
+  const bool blocked = factor_blocked<T>(L);
+  for (auto* f : fs) f->blocked = blocked;
   return HSS_OK;
 }
 
@@ -1472,14 +1491,10 @@ int solve_pass(const std::vector<Item>& items, const Levels& L, const double* sc
   PassPrep pp;
   int rc = solve_prep<T>(items, L, scale, off, rtot, mode, residual_input, roff, R, table, st, tf, pp);
   if (rc || pp.rmax == 0) return rc;
-  bool unused = false;
-  rc = graphed(table.graph, pp.key, st, unused, [&] {
+  return graphed(table.graph, pp.key, st, "solve launch", [&] {
     solve_issue<T>(L, table, pp, st, tf);
-    return true;
+    return cudaSuccess;
   });
-  if (rc) return rc;
-  CUDA_TRY(cudaGetLastError());
-  return HSS_OK;
 }
 
 // The factorization of f's plan and the first solve pass of `items` (all on
@@ -1520,9 +1535,7 @@ int factsolve_prep(hss_factor_s* f, const std::vector<Item>& items, const Levels
     x.err = P->d_err;
   }
   CUDA_TRY(table.upload(s, st));
-  bool all_fast = true;
-  for (size_t h = 0; h < L.by_h->size(); ++h) all_fast = factor_level_fast<T>((*L.by_h)[h]) && all_fast;
-  pp.blocked = all_fast && sizeof(T) == sizeof(float);
+  pp.blocked = factor_blocked<T>(L);
   if (!f->pipe_st) CUDA_TRY(cudaStreamCreateWithFlags(&f->pipe_st, cudaStreamNonBlocking));
   if (!f->fac_st) {
     int least = 0, greatest = 0;
@@ -1565,7 +1578,7 @@ cudaError_t factsolve_issue(hss_factor_s* f, const Levels& L, const SlotTable& t
     chk(cudaStreamWaitEvent(s2, f->pipe_ev[0], 0));
   }
   for (size_t h = 0; h < L.by_h->size(); ++h) {
-    run_factor_level<T>(L, h, f->fac_slots.dev.p, sf);
+    chk(run_factor_level<T>(L, h, f->fac_slots.dev.p, sf));
     chk(cudaEventRecord(f->pipe_ev[4 + h], sf));
     chk(cudaStreamWaitEvent(s2, f->pipe_ev[4 + h], 0));
     run_solve_up_level<T>(L, h, table.dev.p, (int)pp.rmax, s2, pp.blocked, &f->tune_up, false);
@@ -1584,19 +1597,9 @@ int factsolve_pass(hss_factor_s* f, const std::vector<Item>& items, const Levels
   PassPrep pp;
   int rc = factsolve_prep<T>(f, items, L, scale, off, rtot, table, st, pp);
   if (rc) return rc;
-  bool unused = false;
-  cudaError_t ev_err = cudaSuccess;
-  rc = graphed(
-      f->pipe_graph, pp.key, st, unused,
-      [&] {
-        ev_err = factsolve_issue<T>(f, L, table, pp, st);
-        return true;
-      },
+  return graphed(
+      f->pipe_graph, pp.key, st, "pipelined factorization", [&] { return factsolve_issue<T>(f, L, table, pp, st); },
       cudaGraphInstantiateFlagUseNodePriority);
-  if (rc) return rc;
-  if (ev_err != cudaSuccess) return cuda_fail(ev_err, "pipelined factorization events");
-  CUDA_TRY(cudaGetLastError());
-  return HSS_OK;
 }
 
 int read_dev_err(hss_plan_s* P, cudaStream_t st) {
@@ -1676,6 +1679,7 @@ bool record_loop(GraphCache& gc, uint64_t key, int64_t& body_launches, cudaStrea
       ok = rc == HSS_OK && e == cudaSuccess;
     }
   }
+  ok = cudaGetLastError() == cudaSuccess && ok;   // a launch that failed is in neither recording
   cudaGraphExec_t ex = nullptr;
   // kernel nodes keep the priority of the stream they were recorded from (the
   // factorization's high-priority stream)
@@ -2151,30 +2155,33 @@ void count_launches(int64_t n) { add_launches(n); }
 // allocation from now fails.
 std::atomic<int64_t> g_fail_alloc{0};
 
+// The same for launches (HSS_OPT_FAIL_LAUNCH).
+std::atomic<int64_t> g_fail_launch{0};
+
+namespace {
+// Counts one event off an armed failure: true for the one that fails.
+bool armed_fault(std::atomic<int64_t>& left) {
+  int64_t k = left.load();
+  while (k > 0)
+    if (left.compare_exchange_weak(k, k - 1)) return k == 1;
+  return false;
+}
+}  // namespace
+
+cudaError_t launch_fault() { return armed_fault(g_fail_launch) ? cudaErrorLaunchOutOfResources : cudaSuccess; }
+
 cudaError_t dev_alloc(void** p, size_t bytes) {
-  int64_t k = g_fail_alloc.load();
-  while (k > 0) {
-    if (g_fail_alloc.compare_exchange_weak(k, k - 1)) {
-      if (k == 1) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-      }
-      break;
-    }
+  if (armed_fault(g_fail_alloc)) {
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
   }
   return cudaMalloc(p, bytes);
 }
 
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t st) {
-  int64_t k = g_fail_alloc.load();
-  while (k > 0) {
-    if (g_fail_alloc.compare_exchange_weak(k, k - 1)) {
-      if (k == 1) {
-        *p = nullptr;
-        return cudaErrorMemoryAllocation;
-      }
-      break;
-    }
+  if (armed_fault(g_fail_alloc)) {
+    *p = nullptr;
+    return cudaErrorMemoryAllocation;
   }
   // the device's default pool keeps up to 4 GB of freed blocks for reuse
   // (a setting of this process's pool, not of the device)
@@ -2534,6 +2541,11 @@ int hss_set_option(int32_t option, int64_t value) {
   if (option == HSS_OPT_FAIL_ALLOC) {
     if (value < 0) return fail(HSS_ERR_INVALID, "allocation-failure countdown must be >= 0");
     g_fail_alloc.store(value);
+    return HSS_OK;
+  }
+  if (option == HSS_OPT_FAIL_LAUNCH) {
+    if (value < 0) return fail(HSS_ERR_INVALID, "launch-failure countdown must be >= 0");
+    g_fail_launch.store(value);
     return HSS_OK;
   }
   if (option == HSS_OPT_POLL_LIMIT) {

@@ -799,38 +799,44 @@ cudaError_t launch_ulv_factor_pan(const Task* t, int64_t nt, const Slot* s, cons
   *launches = 0;
   if (nt <= 0) return cudaSuccess;
   cudaError_t e = cudaSuccess;
-  auto count = [&](cudaError_t r) {
-    if (e == cudaSuccess) e = r;
+  // the launches in order, none after one that failed
+  auto step = [&](auto launch) {
+    if (e == cudaSuccess) e = launch_fault();
+    if (e == cudaSuccess) e = launch();
     ++*launches;
   };
-  if (d.leaves) {
-    leaf_copy_kernel<T><<<dim3((unsigned)nt, 6), NT, 0, st>>>(t, s);
-    count(cudaGetLastError());
-  }
-  if (d.branches) {
-    merge_kernel<T><<<dim3((unsigned)nt, 6), NT, 0, st>>>(t, s, 0);
-    count(cudaGetLastError());
-    merge_kernel<T><<<dim3((unsigned)nt, 4), NT, 0, st>>>(t, s, 1);
-    count(cudaGetLastError());
-  }
+  if (d.leaves)
+    step([&] {
+      leaf_copy_kernel<T><<<dim3((unsigned)nt, 6), NT, 0, st>>>(t, s);
+      return cudaGetLastError();
+    });
+  for (int stage = 0; d.branches && stage < 2; ++stage)
+    step([&] {
+      merge_kernel<T><<<dim3((unsigned)nt, stage == 0 ? 6 : 4), NT, 0, st>>>(t, s, stage);
+      return cudaGetLastError();
+    });
   for (int p = 0; p * BP < d.kmax; ++p) {
-    count(panel<T, true>(t, nt, s, p, d.mmax, sms, st));
-    count(apply<T, true>(t, nt, s, p, d.nmax + std::max(0, d.kmax - BP * (p + 1)), st));
+    step([&] { return panel<T, true>(t, nt, s, p, d.mmax, sms, st); });
+    step([&] { return apply<T, true>(t, nt, s, p, d.nmax + std::max(0, d.kmax - BP * (p + 1)), st); });
   }
   for (int p = 0; p * BP < d.mkmax; ++p) {
-    count(panel<T, false>(t, nt, s, p, d.nmax, sms, st));
-    count(apply<T, false>(t, nt, s, p, d.mmax + d.kvmax, st));
+    step([&] { return panel<T, false>(t, nt, s, p, d.nmax, sms, st); });
+    step([&] { return apply<T, false>(t, nt, s, p, d.mmax + d.kvmax, st); });
   }
   if (d.rootmax > 0) {
     const int cap = (int)(200 * 1024 / sizeof(T));
     const int rows = d.rootmax * (d.rootmax | 1) <= cap ? d.rootmax : 0;
-    static bool attr_set = false;
-    if (!attr_set && e == cudaSuccess) {
-      e = cudaFuncSetAttribute(root_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cap * sizeof(T)));
-      attr_set = e == cudaSuccess;
-    }
-    root_kernel<T><<<(unsigned)nt, NT, (size_t)rows * (rows | 1) * sizeof(T), st>>>(t, s, rows);
-    count(cudaGetLastError());
+    step([&] {
+      static bool attr_set = false;
+      if (!attr_set) {
+        cudaError_t r =
+            cudaFuncSetAttribute(root_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cap * sizeof(T)));
+        if (r != cudaSuccess) return r;
+        attr_set = true;
+      }
+      root_kernel<T><<<(unsigned)nt, NT, (size_t)rows * (rows | 1) * sizeof(T), st>>>(t, s, rows);
+      return cudaGetLastError();
+    });
   }
   return e;
 }

@@ -136,12 +136,15 @@ void launch_ulv_factor_blk(const Task* t, int64_t nt, const Slot* s, int mmax, i
                            size_t extra, cudaStream_t st, bool pdl);
 // The reduction of one level by panels (hss_factor_pan.cu), FP32 or FP64, nodes up
 // to 512 x 512: largest sizes of the level's nodes (roots apart), and which kinds
-// it has.  *launches gets the number of kernels.
+// it has.  *launches gets the number of kernels; the first error of a launch is
+// returned (and is not left to cudaGetLastError()).
 struct FactorDims {
   int mmax = 0, nmax = 0, kmax = 0, mkmax = 0, kvmax = 0, rootmax = 0;
   bool leaves = false, branches = false;
 };
 bool factor_pan_fits(int mmax, int nmax);
+// The armed failure of a launch (HSS_OPT_FAIL_LAUNCH), or cudaSuccess.
+cudaError_t launch_fault();
 template <typename T>
 cudaError_t launch_ulv_factor_pan(const Task* t, int64_t nt, const Slot* s, const FactorDims& d, int sms, int* launches,
                                   cudaStream_t st);

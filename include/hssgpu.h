@@ -328,7 +328,10 @@ int64_t hss_launch_counter(void);
  * HSS_OPT_FAIL_ALLOC = k > 0 makes the k-th device allocation of this library
  * from now on fail as out of memory, on the host, before the CUDA driver is
  * called (0 disarms): fault injection for the HSS_ERR_OOM paths.  The call
- * that hits it returns HSS_ERR_OOM and leaves no partial object behind. */
+ * that hits it returns HSS_ERR_OOM and leaves no partial object behind.
+ * HSS_OPT_FAIL_LAUNCH = k > 0 makes the k-th kernel launch of a factorization by
+ * panels (FP64 nodes above 40 rows, FP32 nodes above 128) from now on fail in
+ * the same way, on the host (0 disarms); the call returns HSS_ERR_CUDA. */
 enum {
   HSS_OPT_GENERIC_FACTOR = 1,
   HSS_OPT_RESIDUAL_FP64 = 2,
@@ -338,7 +341,8 @@ enum {
   HSS_OPT_FLAT_PRODUCT = 6,
   HSS_OPT_POLL_LIMIT = 7,
   HSS_OPT_FAIL_ALLOC = 8,
-  HSS_OPT_TENSOR_RESIDUAL = 9
+  HSS_OPT_TENSOR_RESIDUAL = 9,
+  HSS_OPT_FAIL_LAUNCH = 10
 };
 int hss_set_option(int32_t option, int64_t value);
 
