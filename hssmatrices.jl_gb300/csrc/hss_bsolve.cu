@@ -20,6 +20,7 @@
 
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 
 namespace hss {
 
@@ -376,11 +377,8 @@ void launch_bsolve_up(const Task* t, int64_t nt, const Slot* s, int mmax, int nm
   if (nt <= 0 || r <= 0) return;
   const Lay ly = layout(mmax, nmax, kmax, kvmax);
   const size_t smem = (size_t)ly.total * sizeof(float);
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(bsolve_up, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBsolveSmemCap);
-    set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)bsolve_up, kBsolveSmemCap);
   const int nchunk = (r + CW - 1) / CW;
   bsolve_up<<<(unsigned)(nt * nchunk), BT, smem, st>>>(t, s, nchunk, ly);
 }
@@ -390,11 +388,8 @@ void launch_bsolve_down(const Task* t, int64_t nt, const Slot* s, int mmax, int 
   if (nt <= 0 || r <= 0) return;
   const Lay ly = layout(mmax, nmax, kmax, kvmax);
   const size_t smem = (size_t)ly.total * sizeof(float);
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(bsolve_down, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBsolveSmemCap);
-    set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)bsolve_down, kBsolveSmemCap);
   const int nchunk = (r + CW - 1) / CW;
   bsolve_down<<<(unsigned)(nt * nchunk), BT, smem, st>>>(t, s, nchunk, ly);
 }

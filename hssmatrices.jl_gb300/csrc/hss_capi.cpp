@@ -836,7 +836,7 @@ int run_pmv(const Levels& L, const Slot* slots, int rmax, bool pairs, SlotTable&
     cudaError_t e = cudaSuccess;
     traced(HSS_TRACE_MV_LEAF, L.leaves.cnt, st, [&] {
       e = launch_pmv_flat(L.flat, L.d_tasks + L.leaves.off, L.leaves.cnt, slots, rmax, L.nleaf, L.mleaf, L.kmax,
-                          pm.pstate.p, pm.ctb.p, pm.dcnt.p, L.device, sm_count(L.device), pmv_poll_limit(), st);
+                          pm.pstate.p, pm.ctb.p, pm.dcnt.p, sm_count(L.device), pmv_poll_limit(), st);
     });
     if (e != cudaSuccess) {
       cudaGetLastError();

@@ -46,6 +46,7 @@
 #include "hss_factor.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 #include "hss_oz.cuh"
 
 namespace hss {
@@ -1026,12 +1027,8 @@ namespace {
 template <typename T, int S>
 void launch_blk_sized(const Task* t, int64_t nt, const Slot* s, int kumax, int kvmax, size_t extra, size_t smem,
                       cudaStream_t st, bool pdl) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(ulv_factor_blk_kernel<T, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(T) == 4 ? kBlkSmemCap : kBlkSmemCap64));
-    attr_set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)ulv_factor_blk_kernel<T, S>, sizeof(T) == 4 ? kBlkSmemCap : kBlkSmemCap64);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)nt);
   cfg.blockDim = dim3(NT);

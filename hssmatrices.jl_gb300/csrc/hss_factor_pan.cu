@@ -39,6 +39,7 @@
 #include "hss_factor.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 #include "hss_oz.cuh"
 
 namespace hss {
@@ -751,14 +752,11 @@ __global__ void __launch_bounds__(NT) root_kernel(const Task* __restrict__ tasks
 
 template <typename T, int S, bool QL, int PL>
 cudaError_t panel_sized(const Task* t, int64_t nt, const Slot* s, int p, cudaStream_t st) {
-  static bool attr_set = false;
   constexpr size_t smem = panel_smem<T, S>();
   auto* k = panel_kernel<T, S, QL, PL>;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SmemOptIn opt_in;
+  const cudaError_t e = opt_in((const void*)k, smem);
+  if (e != cudaSuccess) return e;
   k<<<(unsigned)nt, 32 * PL, smem, st>>>(t, s, p);
   return cudaGetLastError();
 }
@@ -777,13 +775,9 @@ cudaError_t panel(const Task* t, int64_t nt, const Slot* s, int p, int len, int 
 template <typename T, bool QL>
 cudaError_t apply(const Task* t, int64_t nt, const Slot* s, int p, int rows, cudaStream_t st) {
   if (rows <= 0) return cudaSuccess;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e =
-        cudaFuncSetAttribute(apply_kernel<T, QL>, cudaFuncAttributeMaxDynamicSharedMemorySize, ApplySmem<T>::total);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SmemOptIn opt_in;
+  const cudaError_t e = opt_in((const void*)apply_kernel<T, QL>, ApplySmem<T>::total);
+  if (e != cudaSuccess) return e;
   const int ntile = (rows + TR - 1) / TR;
   apply_kernel<T, QL><<<(unsigned)(nt * ntile), AT, ApplySmem<T>::total, st>>>(t, s, p, ntile);
   return cudaGetLastError();
@@ -827,13 +821,9 @@ cudaError_t launch_ulv_factor_pan(const Task* t, int64_t nt, const Slot* s, cons
     const int cap = (int)(200 * 1024 / sizeof(T));
     const int rows = d.rootmax * (d.rootmax | 1) <= cap ? d.rootmax : 0;
     step([&] {
-      static bool attr_set = false;
-      if (!attr_set) {
-        cudaError_t r =
-            cudaFuncSetAttribute(root_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(cap * sizeof(T)));
-        if (r != cudaSuccess) return r;
-        attr_set = true;
-      }
+      static SmemOptIn opt_in;
+      const cudaError_t r = opt_in((const void*)root_kernel<T>, cap * sizeof(T));
+      if (r != cudaSuccess) return r;
       root_kernel<T><<<(unsigned)nt, NT, (size_t)rows * (rows | 1) * sizeof(T), st>>>(t, s, rows);
       return cudaGetLastError();
     });

@@ -45,6 +45,7 @@
 
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 
 namespace hss {
 
@@ -766,8 +767,8 @@ void pmv_flat_space(const FlatTables& f, int64_t nleaves, int kmax, int rmax, in
 }
 
 cudaError_t launch_pmv_flat(const FlatTables& f, const Task* leaves, int64_t nleaves, const Slot* slots, int rmax,
-                            int nleaf, int mleaf, int kmax, uint32_t* state, double* ctb, uint32_t* dcnt, int device,
-                            int sms, uint32_t idle_limit, cudaStream_t st) {
+                            int nleaf, int mleaf, int kmax, uint32_t* state, double* ctb, uint32_t* dcnt, int sms,
+                            uint32_t idle_limit, cudaStream_t st) {
   if (nleaves <= 0) return cudaSuccess;
   const FlatShape shape = flat_shape(f, rmax, sms);
   const FlatLevel& lv = f.lev[shape.level];
@@ -794,13 +795,9 @@ cudaError_t launch_pmv_flat(const FlatTables& f, const Task* leaves, int64_t nle
   a.nbuf = flat_bytes(nleaf, a.km, f.dep, nc, 3) <= kFlatSmemCap ? 3 : 2;
   const size_t smem = flat_bytes(nleaf, a.km, f.dep, nc, a.nbuf);
   auto kern = nc == 1 ? pmv_flat_kernel<1> : nc == 2 ? pmv_flat_kernel<2> : nc == 3 ? pmv_flat_kernel<3> : pmv_flat_kernel<4>;
-  static std::atomic<bool> allowed[8][kFlatCw + 1];
-  std::atomic<bool>& ok = allowed[device & 7][nc];
-  if (device > 7 || !ok) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlatSmemCap);
-    if (e != cudaSuccess) return e;
-    ok = true;
-  }
+  static SmemOptIn opt_in[kFlatCw + 1];
+  const cudaError_t e = opt_in[nc]((const void*)kern, kFlatSmemCap);
+  if (e != cudaSuccess) return e;
   // one block an SM; with little work as many as have a group or a leaf piece per warp
   const int64_t pieces = nleaves * a.nchunk * a.npiece;
   const unsigned grid = (unsigned)std::min<int64_t>(

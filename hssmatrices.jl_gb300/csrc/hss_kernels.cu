@@ -20,6 +20,7 @@
 #include "hss_device.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 
 namespace hss {
 
@@ -946,20 +947,14 @@ size_t mv_down_staged_smem(int ku, int u1, int u2, int v1, int v2) {
                            (size_t)(v1 + v2 + ku) * MV_RC_BLOCK);
 }
 void launch_mv_up_staged(const Task* t, int64_t nt, const Slot* s, size_t smem, int rmax, cudaStream_t st) {
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(mv_up_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)mv_up_staged_kernel, 200 * 1024);
   const int nchunk = (rmax + MV_RC_BLOCK - 1) / MV_RC_BLOCK;
   if (nt > 0 && nchunk > 0) mv_up_staged_kernel<<<(unsigned)(nt * nchunk), NT, smem, st>>>(t, s, MV_RC_BLOCK, nchunk);
 }
 void launch_mv_down_staged(const Task* t, int64_t nt, const Slot* s, size_t smem, int rmax, cudaStream_t st) {
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(mv_down_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)mv_down_staged_kernel, 200 * 1024);
   const int nchunk = (rmax + MV_RC_BLOCK - 1) / MV_RC_BLOCK;
   if (nt > 0 && nchunk > 0) mv_down_staged_kernel<<<(unsigned)(nt * nchunk), NT, smem, st>>>(t, s, MV_RC_BLOCK, nchunk);
 }

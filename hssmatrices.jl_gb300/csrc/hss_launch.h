@@ -96,8 +96,8 @@ bool pmv_flat_fits(const FlatTables& f, int64_t gen, int nleaf, int kmax, int rm
 double pmv_flat_estimate(const FlatTables& f, int64_t nleaves, int64_t gen, int rmax, int sms);
 void pmv_flat_space(const FlatTables& f, int64_t nleaves, int kmax, int rmax, int sms, int64_t* ctb, int64_t* counters);
 cudaError_t launch_pmv_flat(const FlatTables& f, const Task* leaves, int64_t nleaves, const Slot* slots, int rmax,
-                            int nleaf, int mleaf, int kmax, uint32_t* state, double* ctb, uint32_t* dcnt, int device,
-                            int sms, uint32_t idle_limit, cudaStream_t st);
+                            int nleaf, int mleaf, int kmax, uint32_t* state, double* ctb, uint32_t* dcnt, int sms,
+                            uint32_t idle_limit, cudaStream_t st);
 
 // Entry extraction (hss_getindex.cu): basis pass for one list of nodes (one
 // tree height), the off-diagonal tiles, the diagonal leaf blocks.  R / C are

@@ -44,6 +44,7 @@
 
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 #include "hss_oz.cuh"
 
 namespace hss {
@@ -607,12 +608,9 @@ __global__ void __launch_bounds__(OT, 1) ozmv_kernel(const Task* __restrict__ ta
 
 template <int NC>
 cudaError_t launch_nc(int kind, const Task* t, int64_t nt, const Slot* s, int rmax, int rows, int sms, cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(ozmv_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<NC>::smem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SmemOptIn opt_in;
+  const cudaError_t e = opt_in((const void*)ozmv_kernel<NC>, Ring<NC>::smem);
+  if (e != cudaSuccess) return e;
   const int nchunk = (rmax + NC - 1) / NC, ntile = std::max(1, (rows + TR - 1) / TR);
   const int64_t units = nt * nchunk * ntile;
   const uint32_t polls = pmv_poll_limit();
@@ -642,12 +640,9 @@ int64_t ozmv_image_bytes(const Node& nd, bool up) {
 cudaError_t launch_ozmv_prep(int kind, const Task* t, int64_t nt, int rows, int inner, unsigned char* base,
                              cudaStream_t st) {
   if (nt <= 0 || rows <= 0 || inner <= 0) return cudaSuccess;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(ozmv_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrepSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static SmemOptIn opt_in;
+  const cudaError_t e = opt_in((const void*)ozmv_prep_kernel, kPrepSmem);
+  if (e != cudaSuccess) return e;
   const int ntile = (rows + TR - 1) / TR, nchunk = (inner + KC - 1) / KC;
   if (nt * ntile * nchunk > INT32_MAX) return cudaErrorInvalidValue;
   ozmv_prep_kernel<<<(unsigned)(nt * ntile * nchunk), PT, kPrepSmem, st>>>(t, kind, ntile, nchunk, base);

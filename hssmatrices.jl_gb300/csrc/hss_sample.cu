@@ -30,6 +30,7 @@
 
 #include "hss_df.cuh"
 #include "hss_device.cuh"
+#include "hss_optin.h"
 #include "hss_sample.h"
 
 namespace hss {
@@ -251,11 +252,8 @@ template <int NC>
 void launch_dfrows(dim3 grid, cudaStream_t st, const GemmProblem& p, int trans, double alpha, double beta,
                    int64_t kchunk, double* P, const int32_t* lrow, const int32_t* lin) {
   constexpr size_t smem = dfrows_smem<NC>();
-  static bool attr = false;   // set once per instantiation (the size is a compile-time constant)
-  if (!attr) {
-    cudaFuncSetAttribute(dfsample_rows_kernel<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)dfsample_rows_kernel<NC>, smem);
   dfsample_rows_kernel<NC><<<grid, GT, smem, st>>>(p, trans, alpha, beta, kchunk, P, lrow, lin);
 }
 

@@ -35,6 +35,7 @@
 #include <cstdint>
 
 #include "hss_oz.cuh"
+#include "hss_optin.h"
 #include "hss_sample.h"
 
 namespace hss {
@@ -341,20 +342,13 @@ template <int NC>
 cudaError_t launch_tc(TcProblem p, int trans, const SampleTcPlan& pl, unsigned char* xs, cudaStream_t st) {
   const int64_t nchunk = (p.k + KC - 1) / KC;
   const unsigned tiles = (unsigned)((p.r + NC - 1) / NC);
-  static bool attr_set = false;
-  if (!attr_set) {
-    for (auto f : {sample_tc_kernel<NC, false>, sample_tc_kernel<NC, true>}) {
-      cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, Sizes<NC>::smem);
-      if (e != cudaSuccess) return e;
-    }
-    attr_set = true;
-  }
+  static SmemOptIn opt_in[2];
+  auto* kernel = trans ? sample_tc_kernel<NC, true> : sample_tc_kernel<NC, false>;
+  const cudaError_t e = opt_in[trans ? 1 : 0]((const void*)kernel, Sizes<NC>::smem);
+  if (e != cudaSuccess) return e;
   if (nchunk > 0) oz_prep_kernel<NC><<<dim3((unsigned)nchunk, tiles), NC * 16, 0, st>>>(p.X, p.ldx, p.k, p.r, xs);
   const dim3 grid((unsigned)((p.m + SM_ - 1) / SM_), tiles, (unsigned)pl.nsplit);
-  if (trans)
-    sample_tc_kernel<NC, true><<<grid, ST, Sizes<NC>::smem, st>>>(p);
-  else
-    sample_tc_kernel<NC, false><<<grid, ST, Sizes<NC>::smem, st>>>(p);
+  kernel<<<grid, ST, Sizes<NC>::smem, st>>>(p);
   return cudaGetLastError();
 }
 

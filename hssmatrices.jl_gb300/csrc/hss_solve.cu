@@ -37,6 +37,7 @@
 #include "hss_factor.cuh"
 #include "hss_internal.h"
 #include "hss_launch.h"
+#include "hss_optin.h"
 
 namespace hss {
 
@@ -537,12 +538,8 @@ void up_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, 
   const size_t base = (size_t)(MR + 1) * (ST / TPC) * sizeof(T);
   size_t smem = base + want * sizeof(T);
   if (smem > kSolveSmemCap) smem = base;   // operands stay in global memory
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(ulv_solve_up_reg<T, TPC, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSolveSmemCap);
-    set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)ulv_solve_up_reg<T, TPC, MR>, kSolveSmemCap);
   const int nchunk = (rmax + ST / TPC - 1) / (ST / TPC);
   launch_st(ulv_solve_up_reg<T, TPC, MR>, nt * nchunk, smem, st, pdl, t, s, (int64_t)((smem - base) / sizeof(T)), nchunk);
 }
@@ -551,12 +548,8 @@ template <typename T, int TPC, int MR>
 void down_launch(const Task* t, int64_t nt, const Slot* s, size_t want, int rmax, cudaStream_t st, bool pdl) {
   size_t smem = want * sizeof(T);
   if (smem > kSolveSmemCap) smem = 0;
-  static bool set = false;
-  if (!set) {
-    cudaFuncSetAttribute(ulv_solve_down_reg<T, TPC, MR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kSolveSmemCap);
-    set = true;
-  }
+  static SmemOptIn opt_in;
+  opt_in((const void*)ulv_solve_down_reg<T, TPC, MR>, kSolveSmemCap);
   const int nchunk = (rmax + ST / TPC - 1) / (ST / TPC);
   launch_st(ulv_solve_down_reg<T, TPC, MR>, nt * nchunk, smem, st, pdl, t, s, (int)(smem / sizeof(T)), nchunk);
 }

@@ -28,3 +28,18 @@ def run(tmp_path, name, link):
 @pytest.mark.parametrize("name", ["levels_split", "levels_key"])
 def test_linked(lib, tmp_path, name):
     run(tmp_path, name, link=True)
+
+
+@pytest.mark.parametrize("name", ["smem_opt_in"])
+def test_alone(tmp_path, name):
+    run(tmp_path, name, link=False)
+
+
+def test_no_process_wide_opt_in():
+    """The attribute of more than 48 KB of shared memory is set per device: by the opt-in
+    objects, or on every call."""
+    for f in sorted(os.listdir(CSRC)):
+        lines = open(os.path.join(CSRC, f)).read().splitlines()
+        for i, line in enumerate(lines):
+            if "cudaFuncSetAttribute(" in line:
+                assert not any("static bool" in x for x in lines[max(0, i - 4):i]), f"{f}:{i + 1}"
