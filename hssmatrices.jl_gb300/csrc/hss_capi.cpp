@@ -11,6 +11,7 @@
 #include <cmath>
 #include <functional>
 #include <limits>
+#include <mutex>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -195,6 +196,9 @@ struct hss_plan_s {
   float2* d_gen_df = nullptr;           // generators as (hi, lo) float pairs, made on first use
   unsigned char* d_oz = nullptr;        // digit slices of the generators for the tensor-core product (first use)
   int64_t oz_bytes = 0;
+  std::mutex oz_mutex;                  // of the slices' state
+  cudaEvent_t oz_event = nullptr;       // their completion on the stream that made them
+  bool oz_complete = false;
   int32_t* d_sync = nullptr;            // per-node arrival counters of the persistent product
   int pmv_nleaf = 0, pmv_mleaf = 0, pmv_kmax = 0;   // largest leaf columns / rows, largest rank
   int64_t pmv_ninner = 0;                           // branches that are not roots
@@ -271,6 +275,7 @@ hss_plan_s::~hss_plan_s() {
   delete fused[1];
   if (d_gen_df) cudaFree(d_gen_df);
   if (d_oz) cudaFree(d_oz);
+  if (oz_event) cudaEventDestroy(oz_event);
   if (d_gen) cudaFree(d_gen);
   if (d_nodes) cudaFree(d_nodes);
   if (d_tasks) cudaFree(d_tasks);
@@ -966,11 +971,36 @@ int run_matvec_df(const Levels& L, const Slot* slots, int rmax, cudaStream_t st,
 }
 
 // The digit slices of the plan's generators for the tensor-core product, made
-// once per plan (the generators do not change); false when the buffer cannot be
-// allocated (other products run then).
+// once per plan (the generators do not change); false when they cannot be had now
+// (other products run then): no memory, or a stream that is being captured by the
+// caller.  Factorizations of one plan may be solved with on several streams and
+// threads: the first call makes the slices on its stream, and later calls wait for
+// them on theirs until they are known to be complete.
 bool ensure_oz(hss_plan_s* P, cudaStream_t st) {
-  if (P->d_oz) return true;
+  std::lock_guard<std::mutex> lock(P->oz_mutex);
+  if (P->oz_complete) return true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
+  if (P->d_oz) {
+    // (a query is refused to a thread that captures in the default mode)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t q = cudaEventQuery(P->oz_event);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (q == cudaSuccess) return P->oz_complete = true;
+    cudaGetLastError();   // not ready is not an error
+    return q == cudaErrorNotReady && cudaStreamIsCapturing(st, &cs) == cudaSuccess &&
+           cs == cudaStreamCaptureStatusNone && cudaStreamWaitEvent(st, P->oz_event, 0) == cudaSuccess;
+  }
   if (P->oz_bytes <= 0) return false;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  if (!P->oz_event && cudaEventCreateWithFlags(&P->oz_event, cudaEventDisableTiming) != cudaSuccess) {
+    P->oz_event = nullptr;
+    cudaGetLastError();
+    return false;
+  }
   if (dev_alloc((void**)&P->d_oz, (size_t)P->oz_bytes) != cudaSuccess) {
     P->d_oz = nullptr;
     cudaGetLastError();
@@ -990,6 +1020,7 @@ bool ensure_oz(hss_plan_s* P, cudaStream_t st) {
   prep(OZ_FINAL, P->leaves, P->pmv_mleaf, k);
   prep(OZ_UP_BRANCH, br, 3 * k, 2 * k);
   prep(OZ_DOWN, br, 2 * k, k);
+  if (e == cudaSuccess) e = cudaEventRecord(P->oz_event, st);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cudaFree(P->d_oz);
