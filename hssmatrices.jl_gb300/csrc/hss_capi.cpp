@@ -199,6 +199,7 @@ struct hss_plan_s {
   std::mutex oz_mutex;                  // of the slices' state
   cudaEvent_t oz_event = nullptr;       // their completion on the stream that made them
   bool oz_complete = false;
+  bool oz_asked = false;                // a product would have needed them
   int32_t* d_sync = nullptr;            // per-node arrival counters of the persistent product
   int pmv_nleaf = 0, pmv_mleaf = 0, pmv_kmax = 0;   // largest leaf columns / rows, largest rank
   int64_t pmv_ninner = 0;                           // branches that are not roots
@@ -970,6 +971,10 @@ int run_matvec_df(const Levels& L, const Slot* slots, int rmax, cudaStream_t st,
   return HSS_OK;
 }
 
+// Slices up to this size come from the device's pool (a new allocation takes 90 to 140
+// us of a first product of 200).
+constexpr int64_t kOzSmall = int64_t(16) << 20;
+
 // The digit slices of the plan's generators for the tensor-core product, made
 // once per plan (the generators do not change); false when they cannot be had now
 // (other products run then): no memory, or a stream that is being captured by the
@@ -1001,7 +1006,8 @@ bool ensure_oz(hss_plan_s* P, cudaStream_t st) {
     cudaGetLastError();
     return false;
   }
-  if (dev_alloc((void**)&P->d_oz, (size_t)P->oz_bytes) != cudaSuccess) {
+  if ((P->oz_bytes <= kOzSmall ? dev_alloc_async((void**)&P->d_oz, (size_t)P->oz_bytes, st)
+                               : dev_alloc((void**)&P->d_oz, (size_t)P->oz_bytes)) != cudaSuccess) {
     P->d_oz = nullptr;
     cudaGetLastError();
     return false;
@@ -1321,14 +1327,18 @@ int check_cols(hss_plan_s* P, const std::vector<Cols>& io, bool solve) {
   return HSS_OK;
 }
 
+// Time in us that making a plan's slices takes: an allocation, and 0.85 us a MB (n = 65536,
+// k = 32, 327 MB 383; n = 16384 180; 8192 155).
+double slices_us(const hss_plan_s* P) { return 110.0 + 0.85e-6 * (double)P->oz_bytes; }
+
 // Whether the tensor-core product takes a product of r columns.  It needs one
-// launch per tree level and, once per plan, the digit slices (100-400 us with their
-// allocation), and then hardly depends on r up to 32, where the FP64 products grow
+// launch per tree level and, once per plan, the digit slices (whether a plan's first
+// product makes them: oz_first_pays), and then hardly depends on r up to 32, where the FP64 products grow
 // with entries x columns at the FP64 pipe's rate: n = 65536, k = 32 (15.7 M entries)
 // 286 -> 200 us at r = 6, 948 -> 293 at 32, 1838 -> 422 at 64.  Where the flat product
 // applies, the line is its estimate against the tensor-core product's (launches,
 // slices, blocks; fitted as the flat product's) and an eighth of what making the
-// slices takes (545 us at 15.7 M entries, 140 at 2 M); both sides measured, flat /
+// slices takes (383 us at 15.7 M entries, 155 at 2 M); both sides measured, flat /
 // tensor cores in us: n = 32768 r = 4 110 / 143, r = 5 155 /
 // 143; n = 16384 r = 8 110 / 110, r = 10 155 / 114; n = 8192 r = 12 85 / 93, r = 16
 // 111 / 100; n = 10007, leaves of 39 rows, r = 16 108 / 136, r = 20 179 / 154; n = 4000,
@@ -1344,8 +1354,42 @@ bool oz_product_pays(const hss_plan_s* P, int64_t r) {
     return P->gen_len * r >= (P->pmv_kmax >= 16 ? 16000000 : 45000000);
   const double launches = 2.0 * (double)P->by_d.size() - 1.0, gen = (double)P->gen_len;
   const double oz = (6.3 * launches + 2.6e-6 * gen + 0.086 * (double)P->leaves.cnt) * (1.0 + (double)r / 128.0);
-  const double slices = 80.0 + 30e-6 * gen;
-  return pmv_flat_estimate(P->flat, P->leaves.cnt, P->gen_len, (int)r, sm_count(P->device)) > oz + slices / 8;
+  return pmv_flat_estimate(P->flat, P->leaves.cnt, P->gen_len, (int)r, sm_count(P->device)) > oz + slices_us(P) / 8;
+}
+
+// Whether the first product that would need a plan's slices makes them (us, wall time of
+// the call).  A program may make one product with a matrix, which then bears them
+// alone.  They are made at once where the product's gain pays for them
+// (n = 65536: r = 24 844 -> 722, r = 32 1065 -> 731, but r = 6 406 against 641 and
+// 16 635 against 668) or where they are small: up to 16 MB their cost is an
+// allocation from the pool.  The estimates: the queued product by its multiply-adds at
+// the FP64 rate, its tasks' hand-offs and its chain, which overlap (within 20 % of 96 to
+// 1853 us for n = 4096 to 65536, k = 8 to 32); the tensor-core product by launches,
+// slices, blocks and outputs (within 20 % of 71 to 437 us).
+bool oz_first_pays(const hss_plan_s* P, int64_t r) {
+  if (P->oz_bytes <= kOzSmall) return true;
+  const Levels L = plan_levels(P);
+  const double gen = (double)P->gen_len, nodes = (double)P->nodes.size(), lev = (double)P->by_d.size(), c = (double)r;
+  const double oz = 15.0 + 6.3 * (2.0 * lev - 1.0) + 2.6e-6 * gen + 0.086 * (double)P->leaves.cnt + 3e-3 * nodes * c;
+  const double work = 1.9e-6 * gen * c, tasks = 9.5e-3 * nodes * c, chain = (lev - 1.0) * (10.0 + 0.4 * P->pmv_kmax);
+  const double other = use_flat(L, false, (int)std::min<int64_t>(r, INT32_MAX))
+                           ? 15.0 + pmv_flat_estimate(P->flat, P->leaves.cnt, P->gen_len, (int)r, sm_count(P->device))
+                           : std::sqrt(work * work + tasks * tasks + chain * chain);
+  return other > oz + slices_us(P);
+}
+
+// Whether this product of r columns runs on the tensor cores (its slices are there
+// then).  From the second product that would need them on, the line is the one for
+// repeated products.
+bool take_oz(hss_plan_s* P, int64_t r, cudaStream_t st) {
+  if (!oz_product_pays(P, r)) return false;
+  {
+    std::lock_guard<std::mutex> lock(P->oz_mutex);
+    const bool first = !P->oz_asked && !P->d_oz;
+    P->oz_asked = true;
+    if (first && !oz_first_pays(P, r)) return false;
+  }
+  return ensure_oz(P, st);
 }
 
 int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double beta,
@@ -1355,7 +1399,7 @@ int matmul_impl(hss_plan_s* P, const std::vector<Cols>& io, double alpha, double
   for (auto& c : io) rmax = std::max(rmax, c.r);
   if (rmax == 0) return HSS_OK;
   CUDA_TRY(P->mv_ws.ensure((size_t)P->ws_mv * rmax));
-  const bool oz = oz_product_pays(P, rmax) && ensure_oz(P, st);
+  const bool oz = take_oz(P, rmax, st);
   std::vector<Slot> s(P->ntrees);
   for (int32_t t = 0; t < P->ntrees; ++t) {
     Slot& x = s[t];
