@@ -459,6 +459,7 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
       // Block shapes follow from the ranks, so a rank that disagrees with the
       // stored blocks shows up as overlapping blocks: require them disjoint.
       std::vector<std::pair<int64_t, int64_t>> blocks;
+      blocks.reserve(6 * nn);
       for (int64_t i = 0; i < nn; ++i) {
         const Node& x = N[i];
         const GenOffsets& o = O[i];
@@ -480,7 +481,7 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
           add(o.W2, (int64_t)c2.kv * x.kv);
         }
       }
-      std::sort(blocks.begin(), blocks.end());
+      if (!std::is_sorted(blocks.begin(), blocks.end())) std::sort(blocks.begin(), blocks.end());
       for (size_t b = 1; b < blocks.size(); ++b)
         if (blocks[b - 1].first + blocks[b - 1].second > blocks[b].first)
           return fail(HSS_ERR_BAD_DIMS, "generator blocks overlap: ranks disagree with the stored blocks");
@@ -578,9 +579,11 @@ int layout_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, std::vector<Gen
 // so caches keyed on plans use these instead of pointers.
 std::atomic<uint64_t> g_plan_serial{0};
 
+int sm_count(int device);
+
 // Tables of the flat product.  It applies when each subtree's leaves are contiguous
 // in the leaf list (pre-order node numbering gives that) and the trees are not
-// deeper than kFlatDep - 1.
+// deeper than kFlatDep - 1.  Groups are numbered in the sizes that a product can take.
 int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
   const std::vector<Node>& N = P->nodes;
   const int64_t nn = (int64_t)N.size(), nl = P->leaves.cnt;
@@ -613,8 +616,18 @@ int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
       ng[level] += is_root((int32_t)i, 1 << level);
       nbr[level] += up[i] >= 0 && cnt[i] > 1 << level;
     }
-  size_t bytes = (size_t)nn * sizeof(FlatLink), at[kFlatLevels][2];
+  FlatTables f;
+  f.dep = dep;
   for (int level = 0; level < kFlatLevels; ++level) {
+    f.lev[level].ngroup = ng[level];
+    f.lev[level].nbranch = nbr[level];
+  }
+  for (int64_t t = 0; t < nl; ++t) f.leaf_elems += (int64_t)N[leaf_node(t)].gm * N[leaf_node(t)].gn;
+  const uint32_t taken = pmv_flat_levels(f, P->gen_len, P->pmv_nleaf, P->pmv_kmax, sm_count(P->device));
+  if (taken == 0) return HSS_OK;
+  size_t bytes = (size_t)nn * sizeof(FlatLink), at[kFlatLevels][2] = {};
+  for (int level = 0; level < kFlatLevels; ++level) {
+    if (!(taken >> level & 1)) continue;
     at[level][0] = bytes;
     bytes += (size_t)ng[level] * sizeof(FlatGroup);
     at[level][1] = bytes;
@@ -644,6 +657,7 @@ int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
   }
   std::vector<int32_t> gof(nl + 1);   // groups that start before leaf t
   for (int level = 0; level < kFlatLevels; ++level) {
+    if (!(taken >> level & 1)) continue;
     const int gmax = 1 << level;
     FlatGroup* groups = (FlatGroup*)(img.data() + at[level][0]);
     FlatBranch* branches = (FlatBranch*)(img.data() + at[level][1]);
@@ -694,14 +708,14 @@ int build_flat_tables(hss_plan_s* P, const std::vector<Task>& tasks) {
   CUDA_TRY(dev_alloc((void**)&P->d_flat, img.size()));
   CUDA_TRY(cudaMemcpy(P->d_flat, img.data(), img.size(), cudaMemcpyHostToDevice));
   P->flat_bytes = (int64_t)img.size();
-  FlatTables& f = P->flat;
-  for (int level = 0; level < kFlatLevels; ++level)
-    f.lev[level] = FlatLevel{(const FlatGroup*)(P->d_flat + at[level][0]), (const FlatBranch*)(P->d_flat + at[level][1]),
-                             ng[level], nbr[level]};
+  for (int level = 0; level < kFlatLevels; ++level) {
+    if (!(taken >> level & 1)) continue;
+    f.lev[level].groups = (const FlatGroup*)(P->d_flat + at[level][0]);
+    f.lev[level].branches = (const FlatBranch*)(P->d_flat + at[level][1]);
+  }
   f.nodes = P->d_nodes;
-  for (int64_t t = 0; t < nl; ++t) f.leaf_elems += (int64_t)N[leaf_node(t)].gm * N[leaf_node(t)].gn;
   f.links = (const FlatLink*)P->d_flat;
-  f.dep = dep;
+  P->flat = f;
   return HSS_OK;
 }
 
@@ -821,8 +835,6 @@ bool use_pmv(const Levels& L, const SlotTable* pm, bool pairs, int rmax) {
   return pm != nullptr && !g_level_product && L.leaves.cnt > 0 && pmv_fits(L.nleaf, L.mleaf, L.kmax) &&
          pmv_chunks(pairs, rmax) > 0 && pmv_queue_fits(L.nodes_max, L.nslots);
 }
-
-int sm_count(int device);
 
 // The flat product takes FP64 products of few columns on plans that have its tables.
 bool use_flat(const Levels& L, bool pairs, int rmax) {

@@ -749,6 +749,13 @@ bool pmv_flat_fits(const FlatTables& f, int64_t gen, int nleaf, int kmax, int rm
   return gen * rmax <= 45000000 && (kmax >= 16 || (int64_t)f.lev[s.level].ngroup * s.nchunk <= sms);
 }
 
+uint32_t pmv_flat_levels(const FlatTables& f, int64_t gen, int nleaf, int kmax, int sms) {
+  uint32_t levels = 0;
+  for (int r = 1; r <= kFlatCols; ++r)
+    if (pmv_flat_fits(f, gen, nleaf, kmax, r, sms)) levels |= 1u << flat_shape(f, r, sms).level;
+  return levels;
+}
+
 // Estimated time in us: the chain's latency per pass over the groups, and 0.34 ns per
 // multiply-add of an SM, its groups' tree part and its share of the leaf products
 // (fitted to trees of 8 to 1024 leaves of 15 to 250 rows at 1 to 32 columns, within
@@ -772,6 +779,7 @@ cudaError_t launch_pmv_flat(const FlatTables& f, const Task* leaves, int64_t nle
   if (nleaves <= 0) return cudaSuccess;
   const FlatShape shape = flat_shape(f, rmax, sms);
   const FlatLevel& lv = f.lev[shape.level];
+  if (lv.ngroup > 0 && lv.groups == nullptr) return cudaErrorInvalidValue;
   FlatArgs a;
   a.leaves = leaves;
   a.nodes = f.nodes;

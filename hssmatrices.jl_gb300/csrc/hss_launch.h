@@ -81,7 +81,7 @@ constexpr int kFlatCols = 32;   // most columns
 constexpr int kFlatLevels = 4;  // groups of at most 1 << level leaves
 static_assert(kFlatGroup == 1 << (kFlatLevels - 1), "the largest groups");
 struct FlatLevel {
-  const FlatGroup* groups = nullptr;
+  const FlatGroup* groups = nullptr;   // null: no product takes groups of this size
   const FlatBranch* branches = nullptr;
   int32_t ngroup = 0, nbranch = 0;
 };
@@ -93,6 +93,8 @@ struct FlatTables {
   int64_t leaf_elems = 0;   // entries of the leaves' D
 };
 bool pmv_flat_fits(const FlatTables& f, int64_t gen, int nleaf, int kmax, int rmax, int sms);
+// The group sizes (levels, as bits) that products of 1 to kFlatCols columns take.
+uint32_t pmv_flat_levels(const FlatTables& f, int64_t gen, int nleaf, int kmax, int sms);
 double pmv_flat_estimate(const FlatTables& f, int64_t nleaves, int64_t gen, int rmax, int sms);
 void pmv_flat_space(const FlatTables& f, int64_t nleaves, int kmax, int rmax, int sms, int64_t* ctb, int64_t* counters);
 cudaError_t launch_pmv_flat(const FlatTables& f, const Task* leaves, int64_t nleaves, const Slot* slots, int rmax,

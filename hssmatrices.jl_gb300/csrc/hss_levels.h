@@ -73,15 +73,16 @@ void seg_split(Seg& v, std::vector<Task>& tasks, F&& nodes) {
     const Node* nodes;
   };
   v.parts.clear();
-  bool one = true;
+  auto cls = [&](int64_t i) { return size_class(nodes(i)[tasks[v.off + i].node]); };
+  int64_t same = 1;
+  while (same < v.cnt && cls(same) == cls(0)) ++same;
+  if (same >= v.cnt) return;
   std::vector<Item> items((size_t)v.cnt);
   for (int64_t i = 0; i < v.cnt; ++i) {
-    const Task& t = tasks[v.off + i];
     const Node* nd = nodes(i);
+    const Task& t = tasks[v.off + i];
     items[i] = Item{size_class(nd[t.node]), t, nd};
-    one = one && items[i].cls == items[0].cls;
   }
-  if (one) return;
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cls < b.cls; });
   for (int64_t i = 0; i < v.cnt; ++i) {
     if (i == 0 || items[i].cls != items[i - 1].cls) {
