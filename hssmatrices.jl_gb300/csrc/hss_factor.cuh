@@ -8,6 +8,7 @@
 
 #include "hss_device.cuh"
 #include "hss_internal.h"
+#include "hss_recip.cuh"
 
 namespace hss {
 namespace fac {
@@ -19,84 +20,12 @@ constexpr int PL = 8;               // lanes per panel column (QL) or row (LQ)
 constexpr int GP = BP + 1;          // ld of the Gram matrix and of T
 static_assert(NT == 8 * BP, "the panel mapping puts 8 lanes on each of 32 columns (rows)");
 
-__device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
-
 template <typename T>
 __device__ __forceinline__ T gsum8(T v, unsigned gm) {   // sum over the 8 lanes of a group
   v += __shfl_xor_sync(gm, v, 4);
   v += __shfl_xor_sync(gm, v, 2);
   v += __shfl_xor_sync(gm, v, 1);
   return v;
-}
-
-// xLARFG from alpha and the squared tail norm: the norm as sqrt(alpha^2 + ss)
-// (hypot only near overflow or underflow); FP32 with correctly rounded
-// reciprocals, FP64 with the Newton steps above.
-__device__ __forceinline__ void larfg_t(float alpha, float ss, float& beta, float& tau, float& scal) {
-  if (ss == 0.f) {
-    tau = 0.f;
-    beta = alpha;
-    scal = 1.f;
-    return;
-  }
-  const float t = fmaf(alpha, alpha, ss);
-  const float nrm = t <= 3.0e38f ? sqrtf(t) : hypotf(alpha, sqrtf(ss));
-  beta = -copysignf(nrm, alpha);
-  tau = (beta - alpha) * __frcp_rn(beta);
-  scal = __frcp_rn(alpha - beta);
-}
-// 1 / sqrt(t) and 1 / d for normal t, d > 0 from FP32 seeds (relative error e below
-// 2^-21) by one step of third order each: GB300 issues an FP64 warp instruction
-// every 64 clocks per SM sub-partition, and a square root and two divisions are
-// about forty of them on the critical path of every reflector (here 5 and 3).
-__device__ __forceinline__ double widen(float x) {   // exact, without an FP64 instruction (x normal)
-  const uint32_t b = __float_as_uint(x);
-  return __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
-}
-__device__ __forceinline__ double rsqrt_newton(double t) {
-  // t = f 4^q with f in [1/2, 2): the seed from f, the power of two put back
-  const long long b = __double_as_longlong(t);
-  const int q = (int)((b >> 52) - 1022) >> 1;
-  const long long fb = b - ((long long)q << 53);
-  // f's leading bits as an FP32 number
-  const float ff = __uint_as_float((uint32_t)(((fb >> 52) - 1023 + 127) << 23) | (uint32_t)((fb >> 29) & 0x7FFFFF));
-  const double f = __longlong_as_double(fb), y = widen(rsqrtf(ff));
-  const double e = fma(-f * y, y, 1.0);                      // 1 - f y^2
-  const double r = fma(y, e * fma(0.375, e, 0.5), y);
-  return __longlong_as_double(__double_as_longlong(r) - ((long long)q << 52));
-}
-__device__ __forceinline__ double rcp_newton(double d) {
-  const long long b = __double_as_longlong(d);
-  const int q = (int)(b >> 52) - 1023;   // d = f 2^q, f in [1, 2)
-  const double f = __longlong_as_double(b - ((long long)q << 52));
-  const double r = widen(__frcp_rn(__uint_as_float(0x3F800000u | (uint32_t)((b >> 29) & 0x7FFFFF))));
-  const double e = fma(-f, r, 1.0);
-  return __longlong_as_double(__double_as_longlong(fma(r, fma(e, e, e), r)) - ((long long)q << 52));
-}
-
-__device__ __forceinline__ void larfg_t(double alpha, double ss, double& beta, double& tau, double& scal) {
-  // tests on the bits: FP64 comparisons take the FP64 pipe too
-  if ((__double_as_longlong(ss) << 1) == 0) {
-    tau = 0.0;
-    beta = alpha;
-    scal = 1.0;
-    return;
-  }
-  const double t = fma(alpha, alpha, ss);
-  const int et = (int)(__double_as_longlong(t) >> 52);   // biased exponent (t >= 0)
-  if (et > 100 && et < 1946) {
-    const double y = rsqrt_newton(t), a = fabs(alpha);
-    const double nrm = t * y;
-    beta = -copysign(nrm, alpha);
-    tau = fma(a, y, 1.0);                            // (beta - alpha) / beta
-    scal = copysign(rcp_newton(a + nrm), alpha);     // 1 / (alpha - beta)
-    return;
-  }
-  const double nrm = hypot(alpha, sqrt(ss));
-  beta = -copysign(nrm, alpha);
-  tau = (beta - alpha) / beta;
-  scal = 1.0 / (alpha - beta);
 }
 
 // four consecutive elements, 16-byte aligned (FP32) or 32-byte aligned (FP64)
@@ -140,14 +69,6 @@ __device__ __forceinline__ bool larger_mag(float a, float b) {
 __device__ __forceinline__ bool larger_mag(double a, double b) {
   return ((unsigned long long)__double_as_longlong(a) << 1) > ((unsigned long long)__double_as_longlong(b) << 1);
 }
-__device__ __forceinline__ float recip(float d) { return 1.f / d; }
-__device__ __forceinline__ double recip(double d) {
-  const int e = (int)(__double_as_longlong(d) >> 52) & 0x7FF;
-  if (e < 64 || e > 1982) return 1.0 / d;
-  const double r = rcp_newton(__longlong_as_double(__double_as_longlong(d) & 0x7FFFFFFFFFFFFFFFll));
-  return copysign(r, d);
-}
-
 // LU with partial pivoting of an m x m block (ld), columns dealt to the warps in
 // turn.  One barrier per column: while the other warps apply column c, the owner
 // of column c + 1 applies it there first, finds the next pivot (first entry of
@@ -177,10 +98,10 @@ __device__ void lu_blk(T* A, int m, int ld, int32_t* piv, int32_t* err, T* lv, i
       col[idx] = t;
     }
     __syncwarp();
-    const T r = zero ? T(1) : recip(col[c]);
+    const Multiplier<T> mult(zero ? T(1) : col[c]);
     T* l = lv + (c & 1) * m;
     for (int i = c + 1 + lane; i < m; i += 32) {
-      const T x = col[i] * r;
+      const T x = mult(col[i]);
       col[i] = x;
       l[i] = x;
     }

@@ -10,7 +10,9 @@
 // A level is bound by one block's chain, a list of many blocks by the FP64 pipe:
 // * a division is about forty FP64 instructions of 64 clocks on the chain of every
 //   row of a substitution; the diagonal's reciprocals are formed once per block
-//   instead, and a quotient is a product and one correction;
+//   instead, and a quotient is a product and one correction (a finished column is
+//   looked over for entries that this fails, and done again by divisions then; a test
+//   per row cost 1.2 % of a resident solve and 2.3 % of a mixed batch, this 0.3 %);
 // * 8 lanes per right-hand side (four per warp) spend 20 FP64 instructions on a
 //   reflector of 64 rows for four right-hand sides, 32 lanes 10 for one: FP64
 //   lists longer than two rounds of the SMs take 8 lanes, shorter ones 32;
@@ -74,16 +76,6 @@ __device__ __forceinline__ void stage_block(T* dst, int ldd, const T* src, int64
     for (int i = lane + (tril ? c & ~31 : 0); i < rows; i += 32) cpa(dst + i + c * ldd, src + i + (int64_t)c * lds);
 }
 
-// b / d from r = 1 / d: the product and one correction.
-__device__ __forceinline__ float quot(float b, float d, float r) {
-  const float x = b * r;
-  return fmaf(r, fmaf(-d, x, b), x);
-}
-__device__ __forceinline__ double quot(double b, double d, double r) {
-  const double x = b * r;
-  return fma(r, fma(-d, x, b), x);
-}
-
 template <int TPC, typename T>
 __device__ __forceinline__ T gsum(T v) {
 #pragma unroll
@@ -102,7 +94,7 @@ __device__ __forceinline__ void lower_solve(T (&b)[RPT], const T* __restrict__ L
       const int c = s * TPC + o;
       if (c >= nr) break;
       const T bc = __shfl_sync(0xffffffffu, b[s], o, TPC);
-      const T xc = UNIT ? bc : quot(bc, L[c + (int64_t)c * ldl], rd[c]);
+      const T xc = UNIT ? bc : fac::quot(bc, L[c + (int64_t)c * ldl], rd[c]);
       if (gl == o) b[s] = xc;
 #pragma unroll
       for (int s2 = s; s2 < RPT; ++s2) {
@@ -123,7 +115,7 @@ __device__ __forceinline__ void upper_solve(T (&b)[RPT], const T* __restrict__ A
       const int c = s * TPC + o;
       if (c >= nr) continue;
       const T bc = __shfl_sync(0xffffffffu, b[s], o, TPC);
-      const T xc = quot(bc, A[c + (int64_t)c * lda], rd[c]);
+      const T xc = fac::quot(bc, A[c + (int64_t)c * lda], rd[c]);
       if (gl == o) b[s] = xc;
 #pragma unroll
       for (int s2 = 0; s2 <= s; ++s2) {
@@ -131,6 +123,54 @@ __device__ __forceinline__ void upper_solve(T (&b)[RPT], const T* __restrict__ A
         if (row < c) b[s2] -= A[row + (int64_t)c * lda] * xc;
       }
     }
+  }
+}
+
+// Whether a solution in registers holds an entry that quot failed (L: the block whose
+// diagonal it was divided by).
+template <typename T, int TPC, int RPT>
+__device__ __forceinline__ bool failed(const T (&b)[RPT], const T* __restrict__ L, int ld, int nr, int gl) {
+  bool bad = false;
+#pragma unroll
+  for (int s = 0; s < RPT; ++s) {
+    const int row = gl + s * TPC;
+    if (row < nr) bad = bad || fac::quot_failed(b[s], L[row + (int64_t)row * ld]);
+  }
+  return bad;
+}
+
+// The same steps by divisions, on a column in shared memory, for right-hand sides that
+// the reciprocals failed (entries that are infinite, NaN or out of range): every warp
+// that calls takes all its columns through them.
+template <typename T, int TPC>
+__device__ __noinline__ void reflect_slow(T* col, const T* U, int ldU, const T* tq, int m, int k, int mk, int gl) {
+  for (int c = k - 1; c >= 0; --c) {
+    const int p = mk + c;
+    T d = T(0);
+    for (int row = gl; row <= p; row += TPC) d += (row == p ? T(1) : U[row + (int64_t)c * ldU]) * col[row];
+    d = gsum<TPC>(d) * tq[c];
+    for (int row = gl; row <= p; row += TPC) col[row] -= d * (row == p ? T(1) : U[row + (int64_t)c * ldU]);
+    __syncwarp();
+  }
+}
+template <typename T, int TPC>
+__device__ __noinline__ void lower_slow(T* col, const T* L, int ldl, int nr, int gl, bool unit) {
+  for (int c = 0; c < nr; ++c) {
+    const T x = unit ? col[c] : col[c] / L[c + (int64_t)c * ldl];
+    __syncwarp();
+    if (gl == 0) col[c] = x;
+    for (int row = c + 1 + gl; row < nr; row += TPC) col[row] -= L[row + (int64_t)c * ldl] * x;
+    __syncwarp();
+  }
+}
+template <typename T, int TPC>
+__device__ __noinline__ void upper_slow(T* col, const T* A, int lda, int nr, int gl) {
+  for (int c = nr - 1; c >= 0; --c) {
+    const T x = col[c] / A[c + (int64_t)c * lda];
+    __syncwarp();
+    if (gl == 0) col[c] = x;
+    for (int row = gl; row < c; row += TPC) col[row] -= A[row + (int64_t)c * lda] * x;
+    __syncwarp();
   }
 }
 
@@ -149,7 +189,7 @@ __host__ __device__ inline int64_t solve_up_stage_elems(int m, int k, int mk, in
 }
 
 template <typename T, int TPC, int MR>
-__global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ tasks,
+__global__ void __launch_bounds__(ST, sizeof(T) == 4 && MR > 64 ? 4 : MR / TPC > 8 ? 2 : 3) ulv_solve_up_reg(const Task* __restrict__ tasks,
                                                        const Slot* __restrict__ slots, int64_t stage_cap,
                                                        int nchunk) {
   constexpr int RPT = MR / TPC;
@@ -341,6 +381,16 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
       }
       lower_solve<T, TPC, RPT, true>(b, A, ldL, m, gl, s_rd);
       upper_solve<T, TPC, RPT>(b, A, ldL, m, gl, s_rd);
+      if (__any_sync(0xffffffffu, j < r && failed<T, TPC>(b, A, ldL, m, gl))) {
+        T* col = sb + g * LDS;
+        lower_slow<T, TPC>(col, A, ldL, m, gl, true);
+        upper_slow<T, TPC>(col, A, ldL, m, gl);
+#pragma unroll
+        for (int s = 0; s < RPT; ++s) {
+          const int row = gl + s * TPC;
+          b[s] = row < m ? col[row] : T(0);
+        }
+      }
       if (j < r) {
         T* x = ws + nd.wx + (int64_t)j * ld;
 #pragma unroll
@@ -383,10 +433,15 @@ __global__ void __launch_bounds__(ST) ulv_solve_up_reg(const Task* __restrict__ 
       }
       // zloc = L1 \ b[0:mk] (trsm, src/ulvfactor.jl:48)
       lower_solve<T, TPC, RPT, false>(b, Lp, ldL, mk, gl, s_rd);
+      if (__any_sync(0xffffffffu, j < r && failed<T, TPC>(b, Lp, ldL, mk, gl))) {
+        reflect_slow<T, TPC>(sb + g * LDS, Up, ldU, tq, m, k, mk, gl);
+        lower_slow<T, TPC>(sb + g * LDS, Lp, ldL, mk, gl, false);
+      } else {
 #pragma unroll
-      for (int s = 0; s < RPT; ++s) {
-        const int row = gl + s * TPC;
-        if (row < m) sb[row + g * LDS] = b[s];
+        for (int s = 0; s < RPT; ++s) {
+          const int row = gl + s * TPC;
+          if (row < m) sb[row + g * LDS] = b[s];
+        }
       }
     }
     __syncthreads();

@@ -30,7 +30,7 @@ def test_linked(lib, tmp_path, name):
     run(tmp_path, name, link=True)
 
 
-@pytest.mark.parametrize("name", ["smem_opt_in"])
+@pytest.mark.parametrize("name", ["smem_opt_in", "recip"])
 def test_alone(tmp_path, name):
     run(tmp_path, name, link=False)
 
