@@ -8,11 +8,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "hss_host.h"
+#include "hss_internal.h"
 #include "hss_launch.h"
 #include "hss_sample.h"
 
@@ -36,6 +39,40 @@ int sm_count(int device) {
   return n;
 }
 
+// A word per device, in host memory that its kernels can write: a tensor-core sample
+// product whose wait ran out leaves DEV_TIMEOUT there.  The product is asynchronous and
+// has no handle, so that the next hss_sample or hss_sumsq on the device reports it.
+std::atomic<int32_t*> g_sample_status[64];
+
+int32_t* sample_status(int device) {
+  if (device < 0 || device >= 64) return nullptr;
+  std::atomic<int32_t*>& w = g_sample_status[device];
+  if (int32_t* p = w.load()) return p;
+  static std::mutex mutex;
+  std::lock_guard<std::mutex> lock(mutex);
+  int32_t* p = w.load();
+  if (p) return p;
+  // (the caller may be capturing: the allocation is no part of it)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaHostAlloc((void**)&p, sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;   // the NaN outputs remain
+  }
+  *(volatile int32_t*)p = DEV_OK;
+  w.store(p);
+  return p;
+}
+
+int sample_expired(int device) {
+  int32_t* p = device >= 0 && device < 64 ? g_sample_status[device].load() : nullptr;
+  if (!p || *(volatile int32_t*)p == DEV_OK) return HSS_OK;
+  *(volatile int32_t*)p = DEV_OK;
+  return set_error(HSS_ERR_TIMEOUT, "sample product: a wait ran out in an earlier call; its rows are NaN");
+}
+
 // The product on the tensor cores, with stream-ordered scratch, so that calls
 // on different streams do not share it.
 int sample_tc(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_t trans, const double* dX, int64_t ldx,
@@ -43,7 +80,8 @@ int sample_tc(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_
   const SampleTcPlan pl = sample_tc_plan(rows, inner, r, sm_count(device));
   unsigned char* scratch = nullptr;
   RC_TRY(cudaMallocAsync((void**)&scratch, pl.scratch_bytes, st));
-  cudaError_t e = launch_sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, pl, scratch, st);
+  cudaError_t e = launch_sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, pl, scratch,
+                                   pmv_poll_limit(), sample_status(device), st);
   count_launches(pl.nsplit > 1 ? 3 : 2);
   const cudaError_t f = cudaFreeAsync(scratch, st);
   if (e == cudaSuccess) e = f;
@@ -298,6 +336,7 @@ int hss_sample(const double* dA, int64_t lda, int64_t m, int64_t n, int32_t tran
   cudaStream_t st = (cudaStream_t)stream;
   int dev = 0;
   RC_TRY(cudaGetDevice(&dev));
+  if (int rc = sample_expired(dev)) return rc;
   if (sample_tc_pays(inner)) return sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, dev, st);
   return sample_cores(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, dev, st);
 }
@@ -365,7 +404,9 @@ int hss_sumsq(const double* dB, int64_t ldb, int64_t m, int64_t r, double* out, 
   double acc = 0.0;
   for (double v : h) acc += v;
   *out = acc;
-  return HSS_OK;
+  int dev = 0;
+  RC_TRY(cudaGetDevice(&dev));
+  return sample_expired(dev);
 }
 
 int hss_rc_compress(hss_rc R, const double* dA, int64_t lda, const double* dScol, int64_t ldscol,

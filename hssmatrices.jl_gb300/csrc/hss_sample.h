@@ -80,10 +80,13 @@ struct SampleTcPlan {
 // differs from the reference algorithm's ranks with the former rounding, three
 // with samples that are exact to the last bit).
 inline bool sample_tc_pays(int64_t k) { return k > 2048; }
+// limit: polls of a wait before it gives up; the rows of its block are NaN then, and
+// *status (host memory that the device can write, or null) is DEV_TIMEOUT.
 SampleTcPlan sample_tc_plan(int64_t m, int64_t k, int64_t r, int sms);
 cudaError_t launch_sample_tc(const double* A, int64_t lda, int64_t m, int64_t k, int trans, const double* X,
                              int64_t ldx, int64_t r, double* Y, int64_t ldy, double alpha, double beta,
-                             const SampleTcPlan& pl, unsigned char* scratch, cudaStream_t st);
+                             const SampleTcPlan& pl, unsigned char* scratch, uint32_t limit, int32_t* status,
+                             cudaStream_t st);
 // HSS_OPT_SAMPLE_DF: hss_sample computes in double-float (default: FP64).
 extern bool g_sample_df;
 // Diagonal-block products of the leaves (see hss_sample.cu).

@@ -35,6 +35,7 @@
 #include <cstdint>
 
 #include "hss_oz.cuh"
+#include "hss_internal.h"
 #include "hss_optin.h"
 #include "hss_sample.h"
 
@@ -105,6 +106,8 @@ struct TcProblem {
   const unsigned char* xs;  // slices of X
   double alpha, beta;
   double* partial;          // null: Y = alpha acc + beta Y
+  uint32_t limit;           // polls of a wait before it gives up
+  int32_t* status;          // gets DEV_TIMEOUT then
 };
 
 // TRANS: op(A) = A^T, rows of op(A) are columns of A.  Thread layouts of a
@@ -119,7 +122,6 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
   __shared__ __align__(8) uint64_t s_full[2], s_done[2];   // a stage's slices of Omega are in; its MMAs are done
   __shared__ int s_code[4][SM_];
   __shared__ int s_row[SM_], s_col[NC];
-  __shared__ int s_fail;
   using Z = Sizes<NC>;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t row0 = (int64_t)blockIdx.x * SM_;
@@ -138,7 +140,6 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
       oz::mbar_init(&s_done[i]);
     }
     asm volatile("fence.mbarrier_init.release.cluster;");
-    s_fail = 0;
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -184,8 +185,11 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
   const uint32_t tacc = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)oc0;
 
   uint32_t use = 0;   // stages issued so far: ring half use & 1, its use / 2-th use
-  bool ok = true;
-  for (int64_t c = c0; c < c1; ++c) {
+  uint32_t loads = 0, mmas = 0;   // (thread 0) copies and groups of MMAs issued
+  // A wait that runs out makes `fail` true in its thread; nothing is issued after it, and
+  // the block leaves together at the next barrier.
+  bool fail = false, ok = true;
+  for (int64_t c = c0; c < c1 && ok; ++c) {
     // row exponents of the chunk
     uint32_t hmax = 0, have = 0;
 #pragma unroll
@@ -221,9 +225,13 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
       const int h = use & 1;
       unsigned char* abuf = smem + h * Z::stage;
       unsigned char* bbuf = abuf + oz::kSlices * kASlice;
+      if (!ok) continue;
       // the ring half is free once the MMAs of its previous use are done
-      if (use >= 2 && !oz::mbar_wait(&s_done[h], ((use >> 1) - 1) & 1)) s_fail = 1;
-      if (tid == 0) oz::bulk_load(bbuf, xs + c * Z::bchunk + s * Z::bstage, Z::bstage, &s_full[h]);
+      if (use >= 2) fail = fail || !oz::mbar_wait(&s_done[h], ((use >> 1) - 1) & 1, p.limit);
+      if (tid == 0 && !fail) {
+        oz::bulk_load(bbuf, xs + c * Z::bchunk + s * Z::bstage, Z::bstage, &s_full[h]);
+        ++loads;
+      }
       if constexpr (TRANS) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -248,18 +256,23 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
       load(c + 1, s);   // the next chunk's values replace the ones just used
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncthreads();
+      ok = !__syncthreads_or(fail);
+      if (!ok) continue;
       if (tid == 0) {
         asm volatile("tcgen05.fence::after_thread_sync;");
-        if (!oz::mbar_wait(&s_full[h], (use >> 1) & 1)) s_fail = 1;
-        oz::stage_mma<SM_, NC>(tmem, oz::smem_u32(abuf), kASlice, oz::smem_u32(bbuf), s == 0);
-        oz::mma_commit(&s_done[h]);
+        fail = !oz::mbar_wait(&s_full[h], (use >> 1) & 1, p.limit);
+        if (!fail) {
+          oz::stage_mma<SM_, NC>(tmem, oz::smem_u32(abuf), kASlice, oz::smem_u32(bbuf), s == 0);
+          oz::mma_commit(&s_done[h]);
+          ++mmas;
+        }
       }
       ++use;
     }
+    if (!ok) break;
     // all MMAs of the chunk are done when its last stage's are
     const uint32_t last = use - 1;
-    if (!oz::mbar_wait(&s_done[last & 1], (last >> 1) & 1)) s_fail = 1;
+    fail = fail || !oz::mbar_wait(&s_done[last & 1], (last >> 1) & 1, p.limit);
     asm volatile("tcgen05.fence::after_thread_sync;");
     const int ea = s_row[orow];
     uint32_t direct = 0;   // columns of this thread's row that are summed in FP64
@@ -304,12 +317,8 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();   // the accumulators and the codes may be overwritten
+    ok = !__syncthreads_or(fail);   // the accumulators and the codes may be overwritten
     asm volatile("tcgen05.fence::after_thread_sync;");
-    if (s_fail) {
-      ok = false;
-      break;
-    }
   }
 
   if (row0 + orow < p.m) {
@@ -327,11 +336,11 @@ __global__ void __launch_bounds__(ST, 1) sample_tc_kernel(TcProblem p) {
     }
   }
   if (!ok && tid == 0) {
-    // let copies and MMAs that may still be running end (bounded)
-    for (int i = 0; i < 2; ++i) {
-      oz::mbar_wait(&s_full[i], 0);
-      oz::mbar_wait(&s_done[i], 0);
-    }
+    if (p.status) *(volatile int32_t*)p.status = DEV_TIMEOUT;
+    __threadfence_system();
+    // copies and MMAs that may still be running end before the block does (bounded)
+    for (uint32_t i = loads > 2 ? loads - 2 : 0; i < loads; ++i) oz::mbar_wait(&s_full[i & 1], (i >> 1) & 1);
+    for (uint32_t i = mmas > 2 ? mmas - 2 : 0; i < mmas; ++i) oz::mbar_wait(&s_done[i & 1], (i >> 1) & 1);
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
@@ -379,9 +388,10 @@ SampleTcPlan sample_tc_plan(int64_t m, int64_t k, int64_t r, int sms) {
 
 cudaError_t launch_sample_tc(const double* A, int64_t lda, int64_t m, int64_t k, int trans, const double* X,
                              int64_t ldx, int64_t r, double* Y, int64_t ldy, double alpha, double beta,
-                             const SampleTcPlan& pl, unsigned char* scratch, cudaStream_t st) {
+                             const SampleTcPlan& pl, unsigned char* scratch, uint32_t limit, int32_t* status,
+                             cudaStream_t st) {
   double* partial = pl.nsplit > 1 ? (double*)(scratch + pl.slice_bytes) : nullptr;
-  const TcProblem p{A, lda, X, ldx, Y, ldy, m, k, r, pl.per, scratch, alpha, beta, partial};
+  const TcProblem p{A, lda, X, ldx, Y, ldy, m, k, r, pl.per, scratch, alpha, beta, partial, limit, status};
   cudaError_t e = pl.nc == 16 ? launch_tc<16>(p, trans, pl, scratch, st) : launch_tc<32>(p, trans, pl, scratch, st);
   if (e == cudaSuccess && partial) e = launch_sample_reduce(partial, pl.nsplit, m, r, Y, ldy, alpha, beta, st);
   return e;

@@ -361,7 +361,10 @@ int32_t hss_version(void);
 
 /* S = alpha * op(A) * X + beta * S (op(A) = A if trans == 0, A^T if 1):
  * A * Omega and A' * Omega of src/compression.jl:290-291, :326-327, :336-337.
- * X has n (trans 0) or m (trans 1) rows and r columns.  FP64. */
+ * X has n (trans 0) or m (trans 1) rows and r columns.  In FP64 accuracy, above 2048
+ * inner terms on the tensor cores.  Asynchronous; a wait of that kernel that runs
+ * out (HSS_OPT_POLL_LIMIT) leaves NaN in its rows, and the next hss_sample or
+ * hss_sumsq on the device returns HSS_ERR_TIMEOUT. */
 int hss_sample(const double* dA, int64_t lda, int64_t m, int64_t n, int32_t trans, const double* dX, int64_t ldx,
                int64_t r, double* dY, int64_t ldy, double alpha, double beta, void* stream);
 
