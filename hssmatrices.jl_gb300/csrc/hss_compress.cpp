@@ -73,21 +73,6 @@ int sample_expired(int device) {
   return set_error(HSS_ERR_TIMEOUT, "sample product: a wait ran out in an earlier call; its rows are NaN");
 }
 
-// The product on the tensor cores, with stream-ordered scratch, so that calls
-// on different streams do not share it.
-int sample_tc(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_t trans, const double* dX, int64_t ldx,
-              int64_t r, double* dY, int64_t ldy, double alpha, double beta, int device, cudaStream_t st) {
-  const SampleTcPlan pl = sample_tc_plan(rows, inner, r, sm_count(device));
-  unsigned char* scratch = nullptr;
-  RC_TRY(cudaMallocAsync((void**)&scratch, pl.scratch_bytes, st));
-  cudaError_t e = launch_sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, pl, scratch,
-                                   pmv_poll_limit(), sample_status(device), st);
-  count_launches(pl.nsplit > 1 ? 3 : 2);
-  const cudaError_t f = cudaFreeAsync(scratch, st);
-  if (e == cudaSuccess) e = f;
-  return e == cudaSuccess ? HSS_OK : set_cuda_error(e, "sample product");
-}
-
 // The product on the CUDA cores, in FP64 or (HSS_OPT_SAMPLE_DF) double-float.
 int sample_cores(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_t trans, const double* dX,
                  int64_t ldx, int64_t r, double* dY, int64_t ldy, double alpha, double beta, int device,
@@ -104,6 +89,25 @@ int sample_cores(const double* dA, int64_t lda, int64_t rows, int64_t inner, int
     cudaError_t f = cudaFreeAsync(partial, st);
     if (e == cudaSuccess) e = f;
   }
+  return e == cudaSuccess ? HSS_OK : set_cuda_error(e, "sample product");
+}
+
+// The product on the tensor cores, with stream-ordered scratch, so that calls
+// on different streams do not share it; where the scratch (digit slices of X, partial
+// sums: more than the CUDA cores' product takes) cannot be had, on those.
+int sample_tc(const double* dA, int64_t lda, int64_t rows, int64_t inner, int32_t trans, const double* dX, int64_t ldx,
+              int64_t r, double* dY, int64_t ldy, double alpha, double beta, int device, cudaStream_t st) {
+  const SampleTcPlan pl = sample_tc_plan(rows, inner, r, sm_count(device));
+  unsigned char* scratch = nullptr;
+  if (dev_alloc_async((void**)&scratch, pl.scratch_bytes, st) != cudaSuccess) {
+    cudaGetLastError();
+    return sample_cores(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, device, st);
+  }
+  cudaError_t e = launch_sample_tc(dA, lda, rows, inner, trans, dX, ldx, r, dY, ldy, alpha, beta, pl, scratch,
+                                   pmv_poll_limit(), sample_status(device), st);
+  count_launches(pl.nsplit > 1 ? 3 : 2);
+  const cudaError_t f = cudaFreeAsync(scratch, st);
+  if (e == cudaSuccess) e = f;
   return e == cudaSuccess ? HSS_OK : set_cuda_error(e, "sample product");
 }
 
