@@ -94,10 +94,12 @@ struct BlkLayout {
     total = oX + zmax(tail, sz4(extra));
   }
 };
+// The kernel (its S) of a launch.  Nodes without rows (every rank below is 0) may still
+// have column bases, whose translators are staged: S is at least 32.
 template <typename T>
 constexpr int size_bucket(int mmax, int nmax) {
   const int s = mmax > nmax ? mmax : nmax;
-  return sizeof(T) == 8 && s > 32 ? 48 : (s + 31) / 32 * 32;
+  return s <= 32 ? 32 : sizeof(T) == 8 ? 48 : (s + 31) / 32 * 32;
 }
 static_assert(BP * GP + 4 + 2 * SVP <= BP * XP, "the Gram matrix and the broadcast reflectors fit in X");
 
@@ -1025,8 +1027,9 @@ bool factor_blk_fits(int mmax, int nmax, int kumax, int kvmax, size_t extra) {
 
 namespace {
 template <typename T, int S>
-void launch_blk_sized(const Task* t, int64_t nt, const Slot* s, int kumax, int kvmax, size_t extra, size_t smem,
-                      cudaStream_t st, bool pdl) {
+void launch_blk_sized(const Task* t, int64_t nt, const Slot* s, int kumax, int kvmax, size_t extra, cudaStream_t st,
+                      bool pdl) {
+  const size_t smem = BlkLayout(S, kumax, kvmax, extra).total * sizeof(T);   // the layout that the kernel works with
   static SmemOptIn opt_in;
   opt_in((const void*)ulv_factor_blk_kernel<T, S>, sizeof(T) == 4 ? kBlkSmemCap : kBlkSmemCap64);
   cudaLaunchConfig_t cfg = {};
@@ -1047,17 +1050,16 @@ template <typename T>
 void launch_ulv_factor_blk(const Task* t, int64_t nt, const Slot* s, int mmax, int nmax, int kumax, int kvmax,
                            size_t extra, cudaStream_t st, bool pdl) {
   if (nt <= 0) return;
-  const size_t smem = factor_blk_smem<T>(mmax, nmax, kumax, kvmax, extra);
   const int bucket = size_bucket<T>(mmax, nmax);
   if constexpr (sizeof(T) == 8) {
-    if (bucket == 32) launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st, pdl);
-    else launch_blk_sized<T, 48>(t, nt, s, kumax, kvmax, extra, smem, st, pdl);
+    if (bucket == 32) launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, st, pdl);
+    else launch_blk_sized<T, 48>(t, nt, s, kumax, kvmax, extra, st, pdl);
   } else {
     switch (bucket) {
-      case 32: launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
-      case 64: launch_blk_sized<T, 64>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
-      case 96: launch_blk_sized<T, 96>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
-      default: launch_blk_sized<T, 128>(t, nt, s, kumax, kvmax, extra, smem, st, pdl); break;
+      case 32: launch_blk_sized<T, 32>(t, nt, s, kumax, kvmax, extra, st, pdl); break;
+      case 64: launch_blk_sized<T, 64>(t, nt, s, kumax, kvmax, extra, st, pdl); break;
+      case 96: launch_blk_sized<T, 96>(t, nt, s, kumax, kvmax, extra, st, pdl); break;
+      default: launch_blk_sized<T, 128>(t, nt, s, kumax, kvmax, extra, st, pdl); break;
     }
   }
 }
