@@ -34,7 +34,7 @@
 // Measured, us (each leaf its own chain, four blocks an SM -> groups): n = 65536, k =
 // 32: r = 1 99 -> 68, 2 141 -> 113, 4 226 -> 208; n = 16384 r = 1 62 -> 40; n = 10007,
 // leaves of 39 rows, k = 20: r = 1 60 -> 38, 7 (queued product) 129 -> 71; n = 512 r = 1
-// 32 -> 23.  n = 65536, r = 1 inside the launch (57): leaves 12, inner branches 4, chain
+// 32 -> 23; the runs of rows32 add up to 4 % (n = 65536, r = 1).  Inside that launch (57): leaves 12, inner branches 4, chain
 // 9, rest of phase A and the wait 4, phase B 6, path 8, inner 6, U F 6.
 #include <cuda_runtime.h>
 
@@ -216,9 +216,12 @@ __device__ __forceinline__ void dotl(int no, const Term (&t)[NS], int ldx, Epi e
 
 // One row of A x (a lane a row, A at the lane's row: any valid one where the row
 // does not count) for NC columns; lane k of the warp loads x(k, q) and passes it round.
-template <int NC, class X>
+// The terms are added up in runs of U, and the runs' sums one after the other.  One
+// chain has more rounding error (n = 8192, rms in units of roundoff: leaves of 128 rows
+// 3.4 against 1.6, of 40 rows 1.83 against 1.25; the kernel before this one, with
+// several threads a row, 1.6 to 1.9 and 1.23), and saves 2.7 of 66 us at n = 65536, r = 1.
+template <int NC, int U = 16, class X>
 __device__ __forceinline__ void rows32(double (&acc)[NC], const double* A, int64_t lda, int K, X x) {
-  constexpr int U = 16;
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < NC; ++q) acc[q] = 0.0;
@@ -230,14 +233,16 @@ __device__ __forceinline__ void rows32(double (&acc)[NC], const double* A, int64
 #pragma unroll
     for (int u0 = 0; u0 < 32; u0 += U) {
       if (u0 >= kn) break;
-      double v[U];
+      double v[U], run[NC];
+#pragma unroll
+      for (int q = 0; q < NC; ++q) run[q] = 0.0;
       if (u0 + U <= kn) {
 #pragma unroll
         for (int u = 0; u < U; ++u, A += lda) v[u] = __ldg(A);
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
-          for (int q = 0; q < NC; ++q) acc[q] = fma(v[u], __shfl_sync(0xffffffffu, w[q], u0 + u), acc[q]);
+          for (int q = 0; q < NC; ++q) run[q] = fma(v[u], __shfl_sync(0xffffffffu, w[q], u0 + u), run[q]);
       } else {
 #pragma unroll
         for (int u = 0; u < U; ++u) v[u] = u0 + u < kn ? __ldg(A + u * lda) : 0.0;
@@ -245,9 +250,11 @@ __device__ __forceinline__ void rows32(double (&acc)[NC], const double* A, int64
         for (int u = 0; u < U; ++u) {
           if (u0 + u >= kn) break;
 #pragma unroll
-          for (int q = 0; q < NC; ++q) acc[q] = fma(v[u], __shfl_sync(0xffffffffu, w[q], u0 + u), acc[q]);
+          for (int q = 0; q < NC; ++q) run[q] = fma(v[u], __shfl_sync(0xffffffffu, w[q], u0 + u), run[q]);
         }
       }
+#pragma unroll
+      for (int q = 0; q < NC; ++q) acc[q] += run[q];
     }
   }
 }
@@ -274,7 +281,10 @@ __device__ void leaf_unit(const FlatArgs& a, int u) {
     const double* X = sl.B + nd.col0 + (int64_t)j0 * sl.ldb;
     const int64_t ldb = sl.ldb;
     double acc[NC];
-    rows32<NC>(acc, nd.D + min(r0 + lane, m - 1), m, n, [&](int k, int q) { return q < nc ? __ldg(X + k + q * ldb) : 0.0; });
+    auto x = [&](int k, int q) { return q < nc ? __ldg(X + k + q * ldb) : 0.0; };
+    const double* D = nd.D + min(r0 + lane, m - 1);
+    if (n > 64) rows32<NC>(acc, D, m, n, x);
+    else rows32<NC, 8>(acc, D, m, n, x);   // short rows have runs enough only of eight
     const double* Y = sl.Y ? sl.Y + nd.row0 + r0 + lane + (int64_t)j0 * sl.ldy : nullptr;
     const bool yterm = sl.beta != 0.0 && Y != nullptr;
     double* C = sl.C + nd.row0 + r0 + lane + (int64_t)j0 * sl.ldc;
