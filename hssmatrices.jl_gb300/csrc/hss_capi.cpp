@@ -181,7 +181,7 @@ struct hss_plan_s {
   std::vector<int64_t> tree_m, tree_n;
   double* d_gen = nullptr;
   Node* d_nodes = nullptr;
-  Task* d_tasks = nullptr;
+  Task* d_tasks = nullptr;              // in d_nodes' block
   std::vector<Seg> by_h, by_d, mv_up, mv_dn;
   Seg leaves;
   int64_t ws_mv = 0, ws_sv = 0;         // workspace rows
@@ -278,10 +278,8 @@ hss_plan_s::~hss_plan_s() {
   if (d_oz) cudaFree(d_oz);
   if (oz_event) cudaEventDestroy(oz_event);
   if (d_gen) cudaFree(d_gen);
-  if (d_nodes) cudaFree(d_nodes);
-  if (d_tasks) cudaFree(d_tasks);
-  if (d_err) cudaFree(d_err);
-  if (d_sync) cudaFree(d_sync);
+  if (d_nodes) cudaFree(d_nodes);   // and the tasks behind them
+  if (d_err) cudaFree(d_err);       // and d_sync
   if (d_flat) cudaFree(d_flat);
 }
 
@@ -734,11 +732,14 @@ int build_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, bool device_fill
   const int64_t total_gen = gbases.back();
   P->gen_len = total_gen;
   CUDA_TRY(dev_alloc((void**)&P->d_gen, std::max<int64_t>(total_gen, 1) * sizeof(double)));
-  CUDA_TRY(dev_alloc((void**)&P->d_err, sizeof(int32_t)));
-  CUDA_TRY(cudaMemset(P->d_err, 0, sizeof(int32_t)));
+  // the status word and the counters in one block, nodes and tasks in another: making a
+  // plan is allocations and copies (n = 10007, with four separate blocks: 415 -> 385 us,
+  // a first adjoint product, which makes one, 512 -> 487; n = 512 79 -> 68, 112 -> 103)
+  constexpr size_t kErrWords = 64;
   const size_t nsync = std::max<size_t>(P->nodes.size(), 1) * pmv_sync_chunks();
-  CUDA_TRY(dev_alloc((void**)&P->d_sync, nsync * sizeof(int32_t)));
-  CUDA_TRY(cudaMemset(P->d_sync, 0, nsync * sizeof(int32_t)));
+  CUDA_TRY(dev_alloc((void**)&P->d_err, (kErrWords + nsync) * sizeof(int32_t)));
+  CUDA_TRY(cudaMemset(P->d_err, 0, (kErrWords + nsync) * sizeof(int32_t)));
+  P->d_sync = P->d_err + kErrWords;
   for (const Node& x : P->nodes) {
     if (x.leaf) {
       P->pmv_nleaf = std::max(P->pmv_nleaf, x.gn);
@@ -789,13 +790,16 @@ int build_plan(hss_plan_s* P, const std::vector<TreeIn>& trees, bool device_fill
     x.B12 = gp(o.B12); x.B21 = gp(o.B21);
     x.R1 = gp(o.R1); x.R2 = gp(o.R2); x.W1 = gp(o.W1); x.W2 = gp(o.W2);
   }
-  const int64_t total_nodes = (int64_t)P->nodes.size();
-  CUDA_TRY(dev_alloc((void**)&P->d_nodes, total_nodes * sizeof(Node)));
-  CUDA_TRY(cudaMemcpy(P->d_nodes, P->nodes.data(), total_nodes * sizeof(Node), cudaMemcpyHostToDevice));
+  const size_t node_bytes = (P->nodes.size() * sizeof(Node) + 255) & ~size_t(255);
+  const size_t task_bytes = std::max<size_t>(tasks.size(), 1) * sizeof(Task);
+  CUDA_TRY(dev_alloc((void**)&P->d_nodes, node_bytes + task_bytes));
+  P->d_tasks = (Task*)((unsigned char*)P->d_nodes + node_bytes);
   for (auto& t : tasks) t.nodes = P->d_nodes;
   P->h_tasks = tasks;
-  CUDA_TRY(dev_alloc((void**)&P->d_tasks, std::max<size_t>(tasks.size(), 1) * sizeof(Task)));
-  CUDA_TRY(cudaMemcpy(P->d_tasks, tasks.data(), tasks.size() * sizeof(Task), cudaMemcpyHostToDevice));
+  std::vector<unsigned char> img(node_bytes + tasks.size() * sizeof(Task));
+  if (!P->nodes.empty()) std::memcpy(img.data(), P->nodes.data(), P->nodes.size() * sizeof(Node));
+  if (!tasks.empty()) std::memcpy(img.data() + node_bytes, tasks.data(), tasks.size() * sizeof(Task));
+  CUDA_TRY(cudaMemcpy(P->d_nodes, img.data(), img.size(), cudaMemcpyHostToDevice));
   return build_flat_tables(P, tasks);
 }
 
