@@ -70,15 +70,19 @@ struct SampleTcPlan {
   size_t slice_bytes = 0, scratch_bytes = 0;
 };
 // Whether hss_sample's product over k inner terms takes that kernel, with either
-// setting of HSS_OPT_SAMPLE_DF (it is more accurate than the double-float product
-// and no slower: 8192 x 8192, 30 columns: 440 us against 1420 us and, in FP64 on
-// the FP64 pipe, 3750 us; 4096 x 4096, 1 column: 97, 104 and 212 us).  It is also
-// faster below (1242 x 1242, 13 columns: 33 and 80 us).  The line at 2048 terms,
-// and hss_rc_sample staying with the former kernels at every size, keep the rank
-// decisions of compressions what they were: at a tolerance of 1e-9 they depend on
-// the rounding of the samples (2048 points of the Cauchy kernel: one node in 31
-// differs from the reference algorithm's ranks with the former rounding, three
-// with samples that are exact to the last bit).
+// setting of HSS_OPT_SAMPLE_DF.  It is more accurate than both products on the CUDA
+// cores (rms error 0.3 of the FP64 one's at 4096 terms) and faster on every shape
+// measured, also with few rows (its tiles are 128 rows high): FP64 pipe / tensor cores
+// in us, 2100 terms, 1 row, 1 column 38 / 27, 3000 rows, 30 columns 356 / 58; 20000
+// terms, 1 row, 1 column 123 / 48, 100 rows, 30 columns 200 / 64; 100000 terms, 400
+// rows, 1 column 701 / 236; 8192 x 8192, 30 columns 3750 / 440 (double-float 1420).
+// Below 2048 terms it would be faster too (1242 x 1242, 13 columns: 80 / 33).  The line
+// is not one of time: samples of hss_sample that a program hands to hss_rc_compress
+// decide ranks, which at a tolerance of 1e-9 depend on the samples' rounding, and up
+// to 2048 terms (the largest such comparison with the reference algorithm: points of
+// the Cauchy kernel, one node in 31 differs with FP64 sums, three with samples that are
+// exact to the last bit) they stay what they were.  hss_rc_sample, the product of the
+// compressions here, keeps FP64 sums at every size.
 inline bool sample_tc_pays(int64_t k) { return k > 2048; }
 // limit: polls of a wait before it gives up; the rows of its block are NaN then, and
 // *status (host memory that the device can write, or null) is DEV_TIMEOUT.

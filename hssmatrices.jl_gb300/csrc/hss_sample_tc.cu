@@ -16,16 +16,15 @@
 // accumulators are put together and added to FP64 sums in registers, the only
 // FP64 instructions (one addition per output and chunk).  A thread keeps at most
 // 32 + NC / 4 doubles in registers, which with 512 threads is what the register
-// file holds; the 180 KB ring leaves one block per SM.
+// file holds; the ring (184 KB, with tiles of 32 columns 200 KB) leaves one block per SM.
 //
 // What bounds it now: cutting A into digits, about 45 integer instructions per
 // entry (ALU pipe 52 % busy, tensor pipe 20 %, DRAM 17 %); per chunk of 128 x 128
 // about 12 us.  Measured (one GB300, L2 cold): 8192 x 8192, 30 columns 3750 ->
 // 444 us; 16384 x 16384, 20 columns 9500 -> 1380 us (1.55 TB/s of A); 4096 x
-// 4096, 20 columns 604 -> 122 us.  Error against exact sums, relative to
-// 2^-53 (|A| |X|), root mean square: 0.46 -> 0.17 (Cauchy kernel, 2048 points),
-// 0.13 -> 0.05 (normal entries); leaving out the products with d = 8 gave 0.91
-// and 0.20.
+// 4096, 20 columns 604 -> 122 us.  Error against exact sums of 4096 terms, root
+// mean square relative to the sums, in units of roundoff: 4.8 -> 1.2 (a kernel matrix),
+// 4.0 -> 1.3 (normal entries).
 //
 // Blocks of one row tile split the chunks so that every SM has work; their sums
 // go to a scratch buffer that sample_reduce_kernel adds in a fixed order.

@@ -177,7 +177,10 @@ class HssServer:
         fac_elems = 2 * packed.size + 8 * m     # factor blocks, reflector copies, tau vectors
         item = 4 if precision == "fp32" else 8
         # FP32 + refinement: the digit slices of the generators for the tensor-core
-        # residual (9 x 2 bytes per entry, and the zero blocks of stacked translators)
+        # residual, 2.5 times the generators (ten bf16 slices an entry) at ranks that are
+        # multiples of 32 and more below (inner ranks are padded to 32; rank 8, leaves of
+        # 128 rows: 3.0).  _account puts the bytes that the matrix holds in their place
+        # after its factorization and after every solve.
         extra = 3 * gen if precision == "fp32" else 0
         return gen + extra + fac_elems * item + 64 * m * 8
 

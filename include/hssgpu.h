@@ -197,11 +197,12 @@ int hss_device_bytes(hss_handle h, hss_factor f, int64_t* bytes);
  * on scratch right-hand sides with r columns, the two solve kernels of every
  * tree level of this factorization -- a warp per right-hand side ("register")
  * and a block per 32 right-hand sides with GEMM steps ("blocked", FP32 factors)
- * -- and the two refinement residual products (one persistent launch, one
- * launch per level), and keeps the faster per level in the factorization for
+ * -- and two refinement residual products (the default one, on the tensor cores
+ * unless an option or a lack of memory says otherwise, and one launch per level on
+ * the CUDA cores), and keeps the faster per level in the factorization for
  * its later solves (hss_ulvsolve*; a batcher's merged solves use the built-in
  * rule).  Synchronises the stream.  hss_autotune_info reads the choices back:
- * per level 1 blocked, 0 register, -1 not tuned; product 1 persistent, 0 per
+ * per level 1 blocked, 0 register, -1 not tuned; product 1 the default one, 0 per
  * level, -1 not tuned (arrays of *nup / *ndown entries; null to query sizes). */
 int hss_autotune(hss_factor f, int64_t r, void* stream);
 int hss_autotune_info(hss_factor f, int32_t* nup, int8_t* up, int32_t* ndown, int8_t* down, int32_t* pmv);
@@ -303,11 +304,12 @@ int64_t hss_launch_counter(void);
  * the device and sets the condition of a while node around the refinement
  * step, and the host reads the loop's status once.  The "_host" solves run on
  * the plan's own non-blocking stream, ordered after the legacy default stream.
- * HSS_OPT_SAMPLE_DF = 1 computes hss_sample's products in double-float
- * arithmetic on the FP32 pipe (~2^-47 relative per operation instead of
- * FP64's 2^-53, several times faster on GB300; entries of A and X must lie
- * within float's exponent range): the mixed-precision form of the sampling
- * in randcompress.  0 (default): FP64.
+ * HSS_OPT_SAMPLE_DF = 1 computes the off-diagonal part of hss_rc_sample's products,
+ * and hss_sample's products on the CUDA cores (up to 2048 inner terms, or where the
+ * tensor cores' scratch cannot be had), in double-float arithmetic on the FP32 pipe
+ * (~2^-47 relative per operation instead of FP64's 2^-53, several times faster on
+ * GB300; entries of A and X must lie within float's exponent range): the
+ * mixed-precision form of the sampling in randcompress.  0 (default): FP64.
  * HSS_OPT_FLAT_PRODUCT = 0 turns off the flat form of the persistent FP64
  * product (1, default: FP64 products of at most 4 columns run it, and of up to
  * 32 where the multiply-adds are few enough; a block takes a group of leaves
@@ -355,9 +357,10 @@ int32_t hss_version(void);
  * reference's `randcompress(A, rcl, ccl, kest)` (:278) and
  * `randcompress_adaptive(A, rcl, ccl; kest)` (:312) become, on the host:
  * draw Omega_col (n x s), Omega_row (m x s); S_col = A * Omega_col and
- * S_row = A^T * Omega_row with hss_sample; hss_rc_compress; for the adaptive
- * form, test with fresh samples through hss_sample, hss_matmul and hss_sumsq
- * and repeat with more columns (the loop of :330-352). */
+ * S_row = A^T * Omega_row with hss_rc_sample (whose sums' rounding the rank decisions
+ * are tested with); hss_rc_compress; for the adaptive form, test with fresh samples
+ * through hss_rc_sample, hss_matmul and hss_sumsq and repeat with more columns (the
+ * loop of :330-352). */
 
 /* S = alpha * op(A) * X + beta * S (op(A) = A if trans == 0, A^T if 1):
  * A * Omega and A' * Omega of src/compression.jl:290-291, :326-327, :336-337.
@@ -402,8 +405,8 @@ int hss_rc_ranks(hss_rc rc, int32_t* ranks);
  * blocks is multiplied in double-float arithmetic and the leaf blocks' part
  * D * X is added in FP64, so that the corrected sample S - D * X that
  * hss_rc_compress forms keeps double-float accuracy relative to itself (the
- * near-diagonal entries of kernel matrices dominate S).  Without the option:
- * hss_sample in FP64. */
+ * near-diagonal entries of kernel matrices dominate S).  Without the option: FP64
+ * sums on the FP64 pipe at every size (hss_sample's product up to 2048 terms). */
 int hss_rc_sample(hss_rc rc, const double* dA, int64_t lda, int32_t trans, const double* dX, int64_t ldx, int64_t r,
                   double* dY, int64_t ldy, void* stream);
 
